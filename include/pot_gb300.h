@@ -90,7 +90,7 @@ typedef struct OtgDenseProblem {
   void* out_u;        /* knopp: scaling u; log: log_u (natural log)  (n)     */
   void* out_v;        /* knopp: scaling v; log: log_v                (m)     */
   size_t workspace_bytes;
-  int32_t grid;       /* CTAs (0 = all co-resident CTAs); tuning knob        */
+  int32_t grid;       /* most CTAs (0 = the solver's choice); tuning knob     */
   int32_t timeout_ms; /* bound on any single device wait (0 = 4000 ms)       */
   double tau;         /* STAB: absorption threshold on the scalings (> 0)    */
   int32_t check_period; /* STAB: iterations between marginal checks (>= 1) */
@@ -117,6 +117,12 @@ size_t otg_dense_workspace_bytes(int dtype, int64_t n, int64_t m, int hist_cap, 
  *   count and last-iteration flag of OTG_METHOD_STAB). */
 size_t otg_dense_info_offset(int dtype, int64_t n, int64_t m, int hist_cap, int grid);
 int otg_sinkhorn_dense(const OtgDenseProblem* p, void* workspace, cudaStream_t stream);
+
+/* Whether a stored Gibbs kernel (OtgDenseProblem::K, otg_gibbs_kernel) would
+ * save work in this solve: 1 for a float64 scaling form whose passes read the
+ * cost from memory, 0 when the solver keeps the problem on chip (it then
+ * exponentiates every entry once by itself) and for every other form. */
+int otg_dense_wants_gibbs(const OtgDenseProblem* p);
 
 /* Plan and/or loss from potentials: P = exp(-M/reg + u + v) (log form) or
  * diag(u) exp(-M/reg) diag(v) (scaling form); *loss = sum(M * P) in fp64.

@@ -104,6 +104,7 @@ SIGNATURES = {
     "otg_dense_workspace_bytes": (c_sz, [ctypes.c_int, c_i64, c_i64, ctypes.c_int, ctypes.c_int]),
     "otg_dense_info_offset": (c_sz, [ctypes.c_int, c_i64, c_i64, ctypes.c_int, ctypes.c_int]),
     "otg_sinkhorn_dense": (ctypes.c_int, [ctypes.POINTER(OtgDenseProblem), c_vp, c_vp]),
+    "otg_dense_wants_gibbs": (ctypes.c_int, [ctypes.POINTER(OtgDenseProblem)]),
     "otg_dense_plan": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp,
                                       c_dbl, c_vp, c_i64, c_vp, c_vp]),
     "otg_barycenter_workspace_bytes": (c_sz, [ctypes.c_int, ctypes.c_int, c_i64, c_i32]),

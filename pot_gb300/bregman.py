@@ -76,7 +76,8 @@ def solve_dense(M, a, b, reg, method, max_iter, stop_thr, warm_u=None, warm_v=No
     lib = _lib.load()
     n, m = M.shape
     if grid is None:
-        grid = default_grid(n, m, M.dtype)
+        # the solver chooses, but for the stabilised form, which runs the two-pass kernel
+        grid = default_grid(n, m, M.dtype) if method == _lib.OTG_METHOD_STAB else 0
     dt = _lib.dtype_code(M.dtype)
     cap = max(2, max_iter // check_period + 2)
     wsb = lib.otg_dense_workspace_bytes(dt, n, m, cap, grid)
@@ -94,8 +95,8 @@ def solve_dense(M, a, b, reg, method, max_iter, stop_thr, warm_u=None, warm_v=No
     if unbalanced is not None:
         p.reg_m1, p.reg_m2, p.c_ones = float(unbalanced[0]), float(unbalanced[1]), int(unbalanced[2])
     if gibbs is None:
-        gibbs = (method == _lib.OTG_METHOD_KNOPP and unbalanced is None and M.dtype == torch.float64
-                 and n * m * 8 <= GIBBS_MAX_BYTES)
+        gibbs = (method == _lib.OTG_METHOD_KNOPP and unbalanced is None and n * m * 8 <= GIBBS_MAX_BYTES
+                 and lib.otg_dense_wants_gibbs(ctypes.byref(p)) != 0)
     K = None
     if gibbs:
         K = torch.empty((n, m), dtype=M.dtype, device=M.device)

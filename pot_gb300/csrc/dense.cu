@@ -52,18 +52,11 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
-#include "common.cuh"
+#include "dense_common.cuh"
+#include "fused.cuh"
 #include "../../include/pot_gb300.h"
 
 namespace otg {
-
-template <typename T> struct Pair { T mx, s; };
-
-template <typename T>
-__device__ __forceinline__ Pair<T> ldcg_pair(const Pair<T>* p) {
-  const T* q = reinterpret_cast<const T*>(p);
-  return Pair<T>{__ldcg(q), __ldcg(q + 1)};
-}
 
 template <typename T>
 struct DenseArgs {
@@ -95,12 +88,6 @@ struct DenseArgs {
   double* eslab;                        // [nslabs] squared marginal error of each slab (check passes)
 };
 
-// Per-thread maxima carried out of a pass (stabilised: d0; unbalanced:
-// |u_new - u_old|, |u_new|, |u_old|).
-struct Track {
-  double d0 = -INFINITY, d1 = -INFINITY, d2 = -INFINITY;
-};
-
 template <int METHOD> struct LogDomain {
   static constexpr bool value = METHOD == OTG_METHOD_LOG || METHOD == OTG_METHOD_STAB;
 };
@@ -124,31 +111,6 @@ __global__ void gibbs_kernel(const T* __restrict__ M, int64_t n, int64_t m, int6
                              int64_t ldk) {
   for (int64_t i = blockIdx.x; i < n; i += gridDim.x)
     for (int64_t j = threadIdx.x; j < m; j += blockDim.x) K[i * ldk + j] = gibbs<T, OTG_METHOD_KNOPP>(M[i * ldm + j], c);
-}
-
-// Order-preserving map of doubles to unsigned keys (atomicMax on keys = max
-// on values; key 0 is below every value).
-__device__ __forceinline__ unsigned long long order_key(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double key_value(unsigned long long k) {
-  return (k >> 63) ? __longlong_as_double((long long)(k & 0x7fffffffffffffffull)) : __longlong_as_double((long long)~k);
-}
-
-// Block-wide max of one value per thread, then one atomicMax per CTA.  All
-// threads of the block call it.
-__device__ void block_max_atomic(double x, unsigned long long* slot) {
-  __shared__ double red[32];
-  x = warp_max(x);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = -INFINITY;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t = fmax(t, red[k]);
-    if (t != -INFINITY) atomicMax(slot, order_key(t));
-  }
-  __syncthreads();
 }
 
 constexpr int RW = 4;     // rows per warp in the row pass
@@ -742,6 +704,8 @@ struct Layout {
   int grid, Sr, Sc;
   int64_t rchunk, cchunk;
   size_t off_state, off_pcol, off_prow, off_hist, off_ctrl, off_cnt, off_eslab, total;
+  // behind the two-pass kernel's own space: the one-read kernel's (no bytes when it does not take the shape)
+  size_t off_fused, total_fused;
 };
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -764,7 +728,8 @@ int resolve_grid(int requested) {
 }
 
 template <typename T>
-Layout make_layout(int64_t n, int64_t m, int hist_cap, int grid) {
+Layout make_layout(int64_t n, int64_t m, int hist_cap, int requested) {
+  const int grid = resolve_grid<T>(requested);
   constexpr int VW = Vec<T>::N;
   Layout L{};
   L.grid = grid;
@@ -792,6 +757,9 @@ Layout make_layout(int64_t n, int64_t m, int hist_cap, int grid) {
   L.off_cnt = off; off = align_up(off + sizeof(unsigned) * (size_t)nslabs, 256);
   L.off_eslab = off; off = align_up(off + sizeof(double) * (size_t)nslabs, 256);
   L.total = off;
+  L.off_fused = off;
+  off = align_up(off + fused_bytes(sizeof(T) == 8 ? OTG_F64 : OTG_F32, n, m, requested), 256);
+  L.total_fused = off;
   return L;
 }
 
@@ -805,7 +773,7 @@ int launch_dense(const OtgDenseProblem* p, void* ws, cudaStream_t st) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dense_sinkhorn_kernel<T, METHOD, VEC>, 256, 0);
     if ((int64_t)per * sms < grid) return OTG_ERR_UNSUPPORTED;  // co-residency not possible
   }
-  Layout L = make_layout<T>(p->n, p->m, p->hist_cap, grid);
+  Layout L = make_layout<T>(p->n, p->m, p->hist_cap, p->grid);
   if (p->workspace_bytes < L.total) return OTG_ERR_WORKSPACE;
   char* base = static_cast<char*>(ws);
   DenseArgs<T> A{};
@@ -851,9 +819,35 @@ int launch_dense(const OtgDenseProblem* p, void* ws, cudaStream_t st) {
   return OTG_OK;
 }
 
+// The one-read kernel (fused.cuh) where it takes the problem and the
+// workspace has room for it; OTG_ERR_UNSUPPORTED otherwise.
+template <typename T>
+int try_fused(const OtgDenseProblem* p, void* ws, cudaStream_t st) {
+  if (p->method == OTG_METHOD_STAB) return OTG_ERR_UNSUPPORTED;
+  const Layout L = make_layout<T>(p->n, p->m, p->hist_cap, p->grid);
+  if (L.total_fused == L.total || p->workspace_bytes < L.total_fused) return OTG_ERR_UNSUPPORTED;
+  char* base = static_cast<char*>(ws);
+  T* st_ = reinterpret_cast<T*>(base + L.off_state);
+  const int64_t n = p->n, m = p->m;
+  auto al = [](int64_t k) { return (k + 3) / 4 * 4; };
+  FusedState fs{};
+  int64_t o = 0;
+  fs.u0 = st_ + o; o += al(n); fs.u1 = st_ + o; o += al(n); fs.rowc = st_ + o; o += al(n); fs.fref = st_ + o; o += al(n);
+  fs.v0 = st_ + o; o += al(m); fs.v1 = st_ + o; o += al(m);
+  fs.space = base + L.off_fused;
+  fs.hist = reinterpret_cast<double*>(base + L.off_hist);
+  fs.info = reinterpret_cast<int*>(base + L.off_ctrl);
+  fs.bar = reinterpret_cast<unsigned*>(base + L.off_ctrl + 32);
+  fs.timeout_ns = p->timeout_ms > 0 ? (uint64_t)p->timeout_ms * 1000000ull : 4000000000ull;
+  if (cudaMemsetAsync(base + L.off_hist, 0, L.off_cnt - L.off_hist, st) != cudaSuccess) return OTG_ERR_CUDA;
+  return fused_launch(p, fs, st);
+}
+
 template <typename T>
 int dispatch_dense(const OtgDenseProblem* p, void* ws, cudaStream_t st) {
   constexpr int VW = Vec<T>::N;
+  const int rc = try_fused<T>(p, ws, st);
+  if (rc != OTG_ERR_UNSUPPORTED) return rc;
   if (p->method == OTG_METHOD_KNOPP && p->K) {
     // the passes read K in place of M
     OtgDenseProblem q = *p;
@@ -893,13 +887,13 @@ int check_problem(const OtgDenseProblem* p) {
 extern "C" {
 
 size_t otg_dense_workspace_bytes(int dtype, int64_t n, int64_t m, int hist_cap, int grid) {
-  if (dtype == OTG_F64) return make_layout<double>(n, m, hist_cap, resolve_grid<double>(grid)).total;
-  return make_layout<float>(n, m, hist_cap, resolve_grid<float>(grid)).total;
+  if (dtype == OTG_F64) return make_layout<double>(n, m, hist_cap, grid).total_fused;
+  return make_layout<float>(n, m, hist_cap, grid).total_fused;
 }
 
 size_t otg_dense_info_offset(int dtype, int64_t n, int64_t m, int hist_cap, int grid) {
-  if (dtype == OTG_F64) return make_layout<double>(n, m, hist_cap, resolve_grid<double>(grid)).off_hist;
-  return make_layout<float>(n, m, hist_cap, resolve_grid<float>(grid)).off_hist;
+  if (dtype == OTG_F64) return make_layout<double>(n, m, hist_cap, grid).off_hist;
+  return make_layout<float>(n, m, hist_cap, grid).off_hist;
 }
 
 int otg_sinkhorn_dense(const OtgDenseProblem* p, void* workspace, cudaStream_t stream) {
@@ -908,6 +902,11 @@ int otg_sinkhorn_dense(const OtgDenseProblem* p, void* workspace, cudaStream_t s
   if (!workspace) return OTG_ERR_WORKSPACE;
   if (p->dtype == OTG_F64) return dispatch_dense<double>(p, workspace, stream);
   return dispatch_dense<float>(p, workspace, stream);
+}
+
+int otg_dense_wants_gibbs(const OtgDenseProblem* p) {
+  if (!p || p->method != OTG_METHOD_KNOPP || p->dtype != OTG_F64) return 0;
+  return fused_resident(p) ? 0 : 1;
 }
 
 int otg_dense_plan(int dtype, int method, const void* M, int64_t n, int64_t m, int64_t ldm,
@@ -1061,7 +1060,7 @@ int noalloc_scratch(void** out) {
 
 template <typename T>
 int noalloc_solve(const OtgDenseProblem* p, double* err_hist, int32_t* info, cudaStream_t st) {
-  const Layout L = make_layout<T>(p->n, p->m, p->hist_cap, resolve_grid<T>(p->grid));
+  const Layout L = make_layout<T>(p->n, p->m, p->hist_cap, p->grid);
   if (L.total > (size_t)OTG_NOALLOC_SCRATCH_BYTES) return OTG_ERR_NOALLOC_TOO_LARGE;
   void* scratch = nullptr;
   int rc = noalloc_scratch(&scratch);

@@ -1,0 +1,1492 @@
+// Dense Sinkhorn with ONE read of the cost per iteration, one persistent
+// cooperative launch per solve (scaling, log and unbalanced forms; the
+// iterations, stop tests and reverts are those of dense.cu).
+//
+// Once the row update of row i is known, the row's share of the NEXT column
+// update follows from the same entries: with e_ij = exp(x_ij + v_j + shift)
+// and s_i = sum_j e_ij the updated plan row is P_ij = e_ij a_i / s_i, and
+// sum_i P_ij is both the column marginal of the stop test and all that the
+// column update needs, v_j += log(b_j / sum_i P_ij).  So an iteration is
+//   pass   every CTA goes over its own rows: row reduction, row update, then
+//          the scaled entries (still in registers) are added to per-thread
+//          column sums, which go to the CTA's slot
+//   merge  every CTA adds up the slots of its share of the columns in slot
+//          order, updates v and the squared marginal error
+// with one exponential per entry instead of two and half the HBM traffic of
+// a column pass followed by a row pass.
+//
+// Hand-over.  A grid barrier costs about 1.7 us here (fence, atomic and poll:
+// three trips to L2) and the loads behind it one more trip, so the column
+// sums and the new v do not go through barriers: each value is stored in one
+// 64-bit word with the iteration number (a float64 in two such words) and the
+// reader polls the value itself.  A slot is rewritten only after its writer
+// has read all of the next v, which every reader of the slot has contributed
+// to, and v likewise, so single buffers are enough.  Per-iteration flags and
+// error shares travel the same way and every CTA takes the same decisions.
+//
+// Split.  A CTA of 8 warps (255 registers a thread: nothing may spill, as the
+// shared memory leaves an L1 of 28 KB and a spilled loop runs at L2 latency;
+// measured 1.5 to 2 times slower) owns a contiguous range of rows; G warps
+// share a row and 8 / G groups work side by side.  A thread holds NK 16-byte
+// vectors of each of RB rows, at most 256 bytes of entries.
+//   Resident: the CTA's rows stay in shared memory for the whole solve; the
+//   fewest vectors per thread (NK) that cover a row and let the rows fit, so
+//   that up to 8 rows share one reduction (reduce-scatter over the warp, one
+//   barrier), one division and one read of v.
+//   Streamed (cost larger than the SMs' shared memory, 30 MB): NK = 16, one
+//   row at a time per group, so that one group's reduction overlaps another's
+//   exponentials.  A ring of bulk copies issued by one lane per group, in
+//   chunks of half a row; five or six chunks of 32 KB are in flight per SM,
+//   and the copies of the next pass's first rows cross the hand-over.
+//
+// Range of the shortcut.  Log form: the shift of row i is its previous
+// potential less log a_i, so e_ij is the row's previous plan entry over a_i
+// and s_i is near one; rows whose s_i leaves [2^-30, 2^30] (first iterations
+// from a far start, zero weights, non-finite input) take the running-maximum
+// form on the same entries.  A column whose sum is below 2^-70 may have lost
+// terms to underflow: then the whole grid recomputes the column update with
+// running maxima (one extra pass) in that iteration.
+//
+// float64 log form, cost resident: this GPU issues FP64 at about two lanes
+// per clock and SM, and an exponential costs some twenty such operations.
+// The solver stores the plan of the current potentials,
+// K_ij = exp(x_ij + f_i + g_j) (row-normalised), and iterates scalings u, v
+// over it, f + log u and g + log v being the potentials: two FMAs per entry.
+// When a scaling leaves [2^-300, 2^300] the potentials absorb it and K is
+// rebuilt with running maxima.
+#pragma once
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+#include "dense_common.cuh"
+#include "fused.cuh"
+#include "tma.cuh"
+
+namespace otg {
+
+constexpr int FU_THREADS = 256, FU_WARPS = 8;
+// Rows of a batch for NK vectors per row and thread: up to 16 vectors (256
+// bytes) of entries in a thread's registers.
+__host__ __device__ constexpr int fu_rb(int nk) { return nk > 8 ? 1 : nk > 4 ? 2 : nk > 2 ? 4 : 8; }
+constexpr int FU_RING = 6;  // most chunks in flight per group
+enum { FU_LOG = 0, FU_SCAL = 1, FU_UNB = 2, FU_ABS = 3 };
+// flags that a CTA publishes with its merge
+enum { FU_BAD_ROW = 1, FU_BAD_COL = 2, FU_ABORT = 4 };
+
+template <typename T>
+struct FusedArgs {
+  const T* M; int64_t ldm; int n, m; T c;
+  const T *a, *b, *warm_u, *warm_v;
+  int max_iter, period;
+  double stop_thr;
+  T *u0, *u1, *v0, *v1, *rowc, *fref;   // v0, v1: this CTA's columns of the last two iterates
+  unsigned long long *part, *vll, *stll, *ell;   // published words, see Ll
+  T* pairs;                  // [grid][m] (maximum, sum) pairs: first and fallback column pass
+  T* vfix;                   // [m] v of the fallback column pass
+  T *out_u, *out_v;
+  double* hist; int hist_cap;
+  int* info;                 // status, niter, nchecks, abort
+  unsigned* bar;
+  uint64_t timeout_ns;
+  T fi1, fi2; const T *alw, *bew;
+  // split
+  int G, kv, mp, mv, gvec, NC;
+  int kmat;                  // M holds K = exp(-M/reg) already
+  int buf_elems;             // cross-group buffer
+};
+
+// ---------------------------------------------------------------------------
+// Published values: {value, epoch} in one 64-bit word (float), two such words
+// for the halves of a double.  64-bit accesses are single-copy atomic, so a
+// word with the expected epoch holds the expected value.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void ll_st(unsigned long long* p, unsigned lo, unsigned ep) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" :: "l"(p), "l"(((unsigned long long)ep << 32) | lo) : "memory");
+}
+__device__ __forceinline__ unsigned long long ll_ld(const unsigned long long* p) {
+  unsigned long long x;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(x) : "l"(p) : "memory");
+  return x;
+}
+template <typename T> struct Ll;
+template <> struct Ll<float> {
+  static constexpr int N = 1;  // words per value
+  struct W { unsigned long long w; };
+  static __device__ __forceinline__ void put(unsigned long long* p, float x, unsigned ep) { ll_st(p, __float_as_uint(x), ep); }
+  static __device__ __forceinline__ W get(const unsigned long long* p) { return W{ll_ld(p)}; }
+  static __device__ __forceinline__ bool is(const W& x, unsigned ep) { return (unsigned)(x.w >> 32) == ep; }
+  static __device__ __forceinline__ float value(const W& x) { return __uint_as_float((unsigned)x.w); }
+};
+template <> struct Ll<double> {
+  static constexpr int N = 2;
+  struct W { unsigned long long a, b; };
+  static __device__ __forceinline__ void put(unsigned long long* p, double x, unsigned ep) {
+    const unsigned long long e = (unsigned long long)ep << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};"
+                 :: "l"(p), "l"(e | (unsigned)__double2loint(x)), "l"(e | (unsigned)__double2hiint(x)) : "memory");
+  }
+  static __device__ __forceinline__ W get(const unsigned long long* p) {
+    W x;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(x.a), "=l"(x.b) : "l"(p) : "memory");
+    return x;
+  }
+  static __device__ __forceinline__ bool is(const W& x, unsigned ep) {
+    return (unsigned)(x.a >> 32) == ep && (unsigned)(x.b >> 32) == ep;
+  }
+  static __device__ __forceinline__ double value(const W& x) { return __hiloint2double((int)(unsigned)x.b, (int)(unsigned)x.a); }
+};
+
+// Poll one published value (first read `w` done).  Bounded: after timeout_ns,
+// or when another thread has given up, raises the abort flag and returns
+// false.
+template <typename T>
+__device__ __forceinline__ bool ll_wait(const unsigned long long* p, unsigned ep, typename Ll<T>::W& w, int* abort_flag,
+                                        uint64_t timeout_ns) {
+  if (Ll<T>::is(w, ep)) return true;
+  unsigned spins = 0;
+  uint64_t t0 = 0;
+  for (;;) {
+    w = Ll<T>::get(p);
+    if (Ll<T>::is(w, ep)) return true;
+    if ((++spins & 255u) == 0) {
+      if (ld_acquire_i(abort_flag)) return false;
+      const uint64_t t = globaltimer();
+      if (t0 == 0) t0 = t;
+      else if (t - t0 > timeout_ns) { atomicExch(abort_flag, 1); return false; }
+    }
+  }
+}
+
+template <typename T>
+struct FuSmem { T *vs, *gs, *buf, *data; uint64_t* full; };
+
+struct FuRow {                 // this thread's place
+  int r0, r1;                  // rows of the CTA
+  int ga, gb;                  // rows of its group
+  int live;                    // groups with rows
+  int g, NG, gt, tg, warp, lane;
+};
+
+// Ring state of a group: the chunk to consume next (slot, parity of its full
+// barrier); chunks are numbered on across the passes.
+struct FuRing { int slot; uint32_t phase; };
+
+template <typename T>
+__device__ __forceinline__ void fu_get(const T* p, T (&x)[Vec<T>::N]) {
+  unpack(*reinterpret_cast<const typename Vec<T>::type*>(p), x);
+}
+__device__ __forceinline__ void fu_put(float* p, const float (&x)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+}
+__device__ __forceinline__ void fu_put(double* p, const double (&x)[2]) {
+  *reinterpret_cast<double2*>(p) = make_double2(x[0], x[1]);
+}
+
+// A 16-byte vector in registers: two packed pairs of floats (the packed
+// fp32x2 operations round each lane as the scalar ones), or two doubles.
+template <typename T> struct FuV;
+template <> struct FuV<float> {
+  uint64_t a, b;
+  struct S { uint64_t v; };  // a scalar for both lanes
+  static __device__ __forceinline__ S all(float x) { return S{pack2(x, x)}; }
+  static __device__ __forceinline__ FuV zero() { return FuV{0ull, 0ull}; }
+  static __device__ __forceinline__ FuV lds(uint32_t p) {
+    FuV r;
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "r"(p) : "memory");
+    return r;
+  }
+  static __device__ __forceinline__ uint64_t ex(uint64_t t) {
+    float lo, hi;
+    unpack2(t, lo, hi);
+    return pack2(ex2(lo), ex2(hi));
+  }
+  // this += x * r
+  __device__ __forceinline__ void fma_s(const FuV& x, S r) { a = fma2(x.a, r.v, a); b = fma2(x.b, r.v, b); }
+  // this += x * y
+  __device__ __forceinline__ void fma_v(const FuV& x, const FuV& y) { a = fma2(x.a, y.a, a); b = fma2(x.b, y.b, b); }
+  __device__ __forceinline__ void add_v(const FuV& x) { a = add2(a, x.a); b = add2(b, x.b); }
+  // exp2(x c + v + h)
+  static __device__ __forceinline__ FuV expo(const FuV& x, S c, const FuV& v, S h) {
+    return FuV{ex(add2(fma2(x.a, c.v, v.a), h.v)), ex(add2(fma2(x.b, c.v, v.b), h.v))};
+  }
+  // exp2(x c)
+  static __device__ __forceinline__ FuV gibbs(const FuV& x, S c) { return FuV{ex(mul2(x.a, c.v)), ex(mul2(x.b, c.v))}; }
+  static __device__ __forceinline__ FuV arg(const FuV& x, S c, const FuV& v) { return FuV{fma2(x.a, c.v, v.a), fma2(x.b, c.v, v.b)}; }
+  static __device__ __forceinline__ FuV ex_minus(const FuV& t, float m) {
+    const uint64_t k = pack2(-m, -m);
+    return FuV{ex(add2(t.a, k)), ex(add2(t.b, k))};
+  }
+  __device__ __forceinline__ void get(float (&x)[4]) const { unpack2(a, x[0], x[1]); unpack2(b, x[2], x[3]); }
+  static __device__ __forceinline__ FuV of(const float (&x)[4]) { return FuV{pack2(x[0], x[1]), pack2(x[2], x[3])}; }
+  __device__ __forceinline__ float sum() const { float x[4]; get(x); return (x[0] + x[1]) + (x[2] + x[3]); }
+  __device__ __forceinline__ float max_with(float m) const { float x[4]; get(x); return fmaxf(fmax3(m, x[0], x[1]), fmaxf(x[2], x[3])); }
+};
+template <> struct FuV<double> {
+  double a, b;
+  struct S { double v; };
+  static __device__ __forceinline__ S all(double x) { return S{x}; }
+  static __device__ __forceinline__ FuV zero() { return FuV{0.0, 0.0}; }
+  static __device__ __forceinline__ FuV lds(uint32_t p) {
+    FuV r;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(r.a), "=d"(r.b) : "r"(p) : "memory");
+    return r;
+  }
+  __device__ __forceinline__ void fma_s(const FuV& x, S r) { a = fma(x.a, r.v, a); b = fma(x.b, r.v, b); }
+  __device__ __forceinline__ void fma_v(const FuV& x, const FuV& y) { a = fma(x.a, y.a, a); b = fma(x.b, y.b, b); }
+  __device__ __forceinline__ void add_v(const FuV& x) { a += x.a; b += x.b; }
+  static __device__ __forceinline__ FuV expo(const FuV& x, S c, const FuV& v, S h) {
+    return FuV{ex2(fma(x.a, c.v, v.a) + h.v), ex2(fma(x.b, c.v, v.b) + h.v)};
+  }
+  static __device__ __forceinline__ FuV gibbs(const FuV& x, S c) { return FuV{ex2(x.a * c.v), ex2(x.b * c.v)}; }
+  static __device__ __forceinline__ FuV arg(const FuV& x, S c, const FuV& v) { return FuV{fma(x.a, c.v, v.a), fma(x.b, c.v, v.b)}; }
+  static __device__ __forceinline__ FuV ex_minus(const FuV& t, double m) { return FuV{ex2(t.a - m), ex2(t.b - m)}; }
+  __device__ __forceinline__ void get(double (&x)[2]) const { x[0] = a; x[1] = b; }
+  static __device__ __forceinline__ FuV of(const double (&x)[2]) { return FuV{x[0], x[1]}; }
+  __device__ __forceinline__ double sum() const { return a + b; }
+  __device__ __forceinline__ double max_with(double m) const { return fmax(m, fmax(a, b)); }
+};
+
+// One vector of the cost from global memory; rows that are not whole 16-byte
+// vectors are read element by element, entries beyond the row give `pad`.
+template <typename T>
+__device__ __forceinline__ void fu_get_global(const FusedArgs<T>& A, int row, int col, T pad, T (&x)[Vec<T>::N]) {
+  const T* p = A.M + (int64_t)row * A.ldm + col;
+  if (A.gvec) {
+    unpack(ld_stream(reinterpret_cast<const typename Vec<T>::type*>(p)), x);
+  } else {
+#pragma unroll
+    for (int w = 0; w < Vec<T>::N; ++w) x[w] = col + w < A.m ? __ldg(p + w) : pad;
+  }
+}
+
+// A scaling of FU_ABS that needs no absorption: within [2^-300, 2^300].
+__device__ __forceinline__ bool fu_tame(double x) { return x > 4.9e-91 && x < 2.0e90; }
+
+// ---------------------------------------------------------------------------
+// Ring of the streamed form.  Chunk j of a group's pass is half (j & 1) of
+// row ga + j / 2, mp / 2 elements per slot.  The chunks of the next pass
+// follow those of this one (the cost does not change), so the ring never runs
+// dry over the hand-over.
+// ---------------------------------------------------------------------------
+// Chunk j into `slot`; `rows`: rows of the group, M0: its first one.
+template <typename T>
+__device__ __forceinline__ void fu_issue(const T* M0, int64_t ldm, int mv, int half, int rows, T* slots, uint64_t* full, int j,
+                                         int slot) {
+  const int nch = 2 * rows;
+  while (j >= nch) j -= nch;
+  const int c0 = (j & 1) * half, cols = min(half, mv - c0);
+  if (cols > 0) {
+    mbar_arrive_expect_tx(full + slot, (uint32_t)(cols * (int)sizeof(T)));
+    bulk_g2s(slots + slot * half, M0 + (int64_t)(j >> 1) * ldm + c0, (uint32_t)(cols * (int)sizeof(T)), full + slot);
+  } else {
+    mbar_arrive(full + slot);
+  }
+}
+
+// Wait for a chunk (bounded: false after timeout_ns or an abort elsewhere).
+__device__ __forceinline__ bool fu_landed(uint64_t* bar, uint32_t parity, int* abort_flag, uint64_t timeout_ns) {
+  return mbar_wait(bar, parity, abort_flag, timeout_ns);
+}
+
+// ---------------------------------------------------------------------------
+// Reductions over RB rows at once.  Each lane brings its share of every row;
+// after log2(RB) halving steps and the rest of the butterfly, lane l holds
+// the warp's value of row l / LPR.
+// ---------------------------------------------------------------------------
+template <typename T, bool MAX> __device__ __forceinline__ T fu_op(T a, T b) { return MAX ? fmax(a, b) : a + b; }
+
+template <typename T, int RB, bool MAX>
+__device__ __forceinline__ T fu_scatter(T (&s)[RB], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int h = RB / 2; h >= 1; h /= 2) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const T keep = up ? s[i + h] : s[i], give = up ? s[i] : s[i + h];
+      s[i] = fu_op<T, MAX>(keep, __shfl_xor_sync(0xffffffffu, give, o));
+    }
+    o >>= 1;
+  }
+  T x = s[0];
+#pragma unroll
+  for (int q = 16 / RB; q > 0; q >>= 1) x = fu_op<T, MAX>(x, __shfl_xor_sync(0xffffffffu, x, q));
+  return x;
+}
+
+// ... over the G warps of the group: lane l of every warp gets the group's
+// value of row l / LPR.  The scratch alternates, one barrier per call.
+template <typename T, int RB, bool MAX, int RS>
+__device__ __forceinline__ T fu_group(T (&s)[RB], const FuRow& R, int G, T (*red)[FU_WARPS][RS], int& par) {
+  constexpr int LPR = 32 / RB;
+  T x = fu_scatter<T, RB, MAX>(s, R.lane);
+  if (G == 1) return x;
+  const int row = R.lane / LPR, l = R.lane % LPR, w0 = R.g * G;
+  if (l == 0) red[par][R.warp][row] = x;
+  named_bar(1 + R.g, R.gt);
+  T t = MAX ? T(-INFINITY) : T(0);
+  for (int q = l; q < G; q += LPR) t = fu_op<T, MAX>(t, red[par][w0 + q][row]);
+#pragma unroll
+  for (int q = LPR / 2; q > 0; q >>= 1) t = fu_op<T, MAX>(t, __shfl_xor_sync(0xffffffffu, t, q));
+  par ^= 1;
+  return t;
+}
+
+// Column sums of the CTA, over the row groups in group order, to its slot.
+template <typename T, int NK>
+__device__ __forceinline__ void fu_publish_cols(const FusedArgs<T>& A, const FuRow& R, const FuSmem<T>& sm,
+                                                const FuV<T> (&acc)[NK], unsigned ep) {
+  constexpr int W = Vec<T>::N;
+  unsigned long long* dst = A.part + (int64_t)blockIdx.x * A.m * Ll<T>::N;
+  if (R.NG == 1) {
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      const int col = (k * R.gt + R.tg) * W;
+      T x[W];
+      acc[k].get(x);
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        if (col + w < A.m) Ll<T>::put(dst + (col + w) * Ll<T>::N, x[w], ep);
+    }
+    return;
+  }
+  if (R.g < R.live) {
+    T* b = sm.buf + (int64_t)R.g * A.mp;
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      T x[W];
+      acc[k].get(x);
+      if (k < A.kv) fu_put(b + (k * R.gt + R.tg) * W, x);
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < A.m; j += FU_THREADS) {
+    T t = 0;
+#pragma unroll 4
+    for (int g = 0; g < R.live; ++g) t += sm.buf[g * A.mp + j];
+    Ll<T>::put(dst + j * Ll<T>::N, t, ep);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// One pass over the CTA's rows: row updates with sm.vs, scaled entries into
+// the CTA's column sums.  q0, q1, q2: scalars of the group's rows, lane l of
+// a warp holding row 32 k + l (reloaded every 32 rows unless `held`).
+// ---------------------------------------------------------------------------
+template <typename T> struct FuHeld { T q0, q1, q2; };
+
+template <typename T, int MODE>
+__device__ __forceinline__ void fu_fetch(const FusedArgs<T>& A, int row, int end, const T* ucur, FuHeld<T>& H) {
+  if (row >= end) return;
+  if (MODE == FU_LOG) { H.q0 = __ldcg(ucur + row); H.q1 = A.rowc[row]; H.q2 = A.a[row]; }
+  if (MODE == FU_SCAL) H.q1 = A.rowc[row];
+  if (MODE == FU_ABS) H.q1 = A.a[row];
+  if (MODE == FU_UNB) { H.q0 = __ldcg(ucur + row); H.q1 = A.a[row]; H.q2 = A.alw ? A.alw[row] : T(1); }
+}
+
+template <typename T> struct FuTrack { T d0, d1, d2; };
+
+// Row values of a batch from the warps' shares s[]: lane l finishes row
+// l / LPR; r is what the row's entries are scaled with in the column sums.
+template <typename T, int MODE, int RB, int NK>
+__device__ __forceinline__ void fu_rows(const FusedArgs<T>& A, const FuRow& R, T (*red)[FU_WARPS][fu_rb(NK)], T (*rr)[2][fu_rb(NK)],
+                                        int& par, T (&s)[RB], int nr, const FuHeld<T>& H, int at, T& t, T& un, T& r, int& flag,
+                                        FuTrack<T>& tr) {
+  constexpr int LPR = 32 / RB;
+  const int myrow = R.lane / LPR, src = at + myrow;
+  const T p0 = __shfl_sync(0xffffffffu, H.q0, src), p1 = __shfl_sync(0xffffffffu, H.q1, src),
+          p2 = __shfl_sync(0xffffffffu, H.q2, src);
+  // FP64 issues at two lanes per clock: the group's first warp alone adds
+  // the warps' sums and divides (the log form needs the sum everywhere)
+  const bool first_only = sizeof(T) == 8 && MODE != FU_LOG && A.G > 1;
+  if (first_only) {
+    const T x = fu_scatter<T, RB, false>(s, R.lane);
+    if (R.lane % LPR == 0) red[par][R.warp][myrow] = x;
+    named_bar(1 + R.g, R.gt);
+  } else {
+    t = fu_group<T, RB, false>(s, R, A.G, red, par);
+  }
+  if (!first_only || R.tg < 32) {
+    if (first_only) {
+      const int l = R.lane % LPR, w0 = R.g * A.G;
+      t = 0;
+      for (int q = l; q < A.G; q += LPR) t += red[par][w0 + q][myrow];
+#pragma unroll
+      for (int q = LPR / 2; q > 0; q >>= 1) t += __shfl_xor_sync(0xffffffffu, t, q);
+    }
+    if (MODE == FU_LOG) {
+      un = p0 - lg2(t);
+      r = p2 / t;
+    } else if (MODE == FU_SCAL) {
+      r = un = T(1) / (p1 * t);
+      if (myrow < nr && !isfinite(un)) flag = FU_BAD_ROW;
+    } else if (MODE == FU_ABS) {
+      r = un = p1 == T(0) ? T(1) : p1 / t;
+      if (myrow < nr && !fu_tame(un)) flag = FU_BAD_ROW;
+    } else {
+      un = pow(p1 / (p2 * t), A.fi1);
+      if (myrow < nr) {
+        if (!isfinite(un)) flag = FU_BAD_ROW;
+        tr.d0 = fmax(tr.d0, fabs(un - p0)); tr.d1 = fmax(tr.d1, fabs(un)); tr.d2 = fmax(tr.d2, fabs(p0));
+      }
+      r = p2 * un;
+    }
+  }
+  if (first_only) {
+    if (R.tg < 32 && R.lane % LPR == 0) { rr[R.g][0][myrow] = r; rr[R.g][1][myrow] = un; }
+    named_bar(1 + R.g, R.gt);
+    r = rr[R.g][0][myrow];
+    un = rr[R.g][1][myrow];
+    par ^= 1;
+  }
+}
+
+// Running-maximum form of a batch (log form): maxima, then sums of e.
+template <typename T, int NK, int RB, typename Arg>
+__device__ __forceinline__ void fu_rows_max(const FusedArgs<T>& A, const FuRow& R, T (*red)[FU_WARPS][fu_rb(NK)], int& par, int nr,
+                                            FuV<T> (&e)[RB][NK], const FuHeld<T>& H, int at, T& un, T& r, Arg&& arg) {
+  constexpr int LPR = 32 / RB;
+  T mx[RB], s[RB];
+#pragma unroll
+  for (int q = 0; q < RB; ++q) mx[q] = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+#pragma unroll
+    for (int q = 0; q < RB; ++q)
+      if (q < nr) { e[q][k] = arg(q, k); mx[q] = e[q][k].max_with(mx[q]); }
+  }
+  const T mg = fu_group<T, RB, true>(mx, R, A.G, red, par);
+#pragma unroll
+  for (int q = 0; q < RB; ++q) {
+    const T m = __shfl_sync(0xffffffffu, mg, q * LPR);
+    FuV<T> t = FuV<T>::zero();
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (q < nr) { e[q][k] = FuV<T>::ex_minus(e[q][k], m); t.add_v(e[q][k]); }
+    s[q] = t.sum();
+  }
+  const T t = fu_group<T, RB, false>(s, R, A.G, red, par);
+  const int src = at + R.lane / LPR;
+  const T p1 = __shfl_sync(0xffffffffu, H.q1, src), p2 = __shfl_sync(0xffffffffu, H.q2, src);
+  un = p1 - lse_value(mg, t);
+  r = p2 / t;
+}
+
+template <typename T>
+__device__ __forceinline__ bool fu_near_one(T t) { return t >= T(9.313225746154785e-10) && t <= T(1073741824.0); }  // 2^-30, 2^30
+
+// New row values into memory and into the lane that holds them.
+template <typename T, int MODE, int RB>
+__device__ __forceinline__ void fu_keep(const FuRow& R, int rb, int at, int nr, T un, T* unxt, FuHeld<T>& H) {
+  constexpr int LPR = 32 / RB;
+  const int myrow = R.lane / LPR;
+  if (R.tg < 32 && R.lane % LPR == 0 && myrow < nr) unxt[rb + myrow] = un;
+  if (MODE == FU_LOG || MODE == FU_UNB) {
+    const int mine = R.lane - at;
+    const T x = __shfl_sync(0xffffffffu, un, (mine >= 0 && mine < RB ? mine : 0) * LPR);
+    if (mine >= 0 && mine < nr) H.q0 = x;
+  }
+}
+
+// RB rows at a time, from shared memory (RES) or the ring.
+template <typename T, int MODE, int NK, bool RES>
+__device__ __forceinline__ int fu_pass(const FusedArgs<T>& A, const FuRow& R_, const FuSmem<T>& sm,
+                                       T (*red)[FU_WARPS][fu_rb(NK)], T (*rr)[2][fu_rb(NK)], FuRing& ring_, const T* ucur, T* unxt,
+                                       FuHeld<T>& H_, bool held, FuTrack<T>& tr_, unsigned ep) {
+  using V = FuV<T>;
+  constexpr int RB = fu_rb(NK), LPR = 32 / RB;
+  static_assert(RES || RB == 1, "streamed rows go one at a time");
+  // (copies: what the loop reads stays in registers across the inline assembly)
+  const FuRow R = R_;
+  FuRing ring = ring_;
+  FuHeld<T> H = H_;
+  FuTrack<T> tr = tr_;
+  V acc[NK];
+#pragma unroll
+  for (int k = 0; k < NK; ++k) acc[k] = V::zero();
+  const int kv = A.kv, nc = A.NC, mp = A.mp;
+  const uint32_t hop = (uint32_t)R.gt * 16u, pitch = (uint32_t)mp * (uint32_t)sizeof(T);
+  const uint32_t va = smem_addr(sm.vs) + (uint32_t)R.tg * 16u;
+  const uint32_t chunk = pitch / 2;
+  uint32_t xa = smem_addr(sm.data) + (uint32_t)R.tg * 16u;
+  if (RES) xa += (uint32_t)(R.ga - R.r0) * pitch;
+  else xa += (uint32_t)(R.g * nc) * chunk;
+  const typename V::S c = V::all(A.c);
+  const bool kmat = A.kmat != 0;
+  const int G = A.G, mv = A.mv;
+  const T* const Mg = A.M + (int64_t)R.ga * A.ldm;
+  const int64_t ldm = A.ldm;
+  uint64_t* const full = sm.full + R.g * nc;
+  T* const rslot = sm.data + R.g * nc * (mp / 2);
+  int par = 0, flag = 0;
+  for (int rb = R.ga; rb < R.gb; rb += RB) {
+    const int at = (rb - R.ga) & 31;
+    if (!held && at == 0) fu_fetch<T, MODE>(A, rb + R.lane, R.gb, ucur, H);
+    const int nr = min(RB, R.gb - rb);
+    V e[RB][NK];
+    T s[RB];
+    // The loads and exponentials of a batch stand in one block of code: a
+    // branch per vector or row would expose the latency of each (measured
+    // 1.4 times slower).  Rows beyond the batch read its last row again;
+    // nothing comes of their values.
+    auto eval = [&](auto nq) {
+#pragma unroll
+      for (int q = 0; q < decltype(nq)::value; ++q) {
+        const uint32_t xq = xa + min(q, nr - 1) * pitch;
+        const typename V::S h = V::all(MODE == FU_LOG ? __shfl_sync(0xffffffffu, H.q0 - H.q1, at + q) : T(0));
+        V t = V::zero();
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+          const V v = V::lds(va + k * hop), x = V::lds(xq + k * hop);
+          if (MODE == FU_LOG) { e[q][k] = V::expo(x, c, v, h); t.add_v(e[q][k]); }
+          else { e[q][k] = x; t.fma_v(x, v); }
+        }
+        s[q] = t.sum();
+      }
+    };
+    if (!RES) {
+      // the two halves of the row, each as it lands
+      const typename V::S h = V::all(MODE == FU_LOG ? __shfl_sync(0xffffffffu, H.q0 - H.q1, at) : T(0));
+      V t = V::zero();
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const uint32_t xc = xa + (uint32_t)ring.slot * chunk, vc = va + half * (NK / 2) * hop;
+        if (!fu_landed(full + ring.slot, ring.phase, A.info + 3, A.timeout_ns)) flag |= FU_ABORT;
+        if (half == 0 || kv > NK / 2) {
+#pragma unroll
+          for (int kk = 0; kk < NK / 2; ++kk) {
+            const int k = half * (NK / 2) + kk;
+            const V v = V::lds(vc + kk * hop), x = V::lds(xc + kk * hop);
+            if (MODE == FU_LOG) { e[0][k] = V::expo(x, c, v, h); t.add_v(e[0][k]); }
+            else { e[0][k] = kmat ? x : V::gibbs(x, c); t.fma_v(e[0][k], v); }
+          }
+        } else {
+#pragma unroll
+          for (int kk = 0; kk < NK / 2; ++kk) e[0][half * (NK / 2) + kk] = V::zero();
+        }
+        if (++ring.slot == nc) { ring.slot = 0; ring.phase ^= 1; }
+      }
+      s[0] = t.sum();
+    } else if (RB > 1 && nr <= RB / 2) {
+      eval(std::integral_constant<int, (RB > 1 ? RB / 2 : 1)>{});
+#pragma unroll
+      for (int q = RB / 2; q < RB; ++q) s[q] = 0;
+    } else {
+      eval(std::integral_constant<int, RB>{});
+    }
+    T t, un, r;
+    fu_rows<T, MODE, RB, NK>(A, R, red, rr, par, s, nr, H, at, t, un, r, flag, tr);
+    if (MODE == FU_LOG) {
+      // (the same in every warp of the group)
+      if (!__all_sync(0xffffffffu, R.lane / LPR >= nr || fu_near_one(t)))
+        fu_rows_max<T, NK, RB>(A, R, red, par, nr, e, H, at, un, r, [&](int q, int k) {
+          uint32_t xk = xa + q * pitch + k * hop;
+          if (!RES) {
+            int sl = ring.slot - (k < NK / 2 ? 2 : 1);  // the row's chunks are still in their slots
+            if (sl < 0) sl += nc;
+            xk = xa + (uint32_t)sl * chunk + (k % (NK / 2 > 0 ? NK / 2 : 1)) * hop;
+          }
+          return V::arg(V::lds(xk), c, V::lds(va + k * hop));
+        });
+    }
+    if (!RES && R.tg < 32) {
+      // every warp of the group has read the two chunks (the reductions'
+      // barriers): their slots take the chunks NC places on
+      __syncwarp();
+      int s1 = ring.slot - 1;
+      if (s1 < 0) s1 += nc;
+      const int s0 = s1 == 0 ? nc - 1 : s1 - 1;
+      if (R.lane == 0) {
+        const int j = 2 * (rb - R.ga) + nc;
+        fu_issue(Mg, ldm, mv, mp / 2, R.gb - R.ga, rslot, full, j, s0);
+        fu_issue(Mg, ldm, mv, mp / 2, R.gb - R.ga, rslot, full, j + 1, s1);
+      }
+    }
+    fu_keep<T, MODE, RB>(R, rb, at, nr, un, unxt, H);
+#pragma unroll
+    for (int q = 0; q < RB; ++q) {
+      if (q < nr) {
+        const typename V::S rq = V::all(__shfl_sync(0xffffffffu, r, q * LPR));
+#pragma unroll
+        for (int k = 0; k < NK; ++k)
+          acc[k].fma_s(e[q][k], rq);
+      }
+    }
+    if (RES) xa += RB * pitch;
+  }
+  ring_ = ring;
+  H_ = H;
+  if (MODE == FU_UNB) tr_ = tr;
+  fu_publish_cols<T, NK>(A, R, sm, acc, ep);
+  return flag;
+}
+
+// Absorbing pass of FU_ABS: rows of K = exp(x + f + g) with f the exact row
+// update of g = sm.gs (running maximum), f into fref, scalings one; K into
+// the resident rows.
+template <typename T, int NK>
+__device__ __noinline__ void fu_build(const FusedArgs<T>& A, const FuRow& R, const FuSmem<T>& sm, T (*red)[FU_WARPS][fu_rb(NK)],
+                                      T* unxt, unsigned ep) {
+  constexpr int W = Vec<T>::N;
+  const T pad = A.c > T(0) ? T(-INFINITY) : T(INFINITY);
+  FuV<T> acc[NK];
+#pragma unroll
+  for (int k = 0; k < NK; ++k) acc[k] = FuV<T>::zero();
+  int par = 0;
+  for (int row = R.ga; row < R.gb; ++row) {
+    T e[NK][W];
+    T one[1] = {T(-INFINITY)};
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      const int col = (k * R.gt + R.tg) * W;
+      if (k < A.kv) {
+        T x[W], v[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) x[w] = pad;
+        if (col < A.mv) fu_get_global(A, row, col, pad, x);
+        fu_get(sm.gs + col, v);
+#pragma unroll
+        for (int w = 0; w < W; ++w) { e[k][w] = fma(x[w], A.c, v[w]); one[0] = fmax(one[0], e[k][w]); }
+      }
+    }
+    const T mx = fu_group<T, 1, true>(one, R, A.G, red, par);
+    one[0] = 0;
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      if (k < A.kv) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) { e[k][w] = ex2(e[k][w] - mx); one[0] += e[k][w]; }
+      }
+    }
+    const T s = fu_group<T, 1, false>(one, R, A.G, red, par);
+    const T r = A.a[row] / s;
+    T* ks = sm.data + (row - R.r0) * A.mp;
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      if (k < A.kv) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) e[k][w] *= r;
+        acc[k].add_v(FuV<T>::of(e[k]));
+        fu_put(ks + (k * R.gt + R.tg) * W, e[k]);
+      }
+    }
+    if (R.tg == 0) {
+      A.fref[row] = A.rowc[row] - lse_value(mx, s);
+      unxt[row] = T(1);
+    }
+  }
+  fu_publish_cols<T, NK>(A, R, sm, acc, ep);
+}
+
+// Column sums alone (scaling forms, first iteration): sum_i K_ij u_i.
+template <typename T, int NK, bool RES>
+__device__ __noinline__ void fu_colsum(const FusedArgs<T>& A, const FuRow& R, const FuSmem<T>& sm, const T* u, unsigned ep) {
+  constexpr int W = Vec<T>::N;
+  FuV<T> acc[NK];
+#pragma unroll
+  for (int k = 0; k < NK; ++k) acc[k] = FuV<T>::zero();
+  const T c = A.c;
+  for (int row = R.ga; row < R.gb; row += 2) {
+    // two rows' loads in flight
+    T x[2][NK][W], ui[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int r = min(row + q, R.gb - 1);
+      ui[q] = row + q < R.gb ? __ldcg(u + r) : T(0);
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        const int col = (k * R.gt + R.tg) * W;
+        if (RES) { if (k < A.kv) fu_get(sm.data + (r - R.r0) * A.mp + col, x[q][k]); }
+        else fu_get_global(A, r, col < A.mv ? col : 0, T(0), x[q][k]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int k = 0; k < NK; ++k)
+        if (!RES || k < A.kv) {
+          const FuV<T> xv = FuV<T>::of(x[q][k]);
+          acc[k].fma_s(RES || A.kmat ? xv : FuV<T>::gibbs(xv, FuV<T>::all(c)), FuV<T>::all(ui[q]));
+        }
+  }
+  fu_publish_cols<T, NK>(A, R, sm, acc, ep);
+}
+
+// Column log-sum-exps alone (log forms: first iteration and the fallback):
+// (maximum, sum) pairs of x_ij + u_i over the CTA's rows, four vectors of a
+// thread at a time.
+template <typename T, bool TILE>
+__device__ __noinline__ void fu_collse(const FusedArgs<T>& A_, const FuRow& R_, const FuSmem<T>& sm_, const T* u) {
+  constexpr int W = Vec<T>::N, KB = 4;
+  const FusedArgs<T> A = A_;
+  const FuRow R = R_;
+  const FuSmem<T> sm = sm_;
+  const T pad = A.c > T(0) ? T(-INFINITY) : T(INFINITY);
+  for (int k0 = 0; k0 < A.kv; k0 += KB) {
+    T mx[KB][W], s[KB][W];
+#pragma unroll
+    for (int k = 0; k < KB; ++k)
+#pragma unroll
+      for (int w = 0; w < W; ++w) { mx[k][w] = -INFINITY; s[k][w] = 0; }
+    // four rows per update: one rescaling exponential for them
+    for (int row = R.ga; row < R.gb; row += 4) {
+      T ui[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ui[q] = row + q < R.gb ? __ldcg(u + row + q) : T(-INFINITY);
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        const int col = ((k0 + k) * R.gt + R.tg) * W;
+        if (col < A.mv && k0 + k < A.kv) {
+          T x[4][W];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int r = min(row + q, R.gb - 1);
+            if (TILE) fu_get(sm.data + (r - R.r0) * A.mp + col, x[q]);
+            else fu_get_global(A, r, col, pad, x[q]);
+          }
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            T t[4], top = mx[k][w];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { t[q] = row + q < R.gb ? fma(x[q][w], A.c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
+            if (top != -INFINITY) {
+              T sum = s[k][w] * ex2(mx[k][w] - top);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) sum += ex2(t[q] - top);
+              s[k][w] = sum;
+              mx[k][w] = top;
+            }
+          }
+        }
+      }
+    }
+    // over the row groups: the largest maximum first, then the rescaled sums
+    // (a group without rows brings empty pairs)
+    if (R.NG > 1) {
+      T* b = sm.buf + R.g * A.mp;
+#pragma unroll
+      for (int k = 0; k < KB; ++k)
+        if (k0 + k < A.kv) fu_put(b + ((k0 + k) * R.gt + R.tg) * W, mx[k]);
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        const int col = ((k0 + k) * R.gt + R.tg) * W;
+        if (k0 + k < A.kv) {
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            T top = -INFINITY;
+            for (int g = 0; g < R.NG; ++g) top = fmax(top, sm.buf[g * A.mp + col + w]);
+            if (top != -INFINITY) s[k][w] *= ex2(mx[k][w] - top);
+            mx[k][w] = top;
+          }
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < KB; ++k)
+        if (k0 + k < A.kv) fu_put(b + ((k0 + k) * R.gt + R.tg) * W, s[k]);
+      __syncthreads();
+    }
+    if (R.g == 0) {
+      T* dst = A.pairs + 2 * (int64_t)blockIdx.x * A.m;
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        const int col = ((k0 + k) * R.gt + R.tg) * W;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          if (k0 + k < A.kv && col + w < A.m) {
+            T t = s[k][w];
+            if (R.NG > 1) {
+              t = 0;
+              for (int g = 0; g < R.NG; ++g) t += sm.buf[g * A.mp + col + w];
+            }
+            dst[2 * (col + w)] = mx[k][w];
+            dst[2 * (col + w) + 1] = t;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Merge: this CTA's share of the columns over the grid's slots.  LC lanes
+// take adjacent columns and 32 / LC lanes share a column's slots, as do `per`
+// warps; partial sums are added in lane and warp order, so the sum of a
+// column is the same in every run.  fin(j, mx, s) finishes column j.
+// ---------------------------------------------------------------------------
+template <typename T, bool PAIRS, typename Fin>
+__device__ __forceinline__ bool fu_merge(const FusedArgs<T>& A, const FuRow& R, T* s_s, T* s_m, unsigned ep, Fin&& fin) {
+  const int np = gridDim.x;
+  const int cb = (int)((int64_t)A.m * blockIdx.x / gridDim.x), ce = (int)((int64_t)A.m * (blockIdx.x + 1) / gridDim.x);
+  const int mc = ce - cb;
+  int LC = 32;
+  if (!PAIRS) while (LC > 4 && LC / 2 >= mc) LC /= 2;
+  const int SL = 32 / LC, ncb = (mc + LC - 1) / LC;
+  const int per = ncb >= FU_WARPS ? 1 : (ncb ? FU_WARPS / ncb : 1);
+  const int at_once = FU_WARPS / per;
+  const int sub = R.warp % per, mine = R.warp / per;
+  const int step = per * SL;
+  bool ok = true;
+  for (int b0 = 0; b0 < ncb; b0 += at_once) {
+    const int blk = b0 + mine;
+    const int j = cb + blk * LC + R.lane % LC;
+    const bool live = mine < at_once && blk < ncb && j < ce;
+    T mx = -INFINITY, s = 0;
+    if (live) {
+      if (PAIRS) {
+        for (int p = sub; p < np; p += per) {
+          const T* q = A.pairs + 2 * ((int64_t)p * A.m + j);
+          lse_merge(mx, s, __ldcg(q), __ldcg(q + 1));
+        }
+      } else {
+        constexpr int U = sizeof(T) == 8 ? 4 : 8;
+        const int64_t stride = (int64_t)step * A.m * Ll<T>::N;
+        int p = sub * SL + R.lane / LC;
+        const unsigned long long* q = A.part + ((int64_t)p * A.m + j) * Ll<T>::N;
+        for (; p < np; p += U * step, q += U * stride) {
+          typename Ll<T>::W x[U];
+#pragma unroll
+          for (int k = 0; k < U; ++k)
+            if (p + k * step < np) x[k] = Ll<T>::get(q + k * stride);
+#pragma unroll
+          for (int k = 0; k < U; ++k)
+            if (p + k * step < np) {
+              ok = ok && ll_wait<T>(q + k * stride, ep, x[k], A.info + 3, A.timeout_ns);
+              s += Ll<T>::value(x[k]);
+            }
+        }
+      }
+    }
+    if (!PAIRS) {
+      __syncwarp();
+      for (int o = LC; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+    if (per > 1) {
+      s_s[R.warp * 32 + R.lane] = s;
+      if (PAIRS) s_m[R.warp * 32 + R.lane] = mx;
+      __syncthreads();
+      if (live && sub == 0 && R.lane < LC) {
+        for (int q = 1; q < per; ++q) {
+          if (PAIRS) lse_merge(mx, s, s_m[(R.warp + q) * 32 + R.lane], s_s[(R.warp + q) * 32 + R.lane]);
+          else s += s_s[(R.warp + q) * 32 + R.lane];
+        }
+      }
+      __syncthreads();
+    }
+    if (live && sub == 0 && R.lane < LC) fin(j, mx, s);
+  }
+  return ok;
+}
+
+// Grid barrier (start, first and fallback column pass) with one counter that
+// only grows (the launch's control block starts at zero).  Bounded.
+__device__ __forceinline__ bool fu_barrier(unsigned* bar, unsigned& gen, int* abort_flag, uint64_t timeout_ns) {
+  __shared__ int s_ok;
+  __syncthreads();
+  gen += gridDim.x;
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    __threadfence();
+    atomicAdd(bar, 1u);
+    if ((int)(ld_acquire(bar) - gen) < 0) {
+      const uint64_t t0 = globaltimer();
+      unsigned spins = 0;
+      while ((int)(ld_acquire(bar) - gen) < 0) {
+        if ((++spins & 255u) == 0) {
+          if (ld_acquire_i(abort_flag)) { ok = 0; break; }
+          if (globaltimer() - t0 > timeout_ns) { atomicExch(abort_flag, 1); ok = 0; break; }
+        }
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// The whole v of epoch `ep` into sm.vs (poll), the flags that the CTAs
+// published with it, and with `check` their error shares added in CTA order.
+// Every thread gets the same flags and error.
+template <typename T>
+__device__ __forceinline__ int fu_collect(const FusedArgs<T>& A, const FuSmem<T>& sm, unsigned ep, bool check, bool ok,
+                                          double& e2) {
+  int bits = ok ? 0 : FU_ABORT;
+  constexpr int U = 4;
+  for (int j = threadIdx.x; j < A.m; j += U * FU_THREADS) {
+    typename Ll<T>::W x[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (j + k * FU_THREADS < A.m) x[k] = Ll<T>::get(A.vll + (j + k * FU_THREADS) * Ll<T>::N);
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (j + k * FU_THREADS < A.m) {
+        if (!bits && !ll_wait<T>(A.vll + (j + k * FU_THREADS) * Ll<T>::N, ep, x[k], A.info + 3, A.timeout_ns)) bits = FU_ABORT;
+        sm.vs[j + k * FU_THREADS] = Ll<T>::value(x[k]);
+      }
+  }
+  double share = 0.0;
+  for (int p = threadIdx.x; p < (int)gridDim.x; p += FU_THREADS) {
+    Ll<float>::W st = Ll<float>::get(A.stll + p);
+    if (!(bits & FU_ABORT) && !ll_wait<float>(A.stll + p, ep, st, A.info + 3, A.timeout_ns)) bits = FU_ABORT;
+    if (!(bits & FU_ABORT)) bits |= (int)(unsigned)st.w;
+    if (check) {
+      Ll<double>::W w = Ll<double>::get(A.ell + 2 * p);
+      if (!(bits & FU_ABORT) && !ll_wait<double>(A.ell + 2 * p, ep, w, A.info + 3, A.timeout_ns)) bits |= FU_ABORT;
+      share += Ll<double>::value(w);
+    }
+  }
+  int all = 0;
+  if (__syncthreads_or(bits)) {
+    if (__syncthreads_or(bits & FU_BAD_ROW)) all |= FU_BAD_ROW;
+    if (__syncthreads_or(bits & FU_BAD_COL)) all |= FU_BAD_COL;
+    if (__syncthreads_or(bits & FU_ABORT)) all |= FU_ABORT;
+  }
+  if (check) e2 = block_sum_fixed(share);
+  return all;
+}
+
+template <typename T, int MODE, int NK, bool RES>
+__global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __grid_constant__ FusedArgs<T> A) {
+  extern __shared__ __align__(16) unsigned char fu_smem[];
+  __shared__ T red[2][FU_WARPS][fu_rb(NK)];
+  __shared__ T rr[FU_WARPS][2][fu_rb(NK)];
+  __shared__ T s_s[FU_WARPS * 32];
+  constexpr int W = Vec<T>::N;
+  constexpr bool LOGF = MODE == FU_LOG || MODE == FU_ABS;
+  FuRow R;
+  R.r0 = (int)((int64_t)A.n * blockIdx.x / gridDim.x);
+  R.r1 = (int)((int64_t)A.n * (blockIdx.x + 1) / gridDim.x);
+  R.warp = threadIdx.x >> 5;
+  R.lane = threadIdx.x & 31;
+  R.NG = FU_WARPS / A.G;
+  R.g = R.warp / A.G;
+  R.gt = A.G * 32;
+  R.tg = threadIdx.x - R.g * R.gt;
+  {
+    // rows per group; float64: whole batches, as a reduction costs the same
+    // FP64 operations for one row as for a batch
+    constexpr int RB = fu_rb(NK);
+    const int rows = R.r1 - R.r0;
+    int per = (rows + R.NG - 1) / R.NG;
+    if (sizeof(T) == 8) per = (per + RB - 1) / RB * RB;
+    R.live = (rows + per - 1) / per;
+    R.ga = min(R.r1, R.r0 + per * R.g);
+    R.gb = min(R.r1, R.ga + per);
+  }
+  FuSmem<T> sm;
+  sm.vs = reinterpret_cast<T*>(fu_smem);
+  sm.gs = sm.vs + (MODE == FU_ABS ? A.mp : 0);
+  sm.buf = sm.gs + A.mp;
+  sm.full = reinterpret_cast<uint64_t*>(sm.buf + A.buf_elems);  // streamed: NG x NC barriers
+  sm.data = reinterpret_cast<T*>(sm.full + (RES ? 0 : (R.NG * A.NC + 1) / 2 * 2));
+  T* s_m = R.NG > 1 ? sm.buf : sm.vs;  // maxima of the pairs merge (free then: the next v overwrites vs)
+  int* abort_flag = A.info + 3;
+  unsigned gen = 0;
+  const T L2E = T(OTG_LOG2E), LN2 = T(OTG_LN2);
+  const int cb = (int)((int64_t)A.m * blockIdx.x / gridDim.x), ce = (int)((int64_t)A.m * (blockIdx.x + 1) / gridDim.x);
+
+  // initial state: this CTA's rows, its share of the columns, its published words
+  for (int i = R.r0 + threadIdx.x; i < R.r1; i += FU_THREADS) {
+    if (MODE == FU_LOG) { A.u0[i] = A.warm_u ? A.warm_u[i] * L2E : T(0); A.rowc[i] = lg2(A.a[i]); }
+    if (MODE == FU_ABS) { A.fref[i] = A.warm_u ? A.warm_u[i] * L2E : T(0); A.u0[i] = T(1); A.rowc[i] = lg2(A.a[i]); }
+    if (MODE == FU_SCAL) { A.u0[i] = A.warm_u ? exp(A.warm_u[i]) : T(1) / T(A.n); A.rowc[i] = T(1) / A.a[i]; }
+    if (MODE == FU_UNB) A.u0[i] = A.warm_u ? exp(A.warm_u[i]) : T(1);
+  }
+  for (int j = cb + threadIdx.x; j < ce; j += FU_THREADS) {
+    // iteration -1: what a solve that stops before its first iterate returns
+    if (LOGF) A.v1[j] = A.warm_v ? A.warm_v[j] * L2E : T(0);
+    if (MODE == FU_SCAL) A.v1[j] = A.warm_v ? exp(A.warm_v[j]) : T(1) / T(A.m);
+    if (MODE == FU_UNB) A.v1[j] = A.warm_v ? exp(A.warm_v[j]) : T(1);
+    for (int w = 0; w < Ll<T>::N; ++w) A.vll[j * Ll<T>::N + w] = 0ull;
+  }
+  for (int j = threadIdx.x; j < A.m * Ll<T>::N; j += FU_THREADS) A.part[(int64_t)blockIdx.x * A.m * Ll<T>::N + j] = 0ull;
+  if (threadIdx.x < 12) A.ell[(int64_t)12 * blockIdx.x + threadIdx.x] = 0ull;
+  if (threadIdx.x == 0) A.stll[blockIdx.x] = 0ull;
+  // beyond the row: v that adds nothing
+  const T vpad = MODE == FU_LOG ? T(-INFINITY) : T(0);
+  for (int j = threadIdx.x; j < A.mp; j += FU_THREADS) { if (MODE == FU_ABS) sm.gs[j] = 0; sm.vs[j] = vpad; }
+  // resident rows: every thread loads the vectors that it will read
+  if (RES && MODE != FU_ABS) {
+    const T pad = MODE != FU_LOG ? T(0) : (A.c > T(0) ? T(-INFINITY) : T(INFINITY));
+    for (int row = R.ga; row < R.gb; ++row) {
+      T* dst = sm.data + (row - R.r0) * A.mp;
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        const int col = (k * R.gt + R.tg) * W;
+        if (k < A.kv) {
+          T x[W];
+#pragma unroll
+          for (int w = 0; w < W; ++w) x[w] = pad;
+          if (col < A.mv) fu_get_global(A, row, col, pad, x);
+          if (MODE != FU_LOG && !A.kmat) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) x[w] = col + w < A.m ? ex2(x[w] * A.c) : T(0);
+          }
+          fu_put(dst + col, x);
+        }
+      }
+    }
+  }
+  // the ring: zeros beyond the rows (the copies never write there)
+  FuRing ring{0, 0u};
+  if (!RES) {
+    const int chunk = A.mp / 2;
+    for (int j = threadIdx.x; j < R.NG * A.NC * chunk; j += FU_THREADS) sm.data[j] = T(0);
+    for (int j = threadIdx.x; j < R.NG * A.NC; j += FU_THREADS) mbar_init(sm.full + j, 1);
+    fence_mbar_init();
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (R.tg == 0 && R.gb > R.ga)
+      for (int q = 0; q < A.NC; ++q)
+        fu_issue(A.M + (int64_t)R.ga * A.ldm, A.ldm, A.mv, A.mp / 2, R.gb - R.ga, sm.data + R.g * A.NC * (A.mp / 2),
+                 sm.full + R.g * A.NC, q, q);
+  }
+  bool ok = fu_barrier(A.bar, gen, abort_flag, A.timeout_ns);  // the published words are cleared everywhere
+
+  // u, v of the last two iterates (v: this CTA's columns): ucur, vcur are
+  // iteration ii - 1 at the head of the loop
+  T *ucur = A.u0, *unxt = A.u1;
+  T *vcur = A.v1, *vnxt = A.v0;
+  int nchk = 0, status = OTG_STATUS_MAXITER, niter = A.max_iter - 1;
+  double e2 = 0.0;
+  FuHeld<T> H{T(0), T(0), T(0)};
+  const bool held = R.gb - R.ga <= 32;
+  if (held) fu_fetch<T, MODE>(A, R.ga + R.lane, R.gb, ucur, H);
+
+  if (MODE == FU_UNB) {
+    for (int j = threadIdx.x; j < A.m; j += FU_THREADS)
+      sm.vs[j] = (A.bew ? A.bew[j] : T(1)) * (A.warm_v ? exp(A.warm_v[j]) : T(1));
+    __syncthreads();
+    __shared__ T s_mx[6][FU_WARPS];
+    for (int ii = 0; ok && ii < A.max_iter; ++ii) {
+      const unsigned ep = (unsigned)ii + 2u;
+      FuTrack<T> ut{T(-INFINITY), T(-INFINITY), T(-INFINITY)}, vt = ut;
+      int flag = fu_pass<T, MODE, NK, RES>(A, R, sm, red, rr, ring, ucur, unxt, H, held, ut, ep);
+      ok = fu_merge<T, false>(A, R, s_s, s_m, ep, [&](int j, T, T s) {
+        const T be = A.bew ? A.bew[j] : T(1);
+        const T vn = pow(A.b[j] / (be * s), A.fi2);
+        if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
+        const T vo = __ldcg(vcur + j);
+        vnxt[j] = vn;
+        Ll<T>::put(A.vll + j * Ll<T>::N, be * vn, ep);
+        vt.d0 = fmax(vt.d0, fabs(vn - vo));
+        vt.d1 = fmax(vt.d1, fabs(vn));
+        vt.d2 = fmax(vt.d2, fabs(vo));
+      });
+      // this CTA's maxima and flags
+      T mine[6] = {ut.d0, ut.d1, ut.d2, vt.d0, vt.d1, vt.d2};
+#pragma unroll
+      for (int q = 0; q < 6; ++q) { mine[q] = warp_max(mine[q]); if (R.lane == 0) s_mx[q][R.warp] = mine[q]; }
+      if (flag & FU_ABORT) ok = false;
+      flag = __syncthreads_or(flag);  // either flag ends the solve with the previous pair
+      if (threadIdx.x < 6) {
+        T t = s_mx[threadIdx.x][0];
+        for (int w = 1; w < FU_WARPS; ++w) t = fmax(t, s_mx[threadIdx.x][w]);
+        Ll<double>::put(A.ell + 12 * (int64_t)blockIdx.x + 2 * threadIdx.x, (double)t, ep);
+      }
+      if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, flag ? FU_BAD_ROW : 0, ep);
+      const int got = fu_collect(A, sm, ep, false, ok, e2);
+      if (got & FU_ABORT) { ok = false; break; }
+      // everyone's maxima
+      T mx[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) mx[q] = -INFINITY;
+      for (int p = threadIdx.x; p < (int)gridDim.x; p += FU_THREADS) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+          const unsigned long long* w = A.ell + 12 * (int64_t)p + 2 * q;
+          Ll<double>::W x = Ll<double>::get(w);
+          ok = ok && ll_wait<double>(w, ep, x, A.info + 3, A.timeout_ns);
+          mx[q] = fmax(mx[q], (T)Ll<double>::value(x));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 6; ++q) { mx[q] = warp_max(mx[q]); if (R.lane == 0) s_mx[q][R.warp] = mx[q]; }
+      if (__syncthreads_or(!ok)) { ok = false; break; }
+      double mk[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        T t = s_mx[q][0];
+        for (int w = 1; w < FU_WARPS; ++w) t = fmax(t, s_mx[q][w]);
+        mk[q] = (double)t;
+      }
+      __syncthreads();
+      if (got & FU_BAD_ROW) { status = OTG_STATUS_NUMERICAL; niter = ii; break; }  // previous pair kept
+      const double err = 0.5 * (mk[0] / fmax(fmax(mk[1], mk[2]), 1.0) + mk[3] / fmax(fmax(mk[4], mk[5]), 1.0));
+      if (blockIdx.x == 0 && threadIdx.x == 0 && ii < A.hist_cap) A.hist[ii] = err;
+      nchk = ii + 1;
+      T* t;
+      t = ucur; ucur = unxt; unxt = t;
+      t = vcur; vcur = vnxt; vnxt = t;
+      if (err < A.stop_thr) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
+    }
+  } else if (ok && A.max_iter > 0) {
+    // column update of the initial row potentials: the first v
+    int flag = 0;
+    if (LOGF) {
+      fu_collse<T, RES && MODE != FU_ABS>(A, R, sm, MODE == FU_ABS ? A.fref : ucur);
+      ok = fu_barrier(A.bar, gen, abort_flag, A.timeout_ns);
+      if (ok)
+        fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) {
+          Ll<T>::put(A.vll + j * Ll<T>::N, lg2(A.b[j]) - lse_value(mx, s), 1u);
+        });
+    } else {
+      fu_colsum<T, NK, RES>(A, R, sm, ucur, 1u);
+      ok = fu_merge<T, false>(A, R, s_s, s_m, 1u, [&](int j, T, T s) {
+        const T vn = A.b[j] / s;
+        if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
+        Ll<T>::put(A.vll + j * Ll<T>::N, vn, 1u);
+      });
+    }
+    flag = __syncthreads_or(flag) ? FU_BAD_COL : 0;
+    if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, flag, 1u);
+    int got = fu_collect(A, sm, 1u, false, ok, e2);
+    if (got & FU_ABORT) ok = false;
+    bool build = MODE == FU_ABS, again = false;
+    for (int ii = 0; ok; ++ii) {
+      // sm.vs holds v of iteration ii, ucur u of iteration ii - 1
+      if (MODE == FU_SCAL && (got & FU_BAD_COL)) {
+        // zero column sum or non-finite v: the previous pair
+        status = OTG_STATUS_NUMERICAL; niter = ii; break;
+      }
+      const unsigned ep = (unsigned)ii + 2u;
+      FuTrack<T> tr{T(0), T(0), T(0)};
+      flag = 0;
+      if (MODE == FU_ABS && build) {
+        for (int j = threadIdx.x; j < A.m; j += FU_THREADS) {
+          sm.gs[j] = ii == 0 ? sm.vs[j] : sm.gs[j] + lg2(sm.vs[j]);
+          sm.vs[j] = T(1);
+        }
+        if (ii == 0) for (int j = A.m + threadIdx.x; j < A.mp; j += FU_THREADS) sm.vs[j] = T(0);
+        __syncthreads();
+        fu_build<T, NK>(A, R, sm, red, unxt, ep);
+      } else {
+        flag = fu_pass<T, MODE, NK, RES>(A, R, sm, red, rr, ring, ucur, unxt, H, held, tr, ep);
+      }
+      T* t;
+      t = ucur; ucur = unxt; unxt = t;
+      t = vcur; vcur = vnxt; vnxt = t;
+      const bool check = ii % A.period == 0, last = ii + 1 == A.max_iter;
+      e2 = 0.0;
+      ok = fu_merge<T, false>(A, R, s_s, s_m, ep, [&](int j, T, T s) {
+        const T bj = A.b[j], vo = sm.vs[j];
+        vcur[j] = vo;
+        if (check) {
+          // column marginal of (u, v) of iteration ii
+          const double cs = MODE == FU_LOG ? (double)s : (double)(vo * s);
+          e2 += (cs - (double)bj) * (cs - (double)bj);
+        }
+        T vn;
+        if (MODE == FU_LOG) {
+          vn = bj == T(0) ? T(-INFINITY) : vo + lg2(bj / s);
+          if (bj != T(0) && !(s >= T(8.470329472543003e-22))) flag |= FU_BAD_COL;  // 2^-70
+        } else if (MODE == FU_ABS) {
+          vn = bj == T(0) ? T(1) : bj / s;
+          if (!fu_tame(vn)) flag |= FU_BAD_COL;
+        } else {
+          vn = bj / s;
+          if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
+        }
+        Ll<T>::put(A.vll + j * Ll<T>::N, vn, ep);
+      });
+      if (check) {
+        e2 = block_sum_fixed(e2);
+        if (threadIdx.x == 0) Ll<double>::put(A.ell + 2 * blockIdx.x, e2, ep);
+      }
+      if (flag & FU_ABORT) ok = false;
+      int mine = 0;
+      if (__syncthreads_or(flag)) {
+        mine = __syncthreads_or(flag & FU_BAD_ROW) ? FU_BAD_ROW : 0;
+        if (__syncthreads_or(flag & FU_BAD_COL)) mine |= FU_BAD_COL;
+      }
+      if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, mine, ep);
+      got = fu_collect(A, sm, ep, check, ok, e2);
+      if (got & FU_ABORT) { ok = false; break; }
+      if (MODE == FU_SCAL && (got & FU_BAD_ROW)) {
+        // non-finite u: the previous pair
+        t = ucur; ucur = unxt; unxt = t;
+        t = vcur; vcur = vnxt; vnxt = t;
+        status = OTG_STATUS_NUMERICAL; niter = ii; break;
+      }
+      if (check) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) A.hist[nchk < A.hist_cap ? nchk : A.hist_cap - 1] = e2;
+        ++nchk;
+        if (sqrt(e2) < A.stop_thr) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
+      }
+      if (last) { niter = ii; break; }
+      if (MODE == FU_ABS) build = got != 0;
+      if (MODE == FU_LOG) {
+        again = (got & FU_BAD_COL) != 0;
+        if (again) {
+          // a column sum too small to trust: the column update with running maxima
+          fu_collse<T, RES>(A, R, sm, ucur);
+          if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
+          fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) { A.vfix[j] = lg2(A.b[j]) - lse_value(mx, s); });
+          if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
+          for (int j = threadIdx.x; j < A.mp; j += FU_THREADS) sm.vs[j] = j < A.m ? __ldcg(A.vfix + j) : vpad;
+          __syncthreads();
+        }
+      }
+    }
+  }
+  if (!RES) {
+    // copies in flight land before the CTA leaves: NC chunks from the one due next
+    const uint64_t t0 = globaltimer();
+    if (R.tg == 0 && R.gb > R.ga)
+      for (int q = 0; q < A.NC; ++q) {
+        while (!mbar_try_wait(sm.full + R.g * A.NC + ring.slot, ring.phase)) if (globaltimer() - t0 > A.timeout_ns) break;
+        if (++ring.slot == A.NC) { ring.slot = 0; ring.phase ^= 1; }
+      }
+  }
+  __syncthreads();
+  if (!ok) return;
+
+  // Final state in natural units: this CTA's rows and its share of the columns.
+  for (int i = R.r0 + threadIdx.x; i < R.r1; i += FU_THREADS) {
+    const T u = __ldcg(ucur + i);
+    A.out_u[i] = MODE == FU_LOG ? u * LN2 : MODE == FU_ABS ? (__ldcg(A.fref + i) + lg2(u)) * LN2 : u;
+  }
+  for (int j = cb + threadIdx.x; j < ce; j += FU_THREADS) {
+    const T v = __ldcg(vcur + j);
+    // FU_ABS: scalings over the absorbed potentials (none yet when max_iter is 0)
+    A.out_v[j] = MODE == FU_LOG ? v * LN2 : MODE == FU_ABS ? (A.max_iter > 0 ? sm.gs[j] + lg2(v) : v) * LN2 : v;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    A.info[0] = status;
+    A.info[1] = niter;
+    A.info[2] = nchk;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Streamed rows that are not whole 16-byte vectors: one copy into padded rows
+// (scaling forms: of K = exp(-M/reg), unless that is what M holds already).
+// ---------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(256) fused_pack_kernel(const T* __restrict__ M, int64_t n, int64_t m, int64_t ldm, T c,
+                                                         int expo, T pad, T* __restrict__ out, int64_t ldo) {
+  for (int64_t i = blockIdx.x; i < n; i += gridDim.x)
+    for (int j = threadIdx.x; j < ldo; j += blockDim.x) {
+      const T x = j < m ? M[i * ldm + j] : pad;
+      out[i * ldo + j] = expo && j < m ? ex2(x * c) : x;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+struct FuPlan { int grid, G, NK, kv, mp, res, NC, buf_elems; size_t smem; };
+
+// The kernels' static shared memory (merge and reduction scratch), rounded up.
+template <typename T> size_t fu_static_smem(int nk) {
+  return sizeof(T) * (FU_WARPS * (32 + 6 + 4 * (size_t)fu_rb(nk))) + 304;
+}
+
+struct FuDevice { int sms = 0; size_t smem = 0; };
+inline FuDevice fu_device() {
+  FuDevice d;
+  int dev = 0, v = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  d.smem = v > 0 ? (size_t)v : 0;
+  return d;
+}
+
+// CTAs: one per SM at most, each with a row.  Small problems take fewer, and
+// a share of a few rows is rounded up to whole batches, as a CTA's time is
+// that of its batches (n = m = 1024: 128 CTAs of 8 rows 5.5 us per iteration
+// in float32 and 10.8 in float64, 152 CTAs of 7 rows 6.4 and 11.2).
+template <typename T>
+int fu_grid(int64_t n, int64_t m, int requested, int sms) {
+  const int64_t least = sizeof(T) == 4 ? 4096 : 1024;  // entries per CTA
+  int64_t g = (n * m + least - 1) / least;
+  g = std::max<int64_t>(std::min<int64_t>(std::min<int64_t>(g, sms), n), 1);
+  const int64_t V = (m + Vec<T>::N - 1) / Vec<T>::N;
+  int nk = 1;
+  while (nk < 16 && (int64_t)FU_WARPS * 32 * nk < V) nk *= 2;
+  const int64_t rb = fu_rb(nk), rows = (n + g - 1) / g;
+  if (rows < 2 * rb) {
+    const int64_t up = (rows + rb - 1) / rb * rb;
+    g = (n + up - 1) / up;
+  }
+  if (requested > 0) g = std::min<int64_t>(g, requested);
+  return (int)g;
+}
+
+// Split of an n x m problem; `abs`: the float64 log form over a resident K.
+// Returns false when the shape does not fit the kernel.
+template <typename T>
+bool fu_plan(int64_t n, int64_t m, bool abs, int grid, const FuDevice& d, FuPlan& f) {
+  constexpr int W = Vec<T>::N;
+  const int64_t V = (m + W - 1) / W;        // vectors of a row
+  if (V > (int64_t)FU_WARPS * 32 * 16 || n > 0x7fffff00) return false;
+  f.grid = grid;
+  const int64_t rows = (n + grid - 1) / grid;
+  auto split = [&](int nk) {
+    f.NK = nk;
+    f.G = 1;
+    while (f.G < FU_WARPS && (int64_t)f.G * 32 * nk < V) f.G *= 2;
+    f.kv = nk;
+    f.mp = nk * f.G * 32 * W;
+    const int NG = FU_WARPS / f.G;
+    f.buf_elems = NG > 1 ? std::max(NG * f.mp, FU_WARPS * 32) : 0;
+    return (int64_t)f.G * 32 * nk >= V;
+  };
+  f.NC = 0;
+  for (int nk : {1, 2, 3, 4, 6, 8, 12, 16}) {
+    if (!split(nk)) continue;
+    const size_t tile = sizeof(T) * (size_t)rows * f.mp;
+    f.smem = sizeof(T) * ((size_t)f.mp * (abs ? 2 : 1) + f.buf_elems) + tile;
+    f.res = rows <= 65536 && f.smem + fu_static_smem<T>(nk) <= d.smem;
+    if (f.res) return true;
+  }
+  if (abs) return false;
+  split(16);
+  f.kv = (int)((V + f.G * 32 - 1) / (f.G * 32));
+  const size_t half = sizeof(T) * (size_t)(FU_WARPS / f.G) * (f.mp / 2);  // 32 KB over the groups
+  for (f.NC = FU_RING; f.NC >= 4; --f.NC) {
+    f.smem = sizeof(T) * ((size_t)f.mp + f.buf_elems) + f.NC * half + 16 * ((size_t)(FU_WARPS / f.G * f.NC + 1) / 2);
+    if (f.smem + fu_static_smem<T>(16) <= d.smem) return true;
+  }
+  return false;
+}
+
+constexpr size_t FU_PACK_MAX = (size_t)16 << 30;
+
+// Workspace: published words, pairs, fallback v, padded rows.
+struct FuSpace { size_t part, vll, stll, ell, pairs, vfix, pack, total; };
+template <typename T>
+FuSpace fu_space(int64_t n, int64_t m, int grid, const FuDevice& d) {
+  FuSpace w{};
+  size_t off = 0;
+  auto take = [&](size_t b) { const size_t o = off; off += (b + 255) / 256 * 256; return o; };
+  FuPlan f, g;
+  if (!fu_plan<T>(n, m, false, grid, d, f)) return w;
+  w.part = take(8 * (size_t)Ll<T>::N * grid * m);
+  w.vll = take(8 * (size_t)Ll<T>::N * m);
+  w.stll = take(8 * (size_t)grid);
+  w.ell = take(96 * (size_t)grid);
+  w.pairs = take(2 * sizeof(T) * (size_t)grid * m);
+  w.vfix = take(sizeof(T) * (size_t)m);
+  w.pack = off;
+  const bool streamed = !f.res || (sizeof(T) == 8 && !fu_plan<T>(n, m, true, grid, d, g));
+  if (streamed && m % Vec<T>::N) {
+    const size_t b = sizeof(T) * (size_t)n * ((m + Vec<T>::N - 1) / Vec<T>::N * Vec<T>::N);
+    if (b > FU_PACK_MAX) return FuSpace{};
+    take(b);
+  }
+  w.total = off;
+  return w;
+}
+
+template <typename T, int MODE, int NK, bool RES>
+int fu_start(FusedArgs<T>& A, const FuPlan& f, cudaStream_t st) {
+  const void* k = (const void*)fused_sinkhorn_kernel<T, MODE, NK, RES>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) != cudaSuccess) {
+    cudaGetLastError();
+    return OTG_ERR_UNSUPPORTED;
+  }
+  void* args[] = {&A};
+  return cudaLaunchCooperativeKernel(k, dim3(f.grid), dim3(FU_THREADS), args, f.smem, st) == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
+}
+
+template <typename T, int MODE>
+int fu_start_resident(FusedArgs<T>& A, const FuPlan& f, cudaStream_t st) {
+  switch (f.NK) {
+    case 1: return fu_start<T, MODE, 1, true>(A, f, st);
+    case 2: return fu_start<T, MODE, 2, true>(A, f, st);
+    case 3: return fu_start<T, MODE, 3, true>(A, f, st);
+    case 4: return fu_start<T, MODE, 4, true>(A, f, st);
+    case 6: return fu_start<T, MODE, 6, true>(A, f, st);
+    case 8: return fu_start<T, MODE, 8, true>(A, f, st);
+    case 12: return fu_start<T, MODE, 12, true>(A, f, st);
+    default: return fu_start<T, MODE, 16, true>(A, f, st);
+  }
+}
+
+// The launches by mode and type, split over translation units.
+template <typename T> int fu_launch_log(FusedArgs<T>& A, const FuPlan& f, bool abs, cudaStream_t st);
+template <typename T> int fu_launch_scal(FusedArgs<T>& A, const FuPlan& f, cudaStream_t st);
+template <typename T> int fu_launch_unb(FusedArgs<T>& A, const FuPlan& f, cudaStream_t st);
+
+inline int fu_mode(const OtgDenseProblem* p) {
+  return p->method == OTG_METHOD_LOG ? FU_LOG : p->method == OTG_METHOD_KNOPP ? FU_SCAL : p->method == OTG_METHOD_UNB ? FU_UNB : -1;
+}
+
+template <typename T>
+bool fu_choose(const OtgDenseProblem* p, int& mode, const FuDevice& d, FuPlan& f) {
+  mode = fu_mode(p);
+  if (mode < 0) return false;
+  const int grid = fu_grid<T>(p->n, p->m, p->grid, d.sms);
+  if (sizeof(T) == 8 && mode == FU_LOG && fu_plan<T>(p->n, p->m, true, grid, d, f)) { mode = FU_ABS; return true; }
+  return fu_plan<T>(p->n, p->m, false, grid, d, f);
+}
+
+template <typename T>
+int fused_run(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st) {
+  const FuDevice d = fu_device();
+  FuPlan f;
+  int mode;
+  if (!fu_choose<T>(p, mode, d, f)) return OTG_ERR_UNSUPPORTED;
+  constexpr int W = Vec<T>::N;
+  FusedArgs<T> A{};
+  const bool useK = p->method == OTG_METHOD_KNOPP && p->K;
+  A.M = static_cast<const T*>(useK ? p->K : p->M);
+  A.n = (int)p->n; A.m = (int)p->m; A.ldm = useK ? p->ldk : p->ldm;
+  A.c = (T)(-OTG_LOG2E / p->reg);
+  A.mv = (int)((p->m + W - 1) / W * W);
+  A.gvec = p->m % W == 0 && A.ldm % W == 0 && (uintptr_t)A.M % 16 == 0;
+  const FuSpace w = fu_space<T>(p->n, p->m, f.grid, d);
+  char* base = static_cast<char*>(fs.space);
+  A.kmat = useK;
+  if (!f.res && !A.gvec) {
+    if (p->m % W == 0) return OTG_ERR_UNSUPPORTED;  // whole vectors at an odd address or stride: no room set aside
+    T* out = reinterpret_cast<T*>(base + w.pack);
+    const bool expo = mode != FU_LOG && !useK;
+    const T pad = mode != FU_LOG ? T(0) : (A.c > T(0) ? T(-INFINITY) : T(INFINITY));
+    const int blocks = (int)std::min<int64_t>(p->n, (int64_t)d.sms * 8);
+    fused_pack_kernel<T><<<blocks, 256, 0, st>>>(A.M, p->n, p->m, A.ldm, A.c, expo, pad, out, A.mv);
+    if (cudaGetLastError() != cudaSuccess) return OTG_ERR_CUDA;
+    A.M = out; A.ldm = A.mv; A.gvec = 1;
+    if (mode != FU_LOG) A.kmat = 1;
+  }
+  A.a = static_cast<const T*>(p->a); A.b = static_cast<const T*>(p->b);
+  A.warm_u = static_cast<const T*>(p->warm_u); A.warm_v = static_cast<const T*>(p->warm_v);
+  A.max_iter = p->max_iter; A.stop_thr = p->stop_thr; A.period = 10;
+  A.u0 = (T*)fs.u0; A.u1 = (T*)fs.u1; A.v0 = (T*)fs.v0; A.v1 = (T*)fs.v1; A.rowc = (T*)fs.rowc; A.fref = (T*)fs.fref;
+  A.part = (unsigned long long*)(base + w.part); A.vll = (unsigned long long*)(base + w.vll);
+  A.stll = (unsigned long long*)(base + w.stll); A.ell = (unsigned long long*)(base + w.ell);
+  A.pairs = (T*)(base + w.pairs); A.vfix = (T*)(base + w.vfix);
+  A.out_u = (T*)p->out_u; A.out_v = (T*)p->out_v;
+  A.hist = fs.hist; A.hist_cap = p->hist_cap; A.info = fs.info; A.bar = fs.bar;
+  A.timeout_ns = fs.timeout_ns;
+  A.G = f.G; A.kv = f.kv; A.mp = f.mp; A.NC = f.NC; A.buf_elems = f.buf_elems;
+  if (mode == FU_UNB) {
+    A.fi1 = (T)(std::isinf(p->reg_m1) ? 1.0 : p->reg_m1 / (p->reg_m1 + p->reg));
+    A.fi2 = (T)(std::isinf(p->reg_m2) ? 1.0 : p->reg_m2 / (p->reg_m2 + p->reg));
+    A.alw = p->c_ones ? nullptr : A.a;
+    A.bew = p->c_ones ? nullptr : A.b;
+    return fu_launch_unb<T>(A, f, st);
+  }
+  if (mode == FU_SCAL) return fu_launch_scal<T>(A, f, st);
+  return fu_launch_log<T>(A, f, mode == FU_ABS, st);
+}
+
+template <typename T>
+size_t fused_run_bytes(int64_t n, int64_t m, int requested_grid) {
+  const FuDevice d = fu_device();
+  return fu_space<T>(n, m, fu_grid<T>(n, m, requested_grid, d.sms), d).total;
+}
+
+template <typename T>
+bool fused_run_resident(const OtgDenseProblem* p) {
+  FuPlan f;
+  int mode;
+  return fu_choose<T>(p, mode, fu_device(), f) && f.res;
+}
+
+}  // namespace otg

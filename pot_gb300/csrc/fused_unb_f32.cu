@@ -1,0 +1,8 @@
+// float32 unbalanced form of the one-read dense Sinkhorn (fused_impl.cuh).
+#include "fused_impl.cuh"
+
+namespace otg {
+template <> int fu_launch_unb<float>(FusedArgs<float>& A, const FuPlan& f, cudaStream_t st) {
+  return f.res ? fu_start_resident<float, FU_UNB>(A, f, st) : fu_start<float, FU_UNB, 16, false>(A, f, st);
+}
+}  // namespace otg

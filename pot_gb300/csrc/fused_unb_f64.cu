@@ -1,0 +1,8 @@
+// float64 unbalanced form of the one-read dense Sinkhorn (fused_impl.cuh).
+#include "fused_impl.cuh"
+
+namespace otg {
+template <> int fu_launch_unb<double>(FusedArgs<double>& A, const FuPlan& f, cudaStream_t st) {
+  return f.res ? fu_start_resident<double, FU_UNB>(A, f, st) : fu_start<double, FU_UNB, 16, false>(A, f, st);
+}
+}  // namespace otg

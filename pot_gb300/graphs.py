@@ -16,7 +16,7 @@ import ctypes
 import torch
 
 from . import _lib
-from .bregman import NONCONV_MSG, default_grid, read_result, solve_dense
+from .bregman import NONCONV_MSG, read_result, solve_dense
 
 _METHODS = {"sinkhorn": _lib.OTG_METHOD_KNOPP, "sinkhorn_knopp": _lib.OTG_METHOD_KNOPP,
             "sinkhorn_log": _lib.OTG_METHOD_LOG}
@@ -47,7 +47,6 @@ class SinkhornGraph:
         self.b = torch.full((self.m,), 1.0 / self.m, dtype=dtype, device=dev)
         self.P = torch.empty(self.n, self.m, dtype=dtype, device=dev) if want_plan else None
         self.loss = torch.zeros(1, dtype=torch.float64, device=dev)
-        self.grid = default_grid(self.n, self.m, dtype)
         self.M.copy_(torch.rand(self.n, self.m, dtype=dtype, device=dev))
         side = torch.cuda.Stream(dev)
         side.wait_stream(torch.cuda.current_stream(dev))
@@ -63,7 +62,7 @@ class SinkhornGraph:
     def _record(self):
         lib = _lib.load()
         self.r = solve_dense(self.M, self.a, self.b, self.reg, self.method, self.numItermax, self.stopThr,
-                             grid=self.grid, read_back=False)
+                             read_back=False)
         st = _lib.stream_handle(self.M.device)
         dt = _lib.dtype_code(self.M.dtype)
         if self.P is not None:
