@@ -257,8 +257,8 @@ int otg_sinkhorn_batched(const OtgBatchProblem* q, cudaStream_t stream);
  * test of ot/bregman/_sinkhorn.py:880-899 (sinkhorn_log).  Same packed
  * layout as otg_sinkhorn_batched; nsr_max[p] (>= 1) bounds the row split of
  * problem p's column reductions and pc_off[p] places its nsr_max[p] x cols[p]
- * partial pairs (total_partials in all).  The workspace size comes from
- * otg_multi_workspace_bytes.
+ * partial pairs (total_partials in all, or more).  M is 16-byte aligned.
+ * The workspace size comes from otg_multi_workspace_bytes.
  * ---------------------------------------------------------------------- */
 typedef struct OtgMultiProblem {
   int32_t dtype;
@@ -328,7 +328,10 @@ typedef struct OtgMultiProblem {
    * row marginal and a checked column marginal, as in sinkhorn_log.  Needs
    * otg_multi_anderson_bytes() of device memory in anderson_ws. */
   int32_t anderson_depth;
-  int32_t reserved;
+  /* largest ldm of the batch: lets the solver read the blocks once per
+   * iteration where total_partials is at least otg_multi_partials(); 0, or a
+   * smaller total_partials: two passes per iteration */
+  int32_t max_ldm;
   void* anderson_ws;
   size_t anderson_ws_bytes;
 } OtgMultiProblem;
@@ -336,6 +339,9 @@ typedef struct OtgMultiProblem {
 size_t otg_multi_workspace_bytes(int dtype, int32_t nprob, int64_t total_rows, int64_t total_cols,
                                  int64_t total_partials);
 int otg_sinkhorn_multi(const OtgMultiProblem* q, cudaStream_t stream);
+/* total_partials with which the solver reads the blocks once per iteration on
+ * the current device (0: the widest block is too wide for that). */
+int64_t otg_multi_partials(int dtype, int32_t nprob, int64_t total_cols, int64_t max_ldm);
 /* Device bytes of the Anderson history (anderson_ws) for a batch. */
 size_t otg_multi_anderson_bytes(int dtype, int32_t nprob, int64_t total_cols, int32_t depth);
 /* The tail handoff's cluster shape on the current device: CTAs per cluster

@@ -48,7 +48,7 @@ class OtgMultiProblem(ctypes.Structure):
                 ("workspace", c_vp), ("workspace_bytes", c_sz), ("timeout_ms", c_i32), ("omega", c_dbl),
                 ("check_period", c_i32), ("units_per_warp", c_i32), ("split_cap_fill", c_i32),
                 ("split_cap_tail", c_i32), ("tail_problems", c_i32), ("joint_stop", c_i32),
-                ("scaling", c_i32), ("anderson_depth", c_i32), ("reserved", c_i32), ("anderson_ws", c_vp),
+                ("scaling", c_i32), ("anderson_depth", c_i32), ("max_ldm", c_i32), ("anderson_ws", c_vp),
                 ("anderson_ws_bytes", c_sz)]
 
 
@@ -125,6 +125,7 @@ SIGNATURES = {
                                         ctypes.POINTER(c_i32)]),
     "otg_sinkhorn_batched": (ctypes.c_int, [ctypes.POINTER(OtgBatchProblem), c_vp]),
     "otg_multi_workspace_bytes": (c_sz, [ctypes.c_int, c_i32, c_i64, c_i64, c_i64]),
+    "otg_multi_partials": (c_i64, [ctypes.c_int, c_i32, c_i64, c_i64]),
     "otg_sinkhorn_multi": (ctypes.c_int, [ctypes.POINTER(OtgMultiProblem), c_vp]),
     "otg_multi_anderson_bytes": (c_sz, [ctypes.c_int, c_i32, c_i64, c_i32]),
     "otg_pairs_workspace_bytes": (c_sz, [c_i32, c_i64, c_i64, c_i32, c_i32]),

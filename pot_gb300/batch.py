@@ -182,7 +182,10 @@ def _run_multi_once(layout, M_packed, a_packed, b_packed, reg, max_iter, tol, wa
         nsr_max = np.maximum(1, np.minimum(64, (layout.rows_np + 15) // 16)).astype(np.int32)
         sizes = nsr_max.astype(np.int64) * layout.cols_np
         layout.nsr_max_np = nsr_max
-        layout.total_partials = int(sizes.sum())
+        layout.max_ldm = int(layout.ldm_np.max())
+        # room for the row chunks' partials, or for the one-read kernel's worker slots
+        layout.total_partials = max(int(sizes.sum()), int(lib.otg_multi_partials(
+            _lib.dtype_code(dt), B, layout.total_c, layout.max_ldm)))
         layout.nsr_max = torch.tensor(nsr_max, dtype=torch.int32, device=dev)
         layout.pc_off = torch.tensor(np.concatenate([[0], np.cumsum(sizes)[:-1]]), dtype=torch.int64, device=dev)
     dcode = _lib.dtype_code(dt)
@@ -207,7 +210,7 @@ def _run_multi_once(layout, M_packed, a_packed, b_packed, reg, max_iter, tol, wa
         omega=float(omega), check_period=int(check_period), units_per_warp=int(schedule.units_per_warp),
         split_cap_fill=int(schedule.cap_fill), split_cap_tail=int(schedule.cap_tail),
         tail_problems=int(tail_problems), joint_stop=int(bool(joint)), scaling=int(bool(scaling)),
-        anderson_depth=int(anderson), anderson_ws=aws.data_ptr() if awb else None, anderson_ws_bytes=awb)
+        anderson_depth=int(anderson), max_ldm=layout.max_ldm, anderson_ws=aws.data_ptr() if awb else None, anderson_ws_bytes=awb)
     if events is not None:
         events[0].record()
     _lib.check(lib.otg_sinkhorn_multi(ctypes.byref(q), _lib.stream_handle(dev)), "otg_sinkhorn_multi")

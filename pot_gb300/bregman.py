@@ -276,7 +276,7 @@ def _log_multi(bd, a, B, M, reg, numItermax, stopThr, verbose, log, warmstart):
     dt, dev = M.dtype, M.device
     lay = pb.RaggedLayout([n] * H, [m] * H, dt, dev)
     ld = int(lay.ldm_np[0])
-    if ld == m and M.is_contiguous():
+    if ld == m and M.is_contiguous() and M.data_ptr() % 16 == 0:
         Mp = M.reshape(-1)
     else:
         Mp = torch.full((n, ld), float("inf"), dtype=dt, device=dev)

@@ -121,7 +121,7 @@ namespace {
   X(joint_stop) \
   X(scaling) \
   X(anderson_depth) \
-  X(reserved) \
+  X(max_ldm) \
   X(anderson_ws) \
   X(anderson_ws_bytes)
 #define OTG_FIELDS_OtgOnlineProblem(X) \

@@ -49,53 +49,113 @@ __device__ void anderson_step(int D, int m, int64_t co, int64_t stride, const T*
       }
     }
   }
+  // all dots at once: a halving butterfly over the warp (lane l ends with dot
+  // l / 4), then the warps in order.  FP64 issues at two lanes per clock, so
+  // eight separate block sums were a third of the step.
+  {
+    __shared__ double s_part[32][MD];
+    int o = 16;
 #pragma unroll
-  for (int q = 0; q < MD; ++q) {
-    if (q < nh) {
-      const double d = block_sum_fixed(acc[q]);
-      if (threadIdx.x == 0) s_dot[q] = d;
+    for (int h = MD / 2; h >= 1; h /= 2) {
+      const bool up = threadIdx.x & o;
+#pragma unroll
+      for (int q = 0; q < h; ++q) {
+        const double keep = up ? acc[q + h] : acc[q], give = up ? acc[q] : acc[q + h];
+        acc[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+      o >>= 1;
+    }
+    double d = acc[0];
+    for (int q = 16 / MD; q > 0; q >>= 1) d += __shfl_xor_sync(0xffffffffu, d, q);
+    __syncthreads();
+    if ((threadIdx.x & 31) % (32 / MD) == 0) s_part[threadIdx.x >> 5][(threadIdx.x & 31) / (32 / MD)] = d;
+    __syncthreads();
+    if (threadIdx.x < MD) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_part[w][threadIdx.x];
+      s_dot[threadIdx.x] = t;
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < nh; ++q) { G[s * D + q] = s_dot[q]; G[q * D + s] = s_dot[q]; }
-    // (G + lambda I) w = 1 by Gaussian elimination with partial pivoting
-    double Mx[MD][MD + 1];
+  if (threadIdx.x < 32) {
+    // (G + lambda I) w = 1 by Gaussian elimination with partial pivoting, a
+    // row per lane (rows beyond nh are those of the identity): one thread's
+    // elimination, with the separate block sums, took 60 us of the step
+    const int lane = threadIdx.x;
+    double row[MD + 1];
     double tr = 0.0;
-    for (int i = 0; i < nh; ++i) tr += G[i * D + i];
-    const double lam = AND_LAMBDA * tr / nh;
-    for (int i = 0; i < nh; ++i) {
-      for (int j = 0; j < nh; ++j) Mx[i][j] = G[i * D + j] + (i == j ? lam : 0.0);
-      Mx[i][nh] = 1.0;
+    if (lane < nh) {
+#pragma unroll
+      for (int j = 0; j < MD; ++j) row[j] = j < nh ? (lane == s ? s_dot[j] : j == s ? s_dot[lane] : G[lane * D + j]) : 0.0;
+      G[s * D + lane] = s_dot[lane];
+      G[lane * D + s] = s_dot[lane];
+    } else {
+#pragma unroll
+      for (int j = 0; j < MD; ++j) row[j] = j == lane ? 1.0 : 0.0;
     }
+    row[MD] = lane < nh ? 1.0 : 0.0;
+    double diag = 0.0;
+#pragma unroll
+    for (int j = 0; j < MD; ++j) if (j == lane) diag = row[j];
+    for (int i = 0; i < nh; ++i) tr += __shfl_sync(0xffffffffu, diag, i);
+    const double lam = AND_LAMBDA * tr / nh;
+#pragma unroll
+    for (int j = 0; j < MD; ++j) if (j == lane && lane < nh) row[j] += lam;
     bool ok = nh > 1 && tr > 0.0;
-    for (int c = 0; ok && c < nh; ++c) {
-      int piv = c;
-      for (int i = c + 1; i < nh; ++i) if (fabs(Mx[i][c]) > fabs(Mx[piv][c])) piv = i;
-      if (!(fabs(Mx[piv][c]) > 0.0)) { ok = false; break; }
-      if (piv != c) for (int j = c; j <= nh; ++j) { const double t = Mx[c][j]; Mx[c][j] = Mx[piv][j]; Mx[piv][j] = t; }
-      for (int i = c + 1; i < nh; ++i) {
-        const double f = Mx[i][c] / Mx[c][c];
-        for (int j = c; j <= nh; ++j) Mx[i][j] -= f * Mx[c][j];
+#pragma unroll
+    for (int c = 0; c < MD; ++c) {
+      if (c < nh) {
+        // the first of the largest entries of the column at or below the diagonal
+        int piv = c;
+        double best = fabs(__shfl_sync(0xffffffffu, row[c], c));
+        for (int i = c + 1; i < nh; ++i) {
+          const double x = fabs(__shfl_sync(0xffffffffu, row[c], i));
+          if (x > best) { best = x; piv = i; }
+        }
+        if (!(best > 0.0)) ok = false;
+        const int from = lane == c ? piv : lane == piv ? c : lane;
+        double top[MD + 1];
+#pragma unroll
+        for (int j = 0; j <= MD; ++j) {
+          row[j] = __shfl_sync(0xffffffffu, row[j], from);
+          top[j] = __shfl_sync(0xffffffffu, row[j], c);
+        }
+        if (lane > c && lane < nh && ok) {
+          const double f = row[c] / top[c];
+#pragma unroll
+          for (int j = 0; j <= MD; ++j) if (j >= c) row[j] -= f * top[j];
+        }
       }
     }
     double w[MD];
     double sw = 0.0, l1 = 0.0;
-    for (int i = nh - 1; ok && i >= 0; --i) {
-      double t = Mx[i][nh];
-      for (int j = i + 1; j < nh; ++j) t -= Mx[i][j] * w[j];
-      w[i] = t / Mx[i][i];
-      sw += w[i];
+#pragma unroll
+    for (int i = MD - 1; i >= 0; --i) {
+      w[i] = 0.0;
+      if (i < nh) {
+        double t = row[MD];
+#pragma unroll
+        for (int j = 0; j < MD; ++j) if (j > i && j < nh) t -= row[j] * w[j];
+        double x = 0.0;
+#pragma unroll
+        for (int j = 0; j < MD; ++j) if (j == i) x = t / row[j];
+        w[i] = __shfl_sync(0xffffffffu, x, i);
+        sw += w[i];
+      }
     }
     if (ok) {
-      for (int i = 0; i < nh; ++i) { w[i] /= sw; l1 += fabs(w[i]); }
+#pragma unroll
+      for (int i = 0; i < MD; ++i) if (i < nh) { w[i] /= sw; l1 += fabs(w[i]); }
       ok = isfinite(l1) && l1 < AND_MAX_L1;
     }
-    for (int i = 0; i < MD; ++i) s_alpha[i] = ok && i < nh ? w[i] : (i == s ? 1.0 : 0.0);
-    // a first iterate, or a failed solve: the plain step; after a failure
-    // the history restarts with the next iterate
-    s_keep = ok;
-    *cnt_p = ok || nh == 1 ? cnt + 1 : 0;
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < MD; ++i) s_alpha[i] = ok && i < nh ? w[i] : (i == s ? 1.0 : 0.0);
+      // a first iterate, or a failed solve: the plain step; after a failure
+      // the history restarts with the next iterate
+      s_keep = ok;
+      *cnt_p = ok || nh == 1 ? cnt + 1 : 0;
+    }
   }
   __syncthreads();
   if (s_keep) {

@@ -26,6 +26,10 @@
 // v in use, so the stop test measures exactly what it measures for plain
 // sinkhorn_log: the column marginal of (u, v) with u = rowT(v).
 //
+// Batches whose widest block the one-read kernel takes (multi_fused.cuh: up to
+// 16384 float32 or 8192 float64 columns) run there; the kernel of this file
+// is for wider ones and for callers whose workspace has no room for it.
+//
 // One persistent cooperative launch.  Each iteration:
 //   column pass : units (problem, row chunk, slab of 32*VW columns) over all
 //                 active problems -> partial (max, sum) per column  | barrier
@@ -53,113 +57,12 @@
 // batch kernel.
 #include <algorithm>
 #include <cooperative_groups.h>
-#include "common.cuh"
-#include "anderson.cuh"
+#include "multi_common.cuh"
 #include "../../include/pot_gb300.h"
 
 namespace cg = cooperative_groups;
 
 namespace otg {
-
-// 256 threads at no more than 64 registers, four CTAs per SM (float): the
-// loads in flight come from the 32 resident warps (measured: 0.79 of the copy peak
-// against 0.71 for two CTAs of 118 registers with loads software-pipelined
-// one group ahead, on 512 cost blocks of 2048 x 2048).
-constexpr int MT_THREADS = 256;
-// CTAs per SM: float at 64 registers; double keeps 128 registers (no spills)
-template <typename T> struct MtBlocks { static constexpr int value = sizeof(T) == 4 ? 4 : 2; };
-constexpr int MT_RW = 4;       // rows per warp in the row pass
-constexpr int MT_GCOL = 4;     // rows folded per max update (column pass)
-
-template <typename T> struct MPair { T mx, s; };
-
-template <typename T>
-struct MultiArgs {
-  const T* M; const int64_t* m_off; const int32_t* rows; const int32_t* cols; const int32_t* ldm;
-  const int64_t* r_off; const int64_t* c_off;
-  const T* a; const T* b; const T* warm_u;
-  const double* reg;
-  int32_t nprob, max_iter;
-  double stop_thr;
-  // per-problem decomposition: partial buffers sized for nsr_max row chunks;
-  // the split in use (nsr, rchunk) is chosen at every rebuild of the active
-  // list from the amount of work left
-  const int32_t* nsr_max;
-  int32_t* nsr;             // row chunks (column pass), device-chosen
-  int32_t* rchunk;          // rows per chunk, device-chosen
-  const int64_t* pc_off;    // offset of problem's partials [nsr_max][m]
-  // state
-  T* u; T* v0; T* v1;       // base-2 potentials, packed like a / b
-  MPair<T>* pcol;
-  double* err2;             // per problem: squared error of the last check (joint stop)
-  double* e2col;            // per column: squared marginal error (check passes), packed like b
-  bool joint;               // whole-batch stop on the largest error
-  // Anderson mixing of the v update (depth 0: off): history slots of F(v)
-  // and of the residual F(v) - v, [depth][total_cols] each (slot-major,
-  // packed like b), residual Gram matrices [nprob][depth][depth] and the
-  // number of iterates taken so far per problem
-  int and_depth;
-  int64_t total_cols;
-  T* and_F; T* and_R;
-  double* and_G;
-  int32_t* and_cnt;
-  int32_t* active;          // active problem ids [nprob]
-  int64_t* ucol_pre;        // prefix of column-pass units over the active list [nprob+1]
-  int64_t* urow_pre;        // prefix of row-pass units
-  int64_t* colpre;          // prefix of columns (merge) over the active list
-  int32_t* ctl;             // [0] n active, [1] abort
-  int32_t* leave_cnt;       // [2] problems leaving at a decision (alternate decisions)
-  unsigned* bar;
-  // outputs
-  T* out_u; T* out_v;
-  int32_t* status; int32_t* niter; double* err;
-  uint64_t timeout_ns;
-  T omega;                  // over-relaxation (1: plain)
-  bool relax;
-  int period;               // iterations between stop tests
-  int upw, cap_fill, cap_tail;  // schedule: units per warp, row-split caps
-  // tail handoff: most problems handed over (0: never), CTAs per cluster,
-  // shared-memory bytes for one CTA's rows of a cost block
-  int tail_max, tail_cl;
-  int64_t tail_tile;
-};
-
-// Tail kernel limits: columns, rows per CTA
-constexpr int TL_MAXM = 2048;
-constexpr int TL_MAXR = 1024;
-constexpr int TL_THREADS = 256;
-
-// Index of the active slot whose prefix range holds `unit` (pre[k] <= unit < pre[k+1]).
-__device__ __forceinline__ int mt_find(const int64_t* pre, int n, int64_t unit) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldcg(pre + mid) <= unit) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-// Slot cursor over a prefix array: pre[k] <= item < pre[k+1].  Items visited
-// in increasing order mostly stay in the slot or move to the next one, so the
-// binary search (a chain of dependent L2 loads) runs about once per problem.
-struct MtSlot {
-  int k = -1;
-  int64_t lo = 0, hi = 0;
-  __device__ __forceinline__ bool seek(const int64_t* pre, int n, int64_t item) {
-    if (k >= 0 && item >= lo && item < hi) return false;
-    if (k >= 0 && item >= hi && k + 1 < n && __ldcg(pre + k + 2) > item) ++k;
-    else k = mt_find(pre, n, item);
-    lo = __ldcg(pre + k);
-    hi = __ldcg(pre + k + 1);
-    return true;
-  }
-};
-
-// Contiguous share [beg, end) of `total` items for worker w of nw.
-__device__ __forceinline__ void mt_share(int64_t total, long w, long nw, int64_t& beg, int64_t& end) {
-  beg = total * w / nw;
-  end = total * (w + 1) / nw;
-}
 
 template <typename T, bool LOGF>
 __device__ void mt_col_pass(const MultiArgs<T>& A, int nact, long gwarp, long nwarps, int lane) {
@@ -474,18 +377,6 @@ __device__ void mt_rebuild(const MultiArgs<T>& A, int nact, const int32_t* leavi
   __syncthreads();
 }
 
-// Anderson step (one CTA per active problem, anderson.cuh): the new v of
-// every active problem is mixed over its history.  Kept out of line, like
-// the joint decision: it must not weigh on the registers of the passes.
-template <typename T>
-__device__ __noinline__ void mt_anderson(const MultiArgs<T>& A, int nact, const T* vcur, T* vnxt) {
-  for (int k = blockIdx.x; k < nact; k += gridDim.x) {
-    const int p = __ldcg(A.active + k);
-    anderson_step<T>(A.and_depth, A.cols[p], A.c_off[p], A.total_cols, vcur, vnxt, A.and_F, A.and_R,
-                     A.and_G + (int64_t)p * A.and_depth * A.and_depth, A.and_cnt + p);
-  }
-}
-
 // Whole-batch stop decision (joint mode): every problem's error into
 // err2[p] (its column slots summed in a fixed order), then the largest over
 // the batch (a max: the same in any order).  Returns 1 when the batch stops,
@@ -499,18 +390,7 @@ __device__ __noinline__ int mt_joint_decision(const MultiArgs<T>& A, int nact) {
     if (threadIdx.x == 0) A.err2[p] = e2;
   }
   if (!grid_barrier(A.bar, gridDim.x, A.ctl + 1, A.timeout_ns)) return -1;
-  __shared__ double s_mx[MT_THREADS / 32];
-  double mx = 0.0;
-  for (int k = threadIdx.x; k < nact; k += blockDim.x) {
-    const double e2 = __ldcg(A.err2 + __ldcg(A.active + k));
-    mx = isnan(e2) ? (double)INFINITY : fmax(mx, e2);  // a NaN error never meets the test
-  }
-  mx = warp_max(mx);
-  if ((threadIdx.x & 31) == 0) s_mx[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx = fmax(mx, s_mx[w]);
-  __syncthreads();
-  return sqrt(mx) < A.stop_thr ? 1 : 0;
+  return mt_joint_largest<T>(A, nact) < A.stop_thr ? 1 : 0;
 }
 
 template <typename T, bool LOGF>
@@ -965,6 +845,32 @@ size_t anderson_ws_bytes(size_t es, int64_t nprob, int64_t cols, int depth) {
   return 2 * r(es * (size_t)depth * (size_t)cols) + r(8 * (size_t)nprob * depth * depth) + r(4 * (size_t)nprob);
 }
 
+// The one-read kernel's plan on the current device.
+bool fused_plan_here(int dtype, int64_t max_ldm, MultiFusedPlan& f) {
+  if (max_ldm < 1 || max_ldm > 65536) return false;
+  int dev = 0, smem = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return smem > 0 && multi_fused_plan(dtype, (int)max_ldm, (size_t)smem, f);
+}
+
+// Elements of one set of worker slots: the padded columns of all problems,
+// and a widest problem per worker.
+int64_t fused_span(int dtype, int64_t nprob, int64_t total_cols, int64_t max_ldm, const MultiFusedPlan& f, int sms) {
+  const int64_t W = dtype == OTG_F64 ? 2 : 4;
+  return (total_cols + (W - 1) * nprob + (int64_t)sms * (8 / f.G) * max_ldm + 63) / 64 * 64;
+}
+
+// total_partials that the one-read kernel wants (0: it does not take the batch).
+int64_t fused_partials(int dtype, int64_t nprob, int64_t total_cols, int64_t max_ldm) {
+  MultiFusedPlan f;
+  if (!fused_plan_here(dtype, max_ldm, f)) return 0;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (3 * fused_span(dtype, nprob, total_cols, max_ldm, f, sms) + 1) / 2;
+}
+
 template <typename T, bool LOGF>
 int launch_multi(const OtgMultiProblem* q, cudaStream_t st) {
   MultiArgs<T> A{};
@@ -1032,14 +938,30 @@ int launch_multi(const OtgMultiProblem* q, cudaStream_t st) {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaError_t e = cudaSuccess;
+  MultiFusedPlan f;
+  const int64_t need = fused_partials(q->dtype, q->nprob, q->total_cols, q->max_ldm);
+  if (need > 0 && need <= q->total_partials && fused_plan_here(q->dtype, q->max_ldm, f)) {
+    // one read of the blocks per iteration
+    A.fG = f.G; A.fNC = f.NC; A.fmp = f.mp; A.fmm = q->max_ldm;
+    const int64_t span = fused_span(q->dtype, q->nprob, q->total_cols, q->max_ldm, f, sms);
+    A.fpart = reinterpret_cast<T*>(A.pcol);
+    A.fpairs = A.fpart + span;
+    A.fbad = A.nsr;
+    int grid = sms;
+    if (q->grid > 0 && q->grid < grid) grid = q->grid;
+    const int rc = multi_fused_launch(A, LOGF, f.NK, grid, f.smem, leaving, st);
+    if (rc != OTG_OK) return rc;
+  } else {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, multi_sinkhorn_kernel<T, LOGF>, MT_THREADS, 0);
   int grid = sms * std::min(per, MtBlocks<T>::value);
   if (q->grid > 0 && q->grid < grid) grid = q->grid;
   if (grid < 1) return OTG_ERR_UNSUPPORTED;
   void* args[] = {&A, &leaving};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)multi_sinkhorn_kernel<T, LOGF>, dim3(grid), dim3(MT_THREADS),
-                                              args, 0, st);
+  e = cudaLaunchCooperativeKernel((const void*)multi_sinkhorn_kernel<T, LOGF>, dim3(grid), dim3(MT_THREADS),
+                                  args, 0, st);
   if (e != cudaSuccess) return OTG_ERR_CUDA;
+  }
   if (A.tail_max > 0) {
     // behind the batch kernel on the stream; returns at once unless it was handed problems
     cudaLaunchConfig_t cfg = {};
@@ -1075,6 +997,11 @@ size_t otg_multi_workspace_bytes(int dtype, int32_t nprob, int64_t total_rows, i
   return multi_ws(dtype, nprob, total_rows, total_cols, total_partials);
 }
 
+int64_t otg_multi_partials(int dtype, int32_t nprob, int64_t total_cols, int64_t max_ldm) {
+  if (nprob < 1 || total_cols < 1 || (dtype != OTG_F32 && dtype != OTG_F64)) return 0;
+  return fused_partials(dtype, nprob, total_cols, max_ldm);
+}
+
 size_t otg_multi_anderson_bytes(int dtype, int32_t nprob, int64_t total_cols, int32_t depth) {
   if (depth <= 0) return 0;
   return anderson_ws_bytes(dtype == OTG_F64 ? 8 : 4, nprob, total_cols, depth);
@@ -1099,7 +1026,7 @@ int otg_sinkhorn_multi(const OtgMultiProblem* q, cudaStream_t stream) {
       !q->reg || !q->nsr_max || !q->pc_off || !q->out_u || !q->out_v || !q->status || !q->niter ||
       !q->err || !q->workspace)
     return OTG_ERR_ARG;
-  if (q->nprob < 1 || q->max_iter < 1) return OTG_ERR_ARG;
+  if (q->nprob < 1 || q->max_iter < 1 || (uintptr_t)q->M % 16) return OTG_ERR_ARG;
   if (q->anderson_depth < 0 || q->anderson_depth > OTG_ANDERSON_MAX_DEPTH) return OTG_ERR_ARG;
   if (q->anderson_depth > 0 && q->scaling != 0) return OTG_ERR_UNSUPPORTED;
   const bool logf = q->scaling == 0;
