@@ -133,6 +133,18 @@ int otg_dense_plan(int dtype, int method, const void* M, int64_t n, int64_t m, i
                    const void* u, const void* v, double reg, void* P, int64_t ldp, double* loss,
                    cudaStream_t stream);
 
+/* Gradients of sum(M * P) at the Sinkhorn solution P of (a, b, M, reg), fp64,
+ * by implicit differentiation (conjugate gradients to the relative residual
+ * rtol, at most max_iter steps): gM (n x m, row stride ldg), ga (n), gb (m).
+ * info: 4 int32 of device memory, info[3] != 0 afterwards when a device-side
+ * wait ran out.  OTG_ERR_UNSUPPORTED (workspace size 0) for m > 4096.  No
+ * reference counterpart: the reference's torch backend differentiates through
+ * its iterations (ot/bregman/_sinkhorn.py:435-438). */
+size_t otg_sinkhorn_grad_workspace_bytes(int64_t n, int64_t m);
+int otg_sinkhorn_grad(const double* P, int64_t ldp, const double* M, int64_t ldm, int64_t n, int64_t m, const double* a,
+                      const double* b, double reg, double rtol, int32_t max_iter, double* gM, int64_t ldg, double* ga,
+                      double* gb, void* workspace, size_t workspace_bytes, int32_t* info, cudaStream_t stream);
+
 /* K = exp(-M/reg) (n x m, row stride ldk), computed exactly as the scaling
  * form of otg_sinkhorn_dense computes it on the fly: the Gibbs kernel of
  * ot/bregman/_sinkhorn.py:621. */

@@ -68,6 +68,31 @@ def envelope_loss(loss, P, r, method, reg, a, b, M):
     return out
 
 
+def _native_grads(P, M, a, b, reg, rtol, limit):
+    """``implicit_grads`` in one launch (``otg_sinkhorn_grad``), or None for
+    problems that it does not take."""
+    lib = _lib.load()
+    n, m = P.shape
+    P, M = (x if x.stride(1) == 1 and x.stride(0) >= m else x.contiguous() for x in (P, M))
+    a, b = a.contiguous(), b.contiguous()
+    wsb = lib.otg_sinkhorn_grad_workspace_bytes(n, m)
+    if wsb == 0:
+        return None
+    dev = P.device
+    ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+    gM = torch.empty((n, m), dtype=torch.float64, device=dev)
+    ga = torch.empty(n, dtype=torch.float64, device=dev)
+    gb = torch.empty(m, dtype=torch.float64, device=dev)
+    info = torch.empty(4, dtype=torch.int32, device=dev)
+    _lib.check(lib.otg_sinkhorn_grad(_lib.ptr(P), P.stride(0), _lib.ptr(M), M.stride(0), n, m, _lib.ptr(a), _lib.ptr(b),
+                                     float(reg), float(rtol), int(min(limit, 2 ** 31 - 1)), _lib.ptr(gM), m, _lib.ptr(ga),
+                                     _lib.ptr(gb), _lib.ptr(ws), wsb, _lib.ptr(info), _lib.stream_handle(dev)),
+               "otg_sinkhorn_grad")
+    if int(info[3]) != 0:
+        raise RuntimeError("pot_gb300: a device-side wait timed out; the gradients were abandoned")
+    return gM, ga, gb
+
+
 def implicit_grads(P, M, a, b, reg, rtol=1e-12, max_iter=None):
     """(dL/dM, dL/da, dL/db) of L = sum(M * P) at the Sinkhorn solution P of
     (a, b, M, reg), in float64 (see the module docstring)."""
@@ -75,6 +100,11 @@ def implicit_grads(P, M, a, b, reg, rtol=1e-12, max_iter=None):
     M = M.double()
     a = a.double()
     b = b.double()
+    limit = max_iter or max(100, 4 * b.numel())
+    if P.is_cuda:
+        out = _native_grads(P, M, a, b, reg, rtol, limit)
+        if out is not None:
+            return out
     MP = M * P
     r, c = MP.sum(1), MP.sum(0)
     # bins of zero mass have zero rows / columns in P and drop out of the
@@ -97,7 +127,6 @@ def implicit_grads(P, M, a, b, reg, rtol=1e-12, max_iter=None):
     p = z.clone()
     rz = torch.dot(res, z)
     stop = (rtol * torch.linalg.vector_norm(rhs)) ** 2
-    limit = max_iter or max(100, 4 * b.numel())
     for _ in range(limit):
         if float(torch.dot(res, res)) <= float(stop):
             break

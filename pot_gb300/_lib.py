@@ -114,6 +114,9 @@ SIGNATURES = {
     "otg_lazy_loss": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_i64, c_i64, c_i32, c_vp, c_vp, c_dbl, c_vp, c_vp]),
     "otg_multi_tail_config": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(c_i32), ctypes.POINTER(c_i32),
                                               ctypes.POINTER(c_i64), ctypes.POINTER(c_i32)]),
+    "otg_sinkhorn_grad_workspace_bytes": (c_sz, [c_i64, c_i64]),
+    "otg_sinkhorn_grad": (ctypes.c_int, [c_vp, c_i64, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_dbl, c_dbl, c_i32, c_vp,
+                                         c_i64, c_vp, c_vp, c_vp, c_sz, c_vp, c_vp]),
     "otg_gibbs_kernel": (ctypes.c_int, [ctypes.c_int, c_vp, c_i64, c_i64, c_i64, c_dbl, c_vp, c_i64, c_vp]),
     "otg_dense_marginals": (ctypes.c_int, [ctypes.c_int, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_dbl, c_vp, c_vp,
                                            c_vp]),
