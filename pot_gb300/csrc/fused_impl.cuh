@@ -580,30 +580,33 @@ __device__ __noinline__ void fu_collse(const FusedArgs<T>& A_, const FuRow& R_, 
       T ui[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) ui[q] = row + q < R.gb ? __ldcg(u + row + q) : T(-INFINITY);
+      // the block's sixteen loads in flight at once (vectors beyond the row
+      // read its first one and are not stored)
+      T x[KB][4][W];
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
-        const int col = ((k0 + k) * R.gt + R.tg) * W;
-        if (col < A.mv && k0 + k < A.kv) {
-          T x[4][W];
+        const int at = ((k0 + k) * R.gt + R.tg) * W, col = at < A.mv ? at : 0;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int r = min(row + q, R.gb - 1);
-            if (TILE) fu_get(sm.data + (r - R.r0) * A.mp + col, x[q]);
-            else fu_get_global(A, r, col, pad, x[q]);
-          }
+        for (int q = 0; q < 4; ++q) {
+          const int r = min(row + q, R.gb - 1);
+          if (TILE) fu_get(sm.data + (r - R.r0) * A.mp + col, x[k][q]);
+          else fu_get_global(A, r, col, pad, x[k][q]);
+        }
+      }
 #pragma unroll
-          for (int w = 0; w < W; ++w) {
-            T t[4], top = mx[k][w];
+      for (int k = 0; k < KB; ++k) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) { t[q] = row + q < R.gb ? fma(x[q][w], A.c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
-            if (top != -INFINITY) {
-              T sum = s[k][w] * ex2(mx[k][w] - top);
+        for (int w = 0; w < W; ++w) {
+          T t[4], top = mx[k][w];
 #pragma unroll
-              for (int q = 0; q < 4; ++q) sum += ex2(t[q] - top);
-              s[k][w] = sum;
-              mx[k][w] = top;
-            }
-          }
+          for (int q = 0; q < 4; ++q) { t[q] = row + q < R.gb ? fma(x[k][q][w], A.c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
+          // (an empty column so far: the sums stay zero)
+          const T ref = top == -INFINITY ? T(0) : top;
+          T sum = s[k][w] * ex2(mx[k][w] - ref);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sum += ex2(t[q] - ref);
+          s[k][w] = sum;
+          mx[k][w] = top;
         }
       }
     }

@@ -383,31 +383,35 @@ __device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_,
         T ui[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) ui[q] = row + q < sp.end ? __ldcg(up + row + q) : (LOGF ? T(-INFINITY) : T(0));
+        // the block's sixteen loads in flight at once (vectors beyond the row
+        // read its first one and are not stored)
+        T x[KB][4][W];
 #pragma unroll
         for (int k = 0; k < KB; ++k) {
-          const int j = (k0 + k) * R.gt + R.tg;
-          if (j < nv) {
-            T x[4][W];
+          const int j = (k0 + k) * R.gt + R.tg < nv ? (k0 + k) * R.gt + R.tg : 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-              unpack(ld_stream(reinterpret_cast<const typename Vec<T>::type*>(Mp + (int64_t)min(row + q, sp.end - 1) * ldm) + j), x[q]);
+          for (int q = 0; q < 4; ++q)
+            unpack(ld_stream(reinterpret_cast<const typename Vec<T>::type*>(Mp + (int64_t)min(row + q, sp.end - 1) * ldm) + j), x[k][q]);
+        }
 #pragma unroll
-            for (int y = 0; y < W; ++y) {
-              if (LOGF) {
-                T t[4], top = mx[k][y];
+        for (int k = 0; k < KB; ++k) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) { t[q] = row + q < sp.end ? fma(x[q][y], c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
-                if (top != -INFINITY) {
-                  T sum = s[k][y] * ex2(mx[k][y] - top);
+          for (int y = 0; y < W; ++y) {
+            if (LOGF) {
+              // rows beyond the share have u = -inf
+              T t[4], top = mx[k][y];
 #pragma unroll
-                  for (int q = 0; q < 4; ++q) sum += ex2(t[q] - top);
-                  s[k][y] = sum;
-                  mx[k][y] = top;
-                }
-              } else {
+              for (int q = 0; q < 4; ++q) { t[q] = row + q < sp.end ? fma(x[k][q][y], c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
+              // (an empty column so far: the sums stay zero)
+              const T ref = top == -INFINITY ? T(0) : top;
+              T sum = s[k][y] * ex2(mx[k][y] - ref);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) s[k][y] = fma(ex2(x[q][y] * c), ui[q], s[k][y]);
-              }
+              for (int q = 0; q < 4; ++q) sum += ex2(t[q] - ref);
+              s[k][y] = sum;
+              mx[k][y] = top;
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) s[k][y] = fma(ex2(x[k][q][y] * c), ui[q], s[k][y]);
             }
           }
         }
