@@ -250,14 +250,33 @@ __global__ void __launch_bounds__(256) transpose_batched_kernel(const T* __restr
   }
 }
 
-// Plan and values per problem.  grid = (row tiles, problems).
+// Plan and values per problem.  grid = (tiles, problems).
 // out_vals[3p+0] = value_linear, [3p+1] = sum T log(T+1e-16) (entropy form)
 // or sum T log(T/(a b) + 1e-16) (KL form), [3p+2] = sum T.
+//
+// Bound by the read of M and the write of T.  A CTA takes 1024 columns (fewer
+// for narrow problems, with more rows side by side) of a range of rows; a
+// thread keeps what belongs to its 16-byte vector of columns in registers and
+// streams rows.  float: the logarithm of an entry is the exponent that the
+// entry is computed from, clamped at log 1e-16 (off by at most 0.7e-16 per
+// entry of the sum where T is that small), so there is no logarithm per entry;
+// the sums run in float over up to eight rows of a vector (32 entries) and in
+// fp64 beyond, as an fp64 addition issues at two lanes per clock.  double:
+// fp64 throughout.  128 problems of 512 x 512 float: 290 us with a row per
+// CTA, scalar loads, a logarithm and three fp64 additions per pair of entries.
+constexpr int PL_ROWS = 8;   // rows in flight, and between fp64 additions
 template <typename T, int METHOD>
-__global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t) {
+__global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int row_tiles) {
+  using V = typename Vec<T>::type;
+  constexpr int W = Vec<T>::N;
   const int p = blockIdx.y;
   if (p >= t.nprob) return;
   const int n = t.rows[p], m = t.cols[p], ldm = t.ldm[p];
+  const int nv = (m + W - 1) / W;
+  int cx = 256;                                    // vectors side by side
+  while (cx > 32 && cx / 2 >= nv) cx /= 2;
+  const int ry = 256 / cx, chunks = (nv + cx - 1) / cx;
+  const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const T* M = static_cast<const T*>(t.M) + t.m_off[p];
   const T* u = static_cast<const T*>(t.u) + t.r_off[p];
   const T* v = static_cast<const T*>(t.v) + t.c_off[p];
@@ -265,30 +284,71 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t) {
   const T* b = static_cast<const T*>(t.b) + t.c_off[p];
   T* P = t.P ? static_cast<T*>(t.P) + t.m_off[p] : nullptr;
   const T c = (T)(-OTG_LOG2E / t.reg[p]);
-  const T L2E = T(OTG_LOG2E);
-  // sums in the working type within a row, in fp64 across rows: float
-  // inputs keep their logarithms in fp32 (GB300's fp64 rate is a small
-  // fraction of fp32; a per-element fp64 log made this kernel the batch
-  // path's bottleneck), double inputs stay in fp64 throughout
+  const T L2E = T(OTG_LOG2E), LN2 = T(OTG_LN2), L16 = T(-36.841361487904734);  // log 1e-16
+  constexpr bool FAST = sizeof(T) == 4;
   double lin = 0, reg_term = 0, mass = 0;
-  for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    const T ui = u[i];
-    const T ai = a[i];
-    T lr = 0, rr = 0, mr = 0;
-    for (int j = threadIdx.x; j < m; j += blockDim.x) {
-      const T x = M[(int64_t)i * ldm + j];
-      T pij;
-      if (METHOD == OTG_METHOD_LOG) pij = ex2(fma(x, c, (ui + v[j]) * L2E));
-      else pij = ui * ex2(x * c) * v[j];
-      if (P) P[(int64_t)i * ldm + j] = pij;
-      lr = fma(x, pij, lr);
-      mr += pij;
-      if (t.kl) rr = fma(pij, log(pij / (ai * b[j]) + T(1e-16)), rr);
-      else rr = fma(pij, log(pij + T(1e-16)), rr);
+  for (int unit = blockIdx.x; unit < row_tiles * chunks; unit += gridDim.x) {
+    const int jv = (unit % chunks) * cx + tx, tile = unit / chunks;
+    const int i0 = (int)((int64_t)n * tile / row_tiles), i1 = (int)((int64_t)n * (tile + 1) / row_tiles);
+    if (jv >= nv) continue;
+    const int j0 = jv * W;
+    T vj[W], lv[W], bj[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const bool in = j0 + w < m;
+      vj[w] = in ? v[j0 + w] : T(0);
+      bj[w] = in ? b[j0 + w] : T(1);
+      // float: log2 of what the column brings to the entry, less log2 b (KL form)
+      if (FAST) lv[w] = (METHOD == OTG_METHOD_LOG ? T(0) : lg2(vj[w])) - (t.kl ? lg2(bj[w]) : T(0));
     }
-    lin += (double)lr;
-    mass += (double)mr;
-    reg_term += (double)rr;
+    for (int ib = i0 + ty; ib < i1; ib += PL_ROWS * ry) {
+      // the loads of eight rows in flight
+      T x[PL_ROWS][W], us[PL_ROWS], as[PL_ROWS];
+#pragma unroll
+      for (int q = 0; q < PL_ROWS; ++q) {
+        const int i = min(ib + q * ry, i1 - 1);
+        unpack(ld_stream(reinterpret_cast<const V*>(M + (int64_t)i * ldm) + jv), x[q]);
+        us[q] = u[i];
+        as[q] = t.kl ? a[i] : T(1);
+      }
+      T lr = 0, rr = 0, mr = 0;
+#pragma unroll
+      for (int q = 0; q < PL_ROWS; ++q) {
+        const int i = ib + q * ry;
+        if (i < i1) {
+          const T ui = us[q], ai = as[q];
+          T lu = 0;
+          if (FAST) lu = (METHOD == OTG_METHOD_LOG ? T(0) : lg2(ui)) - (t.kl ? lg2(ai) : T(0));
+          T pr[W];
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            T e;  // log2 of the entry without the scalings (scaling form), with the potentials (log form)
+            if (METHOD == OTG_METHOD_LOG) { e = fma(x[q][w], c, (ui + vj[w]) * L2E); pr[w] = ex2(e); }
+            else { e = x[q][w] * c; pr[w] = ui * ex2(e) * vj[w]; }
+            if (j0 + w < m) {
+              lr = fma(x[q][w], pr[w], lr);
+              mr += pr[w];
+              if (FAST) {
+                const T lg = (e + lu + lv[w]) * LN2;
+                rr = fma(pr[w], lg < L16 ? L16 : lg, rr);  // (a NaN stays one)
+              } else if (t.kl) {
+                rr = fma(pr[w], log(pr[w] / (ai * bj[w]) + T(1e-16)), rr);
+              } else {
+                rr = fma(pr[w], log(pr[w] + T(1e-16)), rr);
+              }
+            }
+          }
+          if (P) {
+            V o;
+            T* op = reinterpret_cast<T*>(&o);
+#pragma unroll
+            for (int w = 0; w < W; ++w) op[w] = pr[w];
+            reinterpret_cast<V*>(P + (int64_t)i * ldm)[jv] = o;
+          }
+        }
+      }
+      lin += (double)lr; mass += (double)mr; reg_term += (double)rr;
+    }
   }
   __shared__ double red[3][8];
   lin = warp_sum(lin); reg_term = warp_sum(reg_term); mass = warp_sum(mass);
@@ -630,13 +690,19 @@ int otg_batched_plan(const OtgPlanTable* t, int32_t max_rows, cudaStream_t strea
     return OTG_ERR_ARG;
   if (t->nprob > 65535) return OTG_ERR_UNSUPPORTED;
   if (cudaMemsetAsync(t->out_vals, 0, 3 * sizeof(double) * t->nprob, stream) != cudaSuccess) return OTG_ERR_CUDA;
-  dim3 grid(std::min(max_rows, 64), t->nprob);
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // row tiles: about eight CTAs per SM over the batch, at least 16 rows each
+  const int want = (sms * 8 + t->nprob - 1) / t->nprob;
+  const int row_tiles = std::max(1, std::min(want, (max_rows + 15) / 16));
+  dim3 grid((unsigned)row_tiles, t->nprob);
   if (t->dtype == OTG_F64) {
-    if (t->method == OTG_METHOD_LOG) batched_plan_kernel<double, OTG_METHOD_LOG><<<grid, 256, 0, stream>>>(*t);
-    else batched_plan_kernel<double, OTG_METHOD_KNOPP><<<grid, 256, 0, stream>>>(*t);
+    if (t->method == OTG_METHOD_LOG) batched_plan_kernel<double, OTG_METHOD_LOG><<<grid, 256, 0, stream>>>(*t, row_tiles);
+    else batched_plan_kernel<double, OTG_METHOD_KNOPP><<<grid, 256, 0, stream>>>(*t, row_tiles);
   } else if (t->dtype == OTG_F32) {
-    if (t->method == OTG_METHOD_LOG) batched_plan_kernel<float, OTG_METHOD_LOG><<<grid, 256, 0, stream>>>(*t);
-    else batched_plan_kernel<float, OTG_METHOD_KNOPP><<<grid, 256, 0, stream>>>(*t);
+    if (t->method == OTG_METHOD_LOG) batched_plan_kernel<float, OTG_METHOD_LOG><<<grid, 256, 0, stream>>>(*t, row_tiles);
+    else batched_plan_kernel<float, OTG_METHOD_KNOPP><<<grid, 256, 0, stream>>>(*t, row_tiles);
   } else {
     return OTG_ERR_DTYPE;
   }
