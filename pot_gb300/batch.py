@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from . import _lib, tune
-from ._arrays import Boundary, check_shape, shape_of
+from ._arrays import Boundary, check_shape, shape_of, upload
 from .utils import OTResult
 
 
@@ -34,9 +34,11 @@ class RaggedLayout:
 
     Problem p's cost block is rows[p] x ldm[p] elements starting at m_off[p]
     (ldm rounded up to 16 bytes; padded columns hold +inf); a/u slices start
-    at r_off[p], b/v slices at c_off[p]."""
+    at r_off[p], b/v slices at c_off[p].  With ``wait`` the tables are there
+    for every stream on return; without it, for work queued behind the
+    caller's current stream."""
 
-    def __init__(self, rows, cols, dtype, device):
+    def __init__(self, rows, cols, dtype, device, wait=True):
         rows = np.asarray(rows, dtype=np.int64)
         cols = np.asarray(cols, dtype=np.int64)
         vw = _vw(dtype)
@@ -52,15 +54,19 @@ class RaggedLayout:
         self.total_r = int(rows.sum())
         self.total_c = int(cols.sum())
         self.dtype, self.device = dtype, device
-        dev = device
-        self.rows = torch.tensor(rows, dtype=torch.int32, device=dev)
-        self.cols = torch.tensor(cols, dtype=torch.int32, device=dev)
-        self.ldm = torch.tensor(ldm, dtype=torch.int32, device=dev)
-        self.m_off = torch.tensor(m_off, dtype=torch.int64, device=dev)
-        self.r_off = torch.tensor(r_off, dtype=torch.int64, device=dev)
-        self.c_off = torch.tensor(c_off, dtype=torch.int64, device=dev)
         order = np.argsort(-(rows * cols), kind="stable").astype(np.int32)  # largest work first
-        self.order = torch.tensor(order, dtype=torch.int32, device=dev)
+        # row chunks of the two-pass batch kernel's column reductions
+        nsr_max = np.maximum(1, np.minimum(64, (rows + 15) // 16)).astype(np.int32)
+        partials = nsr_max.astype(np.int64) * cols
+        pc_off = np.concatenate([[0], np.cumsum(partials)[:-1]]).astype(np.int64)
+        self.max_ldm, self.chunk_partials = int(ldm.max()), int(partials.sum())
+        self.nsr_max_np = nsr_max
+        i32 = np.int32
+        (self.m_off, self.r_off, self.c_off, self.pc_off, self.rows, self.cols, self.ldm, self.order, self.nsr_max) = upload(
+            torch.device(device), [m_off.astype(np.int64), r_off.astype(np.int64), c_off.astype(np.int64), pc_off,
+                                   rows.astype(i32), cols.astype(i32), ldm.astype(i32), order, nsr_max])
+        if wait and self.rows.is_cuda:
+            torch.cuda.current_stream(self.rows.device).synchronize()
 
     def block(self, M_packed, p):
         o = int(self.m_off_np[p])
@@ -178,16 +184,10 @@ def _run_multi_once(layout, M_packed, a_packed, b_packed, reg, max_iter, tol, wa
     reg_t = torch.as_tensor(reg, dtype=torch.float64, device=dev).reshape(-1)
     if reg_t.numel() == 1:
         reg_t = reg_t.expand(B).contiguous()
-    if not hasattr(layout, "pc_off"):
-        nsr_max = np.maximum(1, np.minimum(64, (layout.rows_np + 15) // 16)).astype(np.int32)
-        sizes = nsr_max.astype(np.int64) * layout.cols_np
-        layout.nsr_max_np = nsr_max
-        layout.max_ldm = int(layout.ldm_np.max())
+    if not hasattr(layout, "total_partials"):
         # room for the row chunks' partials, or for the one-read kernel's worker slots
-        layout.total_partials = max(int(sizes.sum()), int(lib.otg_multi_partials(
+        layout.total_partials = max(layout.chunk_partials, int(lib.otg_multi_partials(
             _lib.dtype_code(dt), B, layout.total_c, layout.max_ldm)))
-        layout.nsr_max = torch.tensor(nsr_max, dtype=torch.int32, device=dev)
-        layout.pc_off = torch.tensor(np.concatenate([[0], np.cumsum(sizes)[:-1]]), dtype=torch.int64, device=dev)
     dcode = _lib.dtype_code(dt)
     wsb = lib.otg_multi_workspace_bytes(dcode, B, layout.total_r, layout.total_c, layout.total_partials)
     ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
@@ -257,9 +257,8 @@ def batched_sqdist(layout, X_packed, Y_packed, x_off, y_off, dims, want_max=Fals
     dev = layout.device
     M = torch.empty(layout.total_m, dtype=layout.dtype, device=dev)
     mx = torch.empty(layout.B, dtype=layout.dtype, device=dev) if want_max else None
-    dims_t = torch.as_tensor(np.asarray(dims, dtype=np.int32), device=dev)
-    xo = torch.as_tensor(np.asarray(x_off, dtype=np.int64), device=dev)
-    yo = torch.as_tensor(np.asarray(y_off, dtype=np.int64), device=dev)
+    xo, yo, dims_t = upload(dev, [np.asarray(x_off, dtype=np.int64), np.asarray(y_off, dtype=np.int64),
+                                  np.asarray(dims, dtype=np.int32)])
     t = _lib.OtgCostTable(dtype=_lib.dtype_code(layout.dtype), nprob=layout.B, X=X_packed.data_ptr(),
                           Y=Y_packed.data_ptr(), x_off=xo.data_ptr(), y_off=yo.data_ptr(),
                           rows=layout.rows.data_ptr(), cols=layout.cols.data_ptr(), dim=dims_t.data_ptr(),
@@ -275,7 +274,7 @@ def batched_sqdist(layout, X_packed, Y_packed, x_off, y_off, dims, want_max=Fals
 # ot.batch drop-ins
 # ---------------------------------------------------------------------------
 def _uniform_batch(M):
-    layout = RaggedLayout([M.shape[1]] * M.shape[0], [M.shape[2]] * M.shape[0], M.dtype, M.device)
+    layout = RaggedLayout([M.shape[1]] * M.shape[0], [M.shape[2]] * M.shape[0], M.dtype, M.device, wait=False)
     if layout.ldm_np[0] == M.shape[2] and M.is_contiguous() and M.data_ptr() % 16 == 0:
         Mp = M.reshape(-1)
     else:
@@ -298,7 +297,7 @@ def _transposed(layout, Mp):
     problems)."""
     lib = _lib.load()
     B, n, m = layout.B, int(layout.rows_np[0]), int(layout.cols_np[0])
-    lt = RaggedLayout([m] * B, [n] * B, layout.dtype, layout.device)
+    lt = RaggedLayout([m] * B, [n] * B, layout.dtype, layout.device, wait=False)
     ld, ldt = int(layout.ldm_np[0]), int(lt.ldm_np[0])
     Mt = torch.empty(lt.total_m, dtype=layout.dtype, device=layout.device)
     for z0 in range(0, B, _TRANSPOSE_CHUNK):
@@ -387,7 +386,7 @@ def dist_batch(X1, X2=None, metric="sqeuclidean", p=2, nx=None):
     Y = X if X2 is None else bd.to_dev(X2, X.dtype)
     B, n, d = X.shape
     m = Y.shape[1]
-    layout = RaggedLayout([n] * B, [m] * B, X.dtype, X.device)
+    layout = RaggedLayout([n] * B, [m] * B, X.dtype, X.device, wait=False)
     Mp, _ = batched_sqdist(layout, X.reshape(-1).contiguous(), Y.reshape(-1).contiguous(),
                            np.arange(B) * n * d, np.arange(B) * m * d, [d] * B)
     ld = int(layout.ldm_np[0])
@@ -476,9 +475,16 @@ def solve_sample_ragged(Xs, Ys, reg, as_=None, bs=None, reg_relative=False, max_
     rows = [x.shape[0] for x in Xs]
     cols = [y.shape[0] for y in Ys]
     dims = [x.shape[1] for x in Xs]
-    layout = RaggedLayout(rows, cols, dtype, device)
-    X = torch.cat([torch.as_tensor(np.asarray(x), dtype=dtype).reshape(-1) for x in Xs]).to(device)
-    Y = torch.cat([torch.as_tensor(np.asarray(y), dtype=dtype).reshape(-1) for y in Ys]).to(device)
+    layout = RaggedLayout(rows, cols, dtype, device, wait=False)
+    ndt = np.float32 if dtype == torch.float32 else np.float64
+
+    def packed(arrays):
+        return np.concatenate([np.asarray(x).reshape(-1) for x in arrays]).astype(ndt, copy=False)
+
+    def weights(ws, sizes):
+        return packed(ws) if ws is not None else np.repeat((1.0 / np.asarray(sizes, dtype=np.float64)).astype(ndt), sizes)
+
+    X, Y, ap, bp = upload(torch.device(device), [packed(Xs), packed(Ys), weights(as_, rows), weights(bs, cols)])
     x_off = np.concatenate([[0], np.cumsum([r * d for r, d in zip(rows, dims)])[:-1]])
     y_off = np.concatenate([[0], np.cumsum([c * d for c, d in zip(cols, dims)])[:-1]])
     M, mx = batched_sqdist(layout, X, Y, x_off, y_off, dims, want_max=reg_relative)
@@ -487,10 +493,6 @@ def solve_sample_ragged(Xs, Ys, reg, as_=None, bs=None, reg_relative=False, max_
         reg_t = reg_t.expand(B).contiguous()
     if reg_relative:
         reg_t = reg_t * mx.double()
-    ap = (torch.cat([torch.as_tensor(np.asarray(a), dtype=dtype) for a in as_]) if as_ is not None else
-          torch.cat([torch.full((r,), 1.0 / r, dtype=dtype) for r in rows])).to(device)
-    bp = (torch.cat([torch.as_tensor(np.asarray(b), dtype=dtype) for b in bs]) if bs is not None else
-          torch.cat([torch.full((c,), 1.0 / c, dtype=dtype) for c in cols])).to(device)
     code = _lib.OTG_METHOD_LOG if method == "sinkhorn_log" else _lib.OTG_METHOD_KNOPP
     wu = wv = None
     if warmstart is not None:

@@ -31,7 +31,7 @@ def _hist_cap(max_iter):
 
 
 class DenseResult:
-    __slots__ = ("u", "v", "status", "niter", "errs", "workspace", "layout", "nabs", "absorbed_last", "method", "K")
+    __slots__ = ("u", "v", "status", "niter", "errs", "workspace", "layout", "nabs", "absorbed_last", "method", "K", "hist")
 
 
 _SMS = {}
@@ -110,6 +110,7 @@ def solve_dense(M, a, b, reg, method, max_iter, stop_thr, warm_u=None, warm_v=No
     r.status, r.niter, r.errs = None, None, None
     r.layout = (dt, n, m, cap, grid)
     r.method = method
+    r.hist = None
     if read_back:
         read_result(r)
     return r
@@ -130,14 +131,19 @@ def read_result(r):
         r.status = _lib.STATUS_ABORTED
     # the unbalanced form logs the errors themselves, the others squared norms
     r.errs = hist[:nchk].copy() if r.method == _lib.OTG_METHOD_UNB else np.sqrt(hist[:nchk])
+    r.hist = r.workspace[off:off + 8 * nchk].view(torch.float64)  # the same on the device, squared but for the unbalanced form
     if r.status == _lib.STATUS_ABORTED:
         raise RuntimeError("pot_gb300: a device-side wait timed out; the solve was abandoned")
     return r
 
 
-def _errs_as(bd, errs, like):
+def _errs_as(bd, errs, like, r=None):
     if bd.kind == "numpy":
         return [np.float64(e) for e in errs]
+    if r is not None and not bd.host_torch:
+        # the device's own copy: no host round trip
+        t = r.hist if r.method == _lib.OTG_METHOD_UNB else torch.sqrt(r.hist)
+        return list(t.to(like.dtype, copy=True).unbind()) if len(errs) else []
     t = torch.as_tensor(np.asarray(errs, dtype=np.float64), dtype=like.dtype)
     if not bd.host_torch:
         t = t.to(like.device)
@@ -199,7 +205,17 @@ def _warm(bd, warmstart, dtype, n=None, m=None):
 
 def _run_single(bd, a, b, M, reg, method, numItermax, stopThr, verbose, warn, warmstart, want_plan):
     wu, wv = _warm(bd, warmstart, M.dtype, M.shape[0], M.shape[1])
-    r = solve_dense(M, a, b, reg, method, numItermax, stopThr, wu, wv)
+    r = solve_dense(M, a, b, reg, method, numItermax, stopThr, wu, wv, read_back=False)
+    P = None
+    lib = _lib.load()
+    if want_plan:
+        # launched behind the solve, before the host waits for its result
+        P = torch.empty_like(M)
+        _lib.check(lib.otg_dense_plan(_lib.dtype_code(M.dtype), method, ctypes.c_void_p(M.data_ptr()),
+                                      M.shape[0], M.shape[1], M.stride(0), _lib.ptr(r.u), _lib.ptr(r.v),
+                                      float(reg), _lib.ptr(P), P.stride(0), None,
+                                      _lib.stream_handle(M.device)), "otg_dense_plan")
+    read_result(r)
     if r.status == _lib.STATUS_NUMERICAL:
         warnings.warn("Warning: numerical errors at iteration %d" % r.niter)
     if verbose:
@@ -209,14 +225,6 @@ def _run_single(bd, a, b, M, reg, method, numItermax, stopThr, verbose, warn, wa
         _print_errs(errs, method == _lib.OTG_METHOD_LOG)
     if r.status == _lib.STATUS_MAXITER and warn:
         warnings.warn(NONCONV_MSG)
-    P = None
-    lib = _lib.load()
-    if want_plan:
-        P = torch.empty_like(M)
-        _lib.check(lib.otg_dense_plan(_lib.dtype_code(M.dtype), method, ctypes.c_void_p(M.data_ptr()),
-                                      M.shape[0], M.shape[1], M.stride(0), _lib.ptr(r.u), _lib.ptr(r.v),
-                                      float(reg), _lib.ptr(P), P.stride(0), None,
-                                      _lib.stream_handle(M.device)), "otg_dense_plan")
     return r, P
 
 
@@ -239,7 +247,7 @@ def sinkhorn_knopp(a, b, M, reg, numItermax=1000, stopThr=1e-9, verbose=False, l
     r, P = _run_single(bd, ad, bdv, Md, reg, _lib.OTG_METHOD_KNOPP, numItermax, stopThr, verbose,
                        warn, warmstart, True)
     if log:
-        lg = {"err": _errs_as(bd, r.errs, Md), "niter": r.niter, "u": bd.out(r.u), "v": bd.out(r.v)}
+        lg = {"err": _errs_as(bd, r.errs, Md, r), "niter": r.niter, "u": bd.out(r.u), "v": bd.out(r.v)}
         return bd.out(P), lg
     return bd.out(P)
 
@@ -253,7 +261,7 @@ def sinkhorn_log(a, b, M, reg, numItermax=1000, stopThr=1e-9, verbose=False, log
     r, P = _run_single(bd, ad, bdv, Md, reg, _lib.OTG_METHOD_LOG, numItermax, stopThr, verbose,
                        warn, warmstart, True)
     if log:
-        lg = {"err": _errs_as(bd, r.errs, Md), "niter": r.niter, "log_u": bd.out(r.u),
+        lg = {"err": _errs_as(bd, r.errs, Md, r), "niter": r.niter, "log_u": bd.out(r.u),
               "log_v": bd.out(r.v), "u": bd.out(torch.exp(r.u)), "v": bd.out(torch.exp(r.v))}
         return bd.out(P), lg
     return bd.out(P)
@@ -274,7 +282,7 @@ def _log_multi(bd, a, B, M, reg, numItermax, stopThr, verbose, log, warmstart):
     from . import batch as pb
     n, m = M.shape
     dt, dev = M.dtype, M.device
-    lay = pb.RaggedLayout([n] * H, [m] * H, dt, dev)
+    lay = pb.RaggedLayout([n] * H, [m] * H, dt, dev, wait=False)
     ld = int(lay.ldm_np[0])
     if ld == m and M.is_contiguous() and M.data_ptr() % 16 == 0:
         Mp = M.reshape(-1)
@@ -453,7 +461,7 @@ def _stabilized(bd, ad, bdv, Md, reg, numItermax, stopThr, warmstart, verbose, w
     lg = None
     if log:
         alpha, beta = reg * logu, reg * logv
-        lg = {"err": _errs_as(bd, r.errs, Md), "n_iter": r.niter, "logu": bd.out(logu), "logv": bd.out(logv),
+        lg = {"err": _errs_as(bd, r.errs, Md, r), "n_iter": r.niter, "logu": bd.out(logu), "logv": bd.out(logv),
               "alpha": bd.out(alpha), "beta": bd.out(beta), "warmstart": (bd.out(alpha), bd.out(beta))}
     return r, logu, logv, lg
 
@@ -609,9 +617,9 @@ def sinkhorn2(a, b, M, reg, method="sinkhorn", numItermax=1000, stopThr=1e-9, ve
     out = bd.scalar(loss)
     if log:
         if code == _lib.OTG_METHOD_KNOPP:
-            lg = {"err": _errs_as(bd, r.errs, Md), "niter": r.niter, "u": bd.out(r.u), "v": bd.out(r.v)}
+            lg = {"err": _errs_as(bd, r.errs, Md, r), "niter": r.niter, "u": bd.out(r.u), "v": bd.out(r.v)}
         else:
-            lg = {"err": _errs_as(bd, r.errs, Md), "niter": r.niter, "log_u": bd.out(r.u),
+            lg = {"err": _errs_as(bd, r.errs, Md, r), "niter": r.niter, "log_u": bd.out(r.u),
                   "log_v": bd.out(r.v), "u": bd.out(torch.exp(r.u)), "v": bd.out(torch.exp(r.v))}
         return out, lg
     return out

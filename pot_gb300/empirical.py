@@ -118,7 +118,7 @@ def empirical_sinkhorn(X_s, X_t, reg, a=None, b=None, metric="sqeuclidean", numI
     ad = torch.full((ns,), 1.0 / ns, dtype=dt, device=Xd.device) if a is None else bd.to_dev(a, dt)
     bv = torch.full((nt,), 1.0 / nt, dtype=dt, device=Xd.device) if b is None else bd.to_dev(b, dt)
     if not isLazy:
-        layout = pb.RaggedLayout([ns], [nt], dt, Xd.device)
+        layout = pb.RaggedLayout([ns], [nt], dt, Xd.device, wait=False)
         Mp, _ = pb.batched_sqdist(layout, Xd.reshape(-1).contiguous(), Yd.reshape(-1).contiguous(), [0], [0],
                                   [Xd.shape[1]])
         M = Mp.view(ns, int(layout.ldm_np[0]))[:, :nt]

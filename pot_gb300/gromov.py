@@ -56,12 +56,17 @@ class _Planes:
         return self
 
 
+def _bounds(C1, C2, p, q):
+    """[max |C1|, max |C2|, max p, max q] on the device."""
+    return torch.stack([C1.abs().max(), C2.abs().max(), p.max(), q.max()])
+
+
 class TensorProduct:
     """``G(T) = 2 constC - 2 C1 T hC2^T`` with hC2 = 2 C2 (square loss),
     i.e. gwggrad (``ot/gromov/_utils.py:323``); float32 inputs on the
     tensor cores, float64 on the fp64 GEMM."""
 
-    def __init__(self, C1, C2, p, q):
+    def __init__(self, C1, C2, p, q, bounds=None):
         self.dtype, self.device = C1.dtype, C1.device
         self.n, self.m = C1.shape[0], C2.shape[0]
         # constC_ij = alpha_i + beta_j, alpha = C1^2 p, beta = C2^2 q  (_utils.py:233-239)
@@ -73,12 +78,12 @@ class TensorProduct:
             n, m = self.n, self.m
             # exact power-of-two prescales: C1, hC2 from their maxima, T from
             # T_ij <= min(max p, max q), the product C1 T from sum_l T_lk = q_k
-            c1max = float(self.C1.abs().max())
+            c1max, c2max, pmax, qmax = (bounds if bounds is not None else _bounds(self.C1, C2, p, q).tolist())[:4]
             self.s1 = pow2_scale(c1max)
-            self.s2 = pow2_scale(float(self.hC2.abs().max()))
-            tmax = min(float(p.max()), float(q.max()))
+            self.s2 = pow2_scale(2.0 * c2max)
+            tmax = min(pmax, qmax)
             self.sT = pow2_scale(tmax)
-            self.e1 = pow2_scale(self.s1 * c1max * float(q.max()) * self.sT)
+            self.e1 = pow2_scale(self.s1 * c1max * qmax * self.sT)
             self.A1 = _Planes(n, n, self.device).fill(self.C1, self.s1)
             self.B2 = _Planes(m, m, self.device).fill(self.hC2, self.s2)
             self.Tt = _Planes(m, n, self.device)
@@ -213,10 +218,16 @@ def _entropic_gw(Mf, C1, C2, p, q, loss_fun, epsilon, symmetric, alpha, G0, max_
     pd = torch.full((n,), 1.0 / n, dtype=dt, device=dev) if p is None else bd.to_dev(p, dt)
     qd = torch.full((m,), 1.0 / m, dtype=dt, device=dev) if q is None else bd.to_dev(q, dt)
     T = torch.outer(pd, qd) if G0 is None else bd.to_dev(G0, dt).contiguous()
+    # the operands' bounds and symmetry in one read (torch.allclose of each matrix with its transpose)
+    facts = _bounds(C1d, C2d, pd, qd)
     if symmetric is None:
-        symmetric = bool(torch.allclose(C1d, C1d.T, atol=1e-10) and torch.allclose(C2d, C2d.T, atol=1e-10))
-    tp = TensorProduct(C1d, C2d, pd, qd)
-    tpt = None if symmetric else TensorProduct(C1d.T.contiguous(), C2d.T.contiguous(), pd, qd)
+        same = [torch.isclose(C, C.T, rtol=1e-5, atol=1e-10).all().to(dt)[None] for C in (C1d, C2d)]
+        facts = torch.cat([facts] + same)
+    facts = facts.tolist()
+    if symmetric is None:
+        symmetric = facts[4] == 1.0 and facts[5] == 1.0
+    tp = TensorProduct(C1d, C2d, pd, qd, facts)
+    tpt = None if symmetric else TensorProduct(C1d.T.contiguous(), C2d.T.contiguous(), pd, qd, facts)
     numItermax = kwargs.pop("numItermax", 1000)
     stopThr = kwargs.pop("stopThr", 1e-9)
     if warmstart:
@@ -252,12 +263,17 @@ def _entropic_gw(Mf, C1, C2, p, q, loss_fun, epsilon, symmetric, alpha, G0, max_
                     print("{:5s}|{:12s}".format("It.", "Err") + "\n" + "-" * 19)
                 print("{:5d}|{:8e}|".format(cpt, err))
         cpt += 1
-    tp.check_abort()
-    if abs(float(T.sum()) - 1) > 1e-5:
+    # mass, losses and the GEMMs' abort flag in one read
+    last = torch.stack([T.sum(), (tp.grad(T) * T).sum(), (Mfd * T).sum() if Mfd is not None else T.new_zeros(())]).double()
+    if dt == torch.float32:
+        last = torch.cat([last, tp.flag.double()])
+    last = last.tolist()
+    if len(last) > 3 and last[3] != 0.0:
+        tp.check_abort()
+    if abs(last[0] - 1) > 1e-5:
         warnings.warn("Solver failed to produce a transport plan. You might "
                       "want to increase the regularization parameter `epsilon`.")
-    quad = 0.5 * float((tp.grad(T) * T).sum())
-    lin = 0.0 if Mfd is None else float((Mfd * T).sum())
+    quad, lin = 0.5 * last[1], last[2]
     dist = (1.0 - alpha) * lin + alpha * quad if Mfd is not None else quad
     out = {"err": [torch.tensor(e) for e in errs] if bd.kind == "torch" else errs,
            "dist": bd.scalar(torch.tensor(dist, dtype=dt, device=dev)), "dist_f": dist, "lin": lin, "bd": bd}

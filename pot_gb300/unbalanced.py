@@ -31,7 +31,7 @@ def _pair(reg_m):
 
 
 def _kl_vec(p, q):
-    return float(torch.sum(p * torch.log(p / q + 1e-16)))
+    return torch.sum(p * torch.log(p / q + 1e-16))
 
 
 def sinkhorn_knopp_unbalanced(a, b, M, reg, reg_m, reg_type="kl", c=None, warmstart=None, numItermax=1000,
@@ -76,11 +76,12 @@ def sinkhorn_knopp_unbalanced(a, b, M, reg, reg_m, reg_type="kl", c=None, warmst
     if not log:
         return bd.out(P)
     Morig = bd.to_dev(M, Md.dtype) if cd is not None else Md
-    cost = float(vals[0, 0]) if cd is None else float(torch.sum(P * Morig))
+    # the costs stay on the device, in double
+    cost = vals[0, 0] if cd is None else torch.sum(P * Morig).double()
     if cd is not None:
-        reg_term = float(torch.sum(P * torch.log(P / cd + 1e-16)))
+        reg_term = torch.sum(P * torch.log(P / cd + 1e-16)).double()
     else:
-        reg_term = float(vals[0, 1])  # sum P log(P / c + 1e-16) for c = a b^T or c = 1
+        reg_term = vals[0, 1]  # sum P log(P / c + 1e-16) for c = a b^T or c = 1
     total = cost + reg * reg_term
     if rm1 != float("inf") or rm2 != float("inf"):
         lib = _lib.load()
@@ -91,13 +92,12 @@ def sinkhorn_knopp_unbalanced(a, b, M, reg, reg_m, reg_type="kl", c=None, warmst
                                            Md.stride(0), _lib.ptr(lu), _lib.ptr(lv), reg, _lib.ptr(rows),
                                            _lib.ptr(cols), _lib.stream_handle(Md.device)), "otg_dense_marginals")
         if rm1 != float("inf"):
-            total += rm1 * _kl_vec(rows, ad.double())
+            total = total + rm1 * _kl_vec(rows, ad.double())
         if rm2 != float("inf"):
-            total += rm2 * _kl_vec(cols, bv.double())
-    lg = {"err": _errs_as(bd, r.errs, Md), "logu": bd.out(torch.log(u + 1e-300)),
+            total = total + rm2 * _kl_vec(cols, bv.double())
+    lg = {"err": _errs_as(bd, r.errs, Md, r), "logu": bd.out(torch.log(u + 1e-300)),
           "logv": bd.out(torch.log(v + 1e-300)),
-          "cost": bd.scalar(torch.tensor(cost, dtype=Md.dtype, device=Md.device)),
-          "total_cost": bd.scalar(torch.tensor(total, dtype=Md.dtype, device=Md.device))}
+          "cost": bd.scalar(cost.to(Md.dtype)), "total_cost": bd.scalar(total.to(Md.dtype))}
     return bd.out(P), lg
 
 
