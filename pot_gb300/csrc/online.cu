@@ -316,26 +316,12 @@ __device__ __forceinline__ OlRowIn ol_row_in(const OnlinePass& P, int64_t ri, bo
   return v;
 }
 
+// One row's results from its base-2 (max, sum) (OL_FSUM: sum); false for a
+// row that failed.
 template <int MODE>
-__device__ __forceinline__ bool ol_rows_out(const OnlinePass& P, const float* red, int row_local, float mx, float sm,
-                                            int r0, int64_t rbase, int cs, const OlRowIn& in) {
+__device__ __forceinline__ bool ol_row_finish(const OnlinePass& P, int row, int64_t ri, float mx, float sm,
+                                              const OlRowIn& in) {
   constexpr bool FOLD = MODE == OL_FMAX || MODE == OL_FSUM;
-  if constexpr (MODE == OL_FSUM) {
-    for (int g = 0; g < 3; ++g) sm += red[g * 2 * OL_M + OL_M + row_local];
-  } else {
-    for (int g = 0; g < 3; ++g) lse_merge(mx, sm, red[g * 2 * OL_M + row_local], red[g * 2 * OL_M + OL_M + row_local]);
-  }
-  const int row = r0 + row_local;
-  const int64_t ri = rbase + row;  // the row in the packed vectors
-  if constexpr (MODE == OL_MAXP) {
-    if (row < P.n_rows) P.pot_out2[ri] = mx + in.rterm;
-    return true;
-  }
-  if (MODE != OL_FSUM && P.split > 1) {
-    P.part[((size_t)cs * 2) * P.rows_pad + row] = mx;
-    P.part[((size_t)cs * 2 + 1) * P.rows_pad + row] = sm;
-    return true;
-  }
   if (row >= P.n_rows) {
     if constexpr (!FOLD) P.h_out[ri] = -INFINITY;  // padding rows of the resident side
     return true;                                     // (folded: the str form keeps its padding values)
@@ -370,6 +356,28 @@ __device__ __forceinline__ bool ol_rows_out(const OnlinePass& P, const float* re
     P.h_out[ri] = hn;
   }
   return true;
+}
+
+template <int MODE>
+__device__ __forceinline__ bool ol_rows_out(const OnlinePass& P, const float* red, int row_local, float mx, float sm,
+                                            int r0, int64_t rbase, int cs, const OlRowIn& in) {
+  if constexpr (MODE == OL_FSUM) {
+    for (int g = 0; g < 3; ++g) sm += red[g * 2 * OL_M + OL_M + row_local];
+  } else {
+    for (int g = 0; g < 3; ++g) lse_merge(mx, sm, red[g * 2 * OL_M + row_local], red[g * 2 * OL_M + OL_M + row_local]);
+  }
+  const int row = r0 + row_local;
+  const int64_t ri = rbase + row;  // the row in the packed vectors
+  if constexpr (MODE == OL_MAXP) {
+    if (row < P.n_rows) P.pot_out2[ri] = mx + in.rterm;
+    return true;
+  }
+  if (MODE != OL_FSUM && P.split > 1) {
+    P.part[((size_t)cs * 2) * P.rows_pad + row] = mx;
+    P.part[((size_t)cs * 2 + 1) * P.rows_pad + row] = sm;
+    return true;
+  }
+  return ol_row_finish<MODE>(P, row, ri, mx, sm, in);
 }
 
 // Shared-memory carve-up of both pass kernels:
@@ -472,7 +480,7 @@ __global__ void __launch_bounds__(OL_THREADS, 1)
 online_pass_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constant__ CUtensorMap tAl,
                    const __grid_constant__ CUtensorMap tBh, const __grid_constant__ CUtensorMap tBl,
                    const __grid_constant__ CUtensorMap tR, const __grid_constant__ CUtensorMap tS, OnlinePass P) {
-  constexpr bool FOLD = MODE == OL_FMAX || MODE == OL_FSUM;
+  constexpr bool FOLD = MODE == OL_FMAX;  // (shifted-sum passes: online_stream_kernel)
   extern __shared__ unsigned char smem_raw[];
   const OlSmem S = ol_carve(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -582,11 +590,7 @@ online_pass_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constan
     // merge the four column groups of each row
     if (cgrp > 0) { S.red[(cgrp - 1) * 2 * OL_M + row_local] = mx; S.red[(cgrp - 1) * 2 * OL_M + OL_M + row_local] = sm; }
     named_bar(1, OL_EPI * 32);
-    if (cgrp == 0 && ok && !ol_rows_out<MODE>(P, S.red, row_local, mx, sm, r0, 0, cs, rin)) *S.uflag = 1;
-    if constexpr (MODE == OL_FSUM) {
-      named_bar(1, OL_EPI * 32);
-      if (warp == 0 && lane == 0) ol_note_unit(P, S.uflag, 0, r0);
-    }
+    if (cgrp == 0 && ok) ol_rows_out<MODE>(P, S.red, row_local, mx, sm, r0, 0, cs, rin);
   }
   tc_fence_before();
   __syncthreads();
@@ -595,6 +599,10 @@ online_pass_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_constan
     tmem_dealloc(tmem, OL_NBUF * OL_N);
   }
 }
+
+}  // namespace otg
+#include "online_stream.cuh"
+namespace otg {
 
 // A batch of pairs: units (active slot, row block), taken by the CTAs in
 // turn (one CTA per SM keeps its TMEM, barriers and pipeline across its
@@ -1096,6 +1104,15 @@ size_t a16(size_t x) { return (x + 255) / 256 * 256; }
 
 constexpr int OL_MAX_SPLIT = 8;
 
+// Rows of a side of one problem: whole pairs of row blocks, whole 256-point tiles.
+int64_t ol_pad(int64_t n) { return (n + OS_N - 1) / OS_N * OS_N; }
+
+// Floats of a pass's partial results: (max, sum) pairs of a column split, or
+// the shifted-sum pass's slots (one per range, one more per row pair).
+size_t ol_part_floats(int64_t rows) {
+  return std::max(2 * (size_t)OL_MAX_SPLIT * (size_t)rows, ((size_t)OS_MAX_CLUSTERS + (size_t)rows / OS_N) * OS_N);
+}
+
 // Column split for a pass of `nb` row blocks over `tiles` streamed tiles:
 // the S in 1..8 whose grid (nb x S CTAs, one per SM at a time) loses the
 // least to its last partial wave, keeping at least 32 tiles per CTA (fewer
@@ -1126,6 +1143,9 @@ void ol_sum_window(float w, float& lo, float& hi) {
   }
 }
 
+size_t os_smem(bool narrow) { return (narrow ? OsGeo<true>::bytes : OsGeo<false>::bytes) + OS_SMEM_EXTRA; }
+static_assert(OsGeo<false>::bytes + OS_SMEM_EXTRA <= 232448, "shared memory of the shifted-sum pass");
+
 // Dynamic shared memory of every pass kernel instantiation (once).
 bool online_attr() {
   static std::once_flag once;
@@ -1134,7 +1154,8 @@ bool online_attr() {
     const int sm = (int)OL_SMEM;
     ok = cudaFuncSetAttribute(online_pass_kernel<OL_LSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
          cudaFuncSetAttribute(online_pass_kernel<OL_FMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
-         cudaFuncSetAttribute(online_pass_kernel<OL_FSUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
+         cudaFuncSetAttribute(online_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)os_smem(false)) == cudaSuccess &&
+         cudaFuncSetAttribute(online_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)os_smem(true)) == cudaSuccess &&
          cudaFuncSetAttribute(online_batch_kernel<OL_LSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
          cudaFuncSetAttribute(online_batch_kernel<OL_MAXP>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
          cudaFuncSetAttribute(online_batch_kernel<OL_FMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
@@ -1148,7 +1169,7 @@ bool online_attr() {
 extern "C" {
 
 size_t otg_online_workspace_bytes(int64_t n, int64_t m, int32_t d) {
-  const int64_t np = (n + 127) / 128 * 128, mp = (m + 127) / 128 * 128;
+  const int64_t np = ol_pad(n), mp = ol_pad(m);
   const int64_t dp = ol_plane_width(d);
   size_t b = 0;
   b += 2 * a16(2 * np * dp) + 2 * a16(2 * mp * dp);          // half planes
@@ -1156,10 +1177,11 @@ size_t otg_online_workspace_bytes(int64_t n, int64_t m, int32_t d) {
   b += a16(8 * 64);                                          // err slots, flag
   b += a16(8 * (size_t)std::max(np, mp));                    // per-row errors of a check pass
   b += a16(4 * np) + a16(4 * mp);                            // negated norms
-  b += a16(4 * 2 * (size_t)OL_MAX_SPLIT * (size_t)std::max(np, mp));  // column-split partials
+  b += a16(4 * ol_part_floats(std::max(np, mp)));            // partial results
   b += 2 * a16(32 * np) + 2 * a16(32 * mp);                  // extension columns (row, str form)
   b += a16(4 * np) + a16(4 * mp) + a16(np) + a16(mp);        // shifts, failure marks
   b += a16(4 * (size_t)std::max(np, mp) / OL_M + 64);        // failed units, fix-up counters
+  b += a16(4 * (size_t)std::max(np, mp) / OL_M);             // arrivals per row block
   return b;
 }
 
@@ -1169,7 +1191,7 @@ int otg_sinkhorn_online(const OtgOnlineProblem* p, cudaStream_t st) {
   if (p->n < 1 || p->m < 1 || p->d < 1 || p->d > 64 * OL_MAXKT || !(p->reg > 0)) return OTG_ERR_ARG;
   if (p->workspace_bytes < otg_online_workspace_bytes(p->n, p->m, p->d)) return OTG_ERR_WORKSPACE;
   const int64_t n = p->n, m = p->m;
-  const int64_t np = (n + 127) / 128 * 128, mp = (m + 127) / 128 * 128;
+  const int64_t np = ol_pad(n), mp = ol_pad(m);
   const int dp = ol_plane_width(p->d);
   const int nkt = dp == 16 ? 1 : dp / OL_K;  // K-tiles per streamed tile
   // folded passes (one K-tile): alpha in the planes, h and the row shift in
@@ -1195,7 +1217,7 @@ int otg_sinkhorn_online(const OtgOnlineProblem* p, cudaStream_t st) {
   double* erow = reinterpret_cast<double*>(take(8 * (size_t)std::max(np, mp)));
   float* nx = reinterpret_cast<float*>(take(4 * np));
   float* ny = reinterpret_cast<float*>(take(4 * mp));
-  float* part = reinterpret_cast<float*>(take(4 * 2 * (size_t)OL_MAX_SPLIT * (size_t)std::max(np, mp)));
+  float* part = reinterpret_cast<float*>(take(4 * ol_part_floats(std::max(np, mp))));
   // extension columns [row form, str form] of each side
   __half* xe[2];
   __half* ye[2];
@@ -1208,6 +1230,7 @@ int otg_sinkhorn_online(const OtgOnlineProblem* p, cudaStream_t st) {
   int* flist = reinterpret_cast<int*>(take(4 * (size_t)std::max(np, mp) / OL_M + 64));
   int* fcnt = flist + std::max(np, mp) / OL_M;
   unsigned* fdone = reinterpret_cast<unsigned*>(fcnt + 1);
+  unsigned* rcnt = reinterpret_cast<unsigned*>(take(4 * (size_t)std::max(np, mp) / OL_M));
   if (off > p->workspace_bytes) return OTG_ERR_WORKSPACE;
   const float k2 = (float)(OTG_LOG2E / p->reg);
   const float sx = p->scale_x, sy = p->scale_y;
@@ -1241,11 +1264,12 @@ int otg_sinkhorn_online(const OtgOnlineProblem* p, cudaStream_t st) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int split_f = choose_split((int)(np / OL_M), (int)(mp / OL_N), sms);
   const int split_g = choose_split((int)(mp / OL_M), (int)(np / OL_N), sms);
-  // one pass: the pass kernel over (row blocks x column split), then, when
-  // split, the merge of the partials; a shifted-sum pass is followed by its
-  // fix-up (the running-max pass over the units whose rows failed; empty
+  // one pass: the first of each side (and every pass of d > 64) the pass
+  // kernel over (row blocks x column split), then, when split, the merge of
+  // the partials; later ones the shifted sums, each followed by its fix-up (the running-max pass over the units whose rows failed; empty
   // and at once done when none did)
   // (check passes: the per-row errors go to erow, their sum to `eslot`)
+  const int max_clusters = std::max(1, std::min(sms / 2, OS_MAX_CLUSTERS));
   auto pass = [&](OnlinePass& P, const CUtensorMap& ah, const CUtensorMap& al, const CUtensorMap& bh,
                   const CUtensorMap& bl, const CUtensorMap& rx, const CUtensorMap& sx2, int64_t rows_pad, int split,
                   bool first, double* eslot_of_pass) {
@@ -1253,17 +1277,25 @@ int otg_sinkhorn_online(const OtgOnlineProblem* p, cudaStream_t st) {
     const dim3 grid((unsigned)(rows_pad / OL_M), (unsigned)split);
     if (!fold) {
       online_pass_kernel<OL_LSE><<<grid, OL_THREADS, OL_SMEM, st>>>(ah, al, bh, bl, ah, bh, P);
-    } else if (first || split > 1) {
+    } else if (first) {
       online_pass_kernel<OL_FMAX><<<grid, OL_THREADS, OL_SMEM, st>>>(ah, al, bh, bl, rx, sx2, P);
     } else {
-      online_pass_kernel<OL_FSUM><<<grid, OL_THREADS, OL_SMEM, st>>>(ah, al, bh, bl, rx, sx2, P);
+      P.split = 1;
+      OsWork W{(int)(rows_pad / OS_N), P.col_tiles * OL_N / OS_N, 0, part, rcnt};
+      // at least two tiles per range: a range that shares its rows pays about
+      // 2 us for the slots, a tile takes 0.9 us
+      W.clusters = (int)std::min<int64_t>((int64_t)W.row_pairs * std::max(1, W.tiles / 2), max_clusters);
+      if (P.narrow)
+        online_stream_kernel<true><<<2 * W.clusters, OL_THREADS, os_smem(true), st>>>(ah, al, bh, bl, rx, sx2, P, W);
+      else
+        online_stream_kernel<false><<<2 * W.clusters, OL_THREADS, os_smem(false), st>>>(ah, al, bh, bl, rx, sx2, P, W);
       OnlinePass Q = P;
       Q.fixup = 1; Q.units_enc = 1; Q.active = flist; Q.count = fcnt; Q.nrb = (int)(rows_pad / OL_M);
       Q.rows_per_pair = 0; Q.cols_per_pair = 0; Q.alpha_p = nullptr; Q.done_cnt = fdone;
       online_batch_kernel<OL_FMAX><<<(unsigned)std::min<int64_t>(rows_pad / OL_M, sms), OL_THREADS, OL_SMEM, st>>>(
           ah, al, bh, bl, rx, sx2, Q);
     }
-    if (split > 1) online_finalize_kernel<<<(unsigned)((rows_pad + 255) / 256), 256, 0, st>>>(P);
+    if (P.split > 1) online_finalize_kernel<<<(unsigned)((rows_pad + 255) / 256), 256, 0, st>>>(P);
     // the L1 error: the row slots summed in a fixed order (the same value in every run)
     if (P.err) slot_sum_kernel<1024><<<1, 1024, 0, st>>>(P.err, P.n_rows, eslot_of_pass);
   };
