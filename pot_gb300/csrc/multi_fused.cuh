@@ -436,11 +436,21 @@ __device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_,
 }
 
 // Merge over 32-column blocks of the active problems: the slots of a column
-// are added in worker order; with many workers per problem the 8 warps of a
+// are added in worker order, a block per warp, or (`split`) the 8 warps of a
 // CTA share a block's slots (their sums in warp order).  The place of the
 // first block (looked up once until the shares change) is in `P`.
 // fin(p, cj, b, v, mx, s) finishes column cj (packed like b) of problem p.
-struct MfPlace { int64_t lo, hi, base, co, b0, b1; int k, p, m, w0, w1; };
+struct MfPlace { int64_t lo, hi, base, co, b0, b1; int k, p, m, w0, w1, split; };
+
+// A block costs a warp about 1.0 us for its place, v and b and 0.6 us per eight
+// slots, all of it latency; split, the CTA 1.3 us and an eighth of the slots.
+// The split pays for few blocks with many slots (one problem of 1024 columns:
+// 130 slots) and loses as soon as a CTA has many blocks (256 problems of 512
+// columns, 7 slots: 27 blocks per CTA, 36 of 78 us per iteration).
+__device__ __forceinline__ bool mf_split(int64_t blocks, int na, int nact, int ctas) {
+  const int64_t r = (na / nact + 1 + 7) / 8;
+  return ((blocks + ctas - 1) / ctas) * (13 + 6 * r / FU_WARPS) < ((blocks + ctas * FU_WARPS - 1) / (ctas * FU_WARPS)) * (10 + 6 * r);
+}
 template <typename T>
 __device__ __forceinline__ void mf_place(const MultiArgs<T>& A, MfPlace& P, int64_t blk, int na, int nact) {
   MtSlot sl{P.k, P.lo, P.hi};
@@ -458,7 +468,8 @@ template <typename T>
 __device__ __noinline__ MfPlace mf_first_place(const MultiArgs<T>& A, int na, int nact) {
   const int64_t blocks = __ldcg(A.colpre + nact);
   MfPlace P{};
-  if (na > 4 * nact) mt_share(blocks, blockIdx.x, gridDim.x, P.b0, P.b1);
+  P.split = mf_split(blocks, na, nact, gridDim.x);
+  if (P.split) mt_share(blocks, blockIdx.x, gridDim.x, P.b0, P.b1);
   else mt_share(blocks, (long)blockIdx.x * FU_WARPS + (threadIdx.x >> 5), (long)gridDim.x * FU_WARPS, P.b0, P.b1);
   P.k = -1;
   if (P.b0 < P.b1) mf_place(A, P, P.b0, na, nact);
@@ -468,8 +479,8 @@ template <typename T, bool PAIRS, typename Fin>
 __device__ __forceinline__ void mf_merge(const MultiArgs<T>& A, const MfPlace& first, int na, int nact, T (*scr)[2][32], bool flagged,
                                          const T* vcur, Fin&& fin) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool split = na > 4 * nact;
   MfPlace P = first;
+  const bool split = P.split;
   for (int64_t blk = P.b0; blk < P.b1; ++blk) {
     mf_place(A, P, blk, na, nact);
     if (flagged && __ldcg(A.fbad + P.p) == 0) continue;
