@@ -943,7 +943,7 @@ int launch_multi(const OtgMultiProblem* q, cudaStream_t st) {
   const int64_t need = fused_partials(q->dtype, q->nprob, q->total_cols, q->max_ldm);
   if (need > 0 && need <= q->total_partials && fused_plan_here(q->dtype, q->max_ldm, f)) {
     // one read of the blocks per iteration
-    A.fG = f.G; A.fNC = f.NC; A.fmp = f.mp; A.fmm = q->max_ldm;
+    A.fG = f.G; A.fNK = f.NK; A.fNC = f.NC; A.fmp = f.mp; A.fmm = q->max_ldm;
     const int64_t span = fused_span(q->dtype, q->nprob, q->total_cols, q->max_ldm, f, sms);
     A.fpart = reinterpret_cast<T*>(A.pcol);
     A.fpairs = A.fpart + span;

@@ -70,7 +70,7 @@ struct MultiArgs {
   // one-read kernel (multi_fused.cuh): warps per row, ring chunks per worker,
   // columns of a worker's v, widest block; column sums and (maximum, sum)
   // pairs of the workers; per problem: column sums too small to trust
-  int fG, fNC, fmp, fmm;
+  int fG, fNK, fNC, fmp, fmm;
   T* fpart; T* fpairs;
   int32_t* fbad;
 };

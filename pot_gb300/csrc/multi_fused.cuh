@@ -40,8 +40,19 @@ struct MfRing { int slot; uint32_t phase; bool primed; };
 // A worker's share and place in it: problem slot k, rows [row, end) of it.
 struct MfSpan { int k, row, end; };
 
+// Cost of a row in a kernel of NK vectors per lane, in vectors.  A batch of
+// rows costs its chain of latencies whatever the width, then float32 its
+// bytes: per row 0.42 ns at 64 floats, 0.46 at 512, 0.68 at 1024 with NK = 8
+// (0.15 to 0.22 with NK = 2, 0.81 to 1.29 with 16).  float64 costs the
+// exponentials of the half or all of the NK vectors that are evaluated: 6.8
+// and 11.6 ns with NK = 4.  (Weights in proportion to the width left the
+// worker with the narrowest rows 2.2 times the mean on 256 ragged blocks.)
 template <typename T>
-__device__ __forceinline__ int mf_weight(int ldm) { return ldm / Vec<T>::N + 64; }
+__device__ __forceinline__ int mf_weight(const MultiArgs<T>& A, int ldm) {
+  const int nv = ldm / Vec<T>::N;
+  if (sizeof(T) == 8) return 2 * nv > A.fNK * A.fG * 32 ? 40 * A.fNK : 24 * A.fNK;
+  return nv + 45 * A.fNK * A.fG;
+}
 
 // Share [beg, end) of worker w in weight units.
 __device__ __forceinline__ void mf_range(int64_t total, int w, int na, int64_t& beg, int64_t& end) {
@@ -61,7 +72,7 @@ template <typename T>
 __device__ __forceinline__ MfSpan mf_span(const MultiArgs<T>& A, int k, int64_t beg, int64_t end) {
   const int p = __ldcg(A.active + k);
   const int64_t base = __ldcg(A.urow_pre + k);
-  const int wt = mf_weight<T>(A.ldm[p]), n = A.rows[p];
+  const int wt = mf_weight(A, A.ldm[p]), n = A.rows[p];
   MfSpan s;
   s.k = k;
   s.row = beg <= base ? 0 : (int)min((int64_t)n, (beg - base + wt - 1) / wt);
@@ -461,7 +472,7 @@ __device__ __forceinline__ void mf_place(const MultiArgs<T>& A, MfPlace& P, int6
   P.co = A.c_off[P.p];
   const int64_t pos = __ldcg(A.urow_pre + P.k), total = __ldcg(A.urow_pre + nact);
   P.w0 = mf_worker(total, na, pos);
-  P.w1 = mf_worker(total, na, pos + (int64_t)(A.rows[P.p] - 1) * mf_weight<T>(A.ldm[P.p]));
+  P.w1 = mf_worker(total, na, pos + (int64_t)(A.rows[P.p] - 1) * mf_weight(A, A.ldm[P.p]));
   P.base = __ldcg(A.ucol_pre + P.k);
 }
 template <typename T>
@@ -557,7 +568,7 @@ __device__ __noinline__ void mf_rebuild(const MultiArgs<T>& A, int nact, const i
     int64_t own[4] = {0, 0, 0, 0};
     if (k < na) {
       const int p = A.active[k], ldm = A.ldm[p];
-      own[0] = (int64_t)A.rows[p] * mf_weight<T>(ldm);
+      own[0] = (int64_t)A.rows[p] * mf_weight(A, ldm);
       own[1] = ldm;
       own[2] = (A.cols[p] + 31) / 32;
       own[3] = A.rows[p];
@@ -599,7 +610,7 @@ __device__ __noinline__ void mf_rebuild(const MultiArgs<T>& A, int nact, const i
     // eight rows per worker at least, and a share never lighter than a row
     // (each worker between a problem's first and last one then has a row of it)
     int64_t nw = s_run[3] / 8;
-    nw = min(nw, s_run[0] / mf_weight<T>(A.fmm));
+    nw = min(nw, s_run[0] / mf_weight(A, A.fmm));
     nw = max((int64_t)1, min(nw, (int64_t)nworkers));
     A.ctl[7] = (int)nw;
     A.ctl[2] = tail;
