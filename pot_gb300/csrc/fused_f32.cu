@@ -4,7 +4,7 @@
 namespace otg {
 template <> int fu_launch_log<float>(FusedArgs<float>& A, const FuPlan& f, bool abs, cudaStream_t st) {
   (void)abs;
-  return f.res ? fu_start_resident<float, FU_LOG>(A, f, st) : fu_start<float, FU_LOG, 16, false>(A, f, st);
+  return f.res ? fu_start_resident<float, FU_LOG>(A, f, st) : fu_start_streamed<float, FU_LOG>(A, f, st);
 }
 
 int fused_launch_f32(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st) { return fused_run<float>(p, fs, st); }

@@ -3,7 +3,7 @@
 
 namespace otg {
 template <> int fu_launch_log<double>(FusedArgs<double>& A, const FuPlan& f, bool abs, cudaStream_t st) {
-  return abs ? fu_start_resident<double, FU_ABS>(A, f, st) : f.res ? OTG_ERR_UNSUPPORTED : fu_start<double, FU_LOG, 16, false>(A, f, st);
+  return abs ? fu_start_resident<double, FU_ABS>(A, f, st) : f.res ? OTG_ERR_UNSUPPORTED : fu_start_streamed<double, FU_LOG>(A, f, st);
 }
 
 int fused_launch_f64(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st) { return fused_run<double>(p, fs, st); }

@@ -33,11 +33,12 @@
 //   fewest vectors per thread (NK) that cover a row and let the rows fit, so
 //   that up to 8 rows share one reduction (reduce-scatter over the warp, one
 //   barrier), one division and one read of v.
-//   Streamed (cost larger than the SMs' shared memory, 30 MB): NK = 16, one
+//   Streamed (cost larger than the SMs' shared memory, 30 MB): NK = 10 to 16,
+//   the even number that covers the row with the fewest groups' threads, one
 //   row at a time per group, so that one group's reduction overlaps another's
 //   exponentials.  A ring of bulk copies issued by one lane per group, in
-//   chunks of half a row; five or six chunks of 32 KB are in flight per SM,
-//   and the copies of the next pass's first rows cross the hand-over.
+//   chunks of half a row; 120 to 200 KB are in flight per SM, and the copies
+//   of the next pass's first rows cross the hand-over.
 //
 // Range of the shortcut.  Log form: the shift of row i is its previous
 // potential less log a_i, so e_ij is the row's previous plan entry over a_i
@@ -64,7 +65,7 @@
 
 namespace otg {
 
-constexpr int FU_RING = 6;  // most chunks in flight per group
+constexpr int FU_RING = 9;  // most chunks in flight per group
 enum { FU_LOG = 0, FU_SCAL = 1, FU_UNB = 2, FU_ABS = 3 };
 // flags that a CTA publishes with its merge
 enum { FU_BAD_ROW = 1, FU_BAD_COL = 2, FU_ABORT = 4 };
@@ -1168,12 +1169,19 @@ bool fu_plan(int64_t n, int64_t m, bool abs, int grid, const FuDevice& d, FuPlan
     if (f.res) return true;
   }
   if (abs) return false;
+  // a row's vectors beyond its end cost as much as the others: 4100 floats
+  // (1025 vectors, 9 per thread) took 27.1 us per pass over 3001 rows with
+  // NK = 16.  With up to 8 per thread the second half of 16 is left out.
   split(16);
-  f.kv = (int)((V + f.G * 32 - 1) / (f.G * 32));
-  const size_t half = sizeof(T) * (size_t)(FU_WARPS / f.G) * (f.mp / 2);  // 32 KB over the groups
+  const int need = (int)((V + f.G * 32 - 1) / (f.G * 32)), nk = need <= 8 ? 16 : std::max(10, (need + 1) / 2 * 2);
+  f.NK = nk;
+  f.mp = nk * f.G * 32 * W;
+  f.buf_elems = FU_WARPS / f.G > 1 ? std::max(FU_WARPS / f.G * f.mp, FU_WARPS * 32) : 0;
+  f.kv = need;
+  const size_t half = sizeof(T) * (size_t)(FU_WARPS / f.G) * (f.mp / 2);  // 20 to 32 KB over the groups
   for (f.NC = FU_RING; f.NC >= 4; --f.NC) {
     f.smem = sizeof(T) * ((size_t)f.mp + f.buf_elems) + f.NC * half + 16 * ((size_t)(FU_WARPS / f.G * f.NC + 1) / 2);
-    if (f.smem + fu_static_smem<T>(16) <= d.smem) return true;
+    if (f.smem + fu_static_smem<T>(nk) <= d.smem) return true;
   }
   return false;
 }
@@ -1228,6 +1236,16 @@ int fu_start_resident(FusedArgs<T>& A, const FuPlan& f, cudaStream_t st) {
     case 8: return fu_start<T, MODE, 8, true>(A, f, st);
     case 12: return fu_start<T, MODE, 12, true>(A, f, st);
     default: return fu_start<T, MODE, 16, true>(A, f, st);
+  }
+}
+
+template <typename T, int MODE>
+int fu_start_streamed(FusedArgs<T>& A, const FuPlan& f, cudaStream_t st) {
+  switch (f.NK) {
+    case 10: return fu_start<T, MODE, 10, false>(A, f, st);
+    case 12: return fu_start<T, MODE, 12, false>(A, f, st);
+    case 14: return fu_start<T, MODE, 14, false>(A, f, st);
+    default: return fu_start<T, MODE, 16, false>(A, f, st);
   }
 }
 

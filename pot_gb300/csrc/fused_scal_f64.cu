@@ -3,6 +3,6 @@
 
 namespace otg {
 template <> int fu_launch_scal<double>(FusedArgs<double>& A, const FuPlan& f, cudaStream_t st) {
-  return f.res ? fu_start_resident<double, FU_SCAL>(A, f, st) : fu_start<double, FU_SCAL, 16, false>(A, f, st);
+  return f.res ? fu_start_resident<double, FU_SCAL>(A, f, st) : fu_start_streamed<double, FU_SCAL>(A, f, st);
 }
 }  // namespace otg

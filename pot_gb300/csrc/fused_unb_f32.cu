@@ -3,6 +3,6 @@
 
 namespace otg {
 template <> int fu_launch_unb<float>(FusedArgs<float>& A, const FuPlan& f, cudaStream_t st) {
-  return f.res ? fu_start_resident<float, FU_UNB>(A, f, st) : fu_start<float, FU_UNB, 16, false>(A, f, st);
+  return f.res ? fu_start_resident<float, FU_UNB>(A, f, st) : fu_start_streamed<float, FU_UNB>(A, f, st);
 }
 }  // namespace otg

@@ -3,6 +3,6 @@
 
 namespace otg {
 template <> int fu_launch_unb<double>(FusedArgs<double>& A, const FuPlan& f, cudaStream_t st) {
-  return f.res ? fu_start_resident<double, FU_UNB>(A, f, st) : fu_start<double, FU_UNB, 16, false>(A, f, st);
+  return f.res ? fu_start_resident<double, FU_UNB>(A, f, st) : fu_start_streamed<double, FU_UNB>(A, f, st);
 }
 }  // namespace otg
