@@ -18,6 +18,82 @@ namespace otg {
 constexpr double AND_LAMBDA = 1e-10;   // Tikhonov term, relative to trace / D
 constexpr double AND_MAX_L1 = 1e4;     // larger sum |alpha|: restart with the plain step
 
+// The weights of the mixed iterate, by one warp: lane q < nh brings the dot
+// <r_new, R_q> and gets the weight of slot q.  Updates G; false: take the
+// plain step.
+//
+// (G + lambda I) w = 1 by Gauss-Jordan elimination with partial pivoting, a
+// row per lane (rows beyond nh are those of the identity).  A chain of
+// latencies: an FP64 division takes about 0.5 us here, so there is one per
+// pivot and two more (elimination with back substitution by the warp: 25 of
+// them, 27 us for a step; by one thread 60 us).
+__device__ __forceinline__ bool anderson_solve(int D, int nh, int s, double dot, double* G, int lane, double& w) {
+  constexpr int MD = OTG_ANDERSON_MAX_DEPTH;
+  double row[MD + 1], dots[MD];
+#pragma unroll
+  for (int j = 0; j < MD; ++j) dots[j] = __shfl_sync(0xffffffffu, dot, j);
+  if (lane < nh) {
+#pragma unroll
+    for (int j = 0; j < MD; ++j) row[j] = j < nh ? (lane == s ? dots[j] : j == s ? dot : __ldcg(G + lane * D + j)) : 0.0;
+    G[s * D + lane] = dot;
+    G[lane * D + s] = dot;
+  } else {
+#pragma unroll
+    for (int j = 0; j < MD; ++j) row[j] = j == lane ? 1.0 : 0.0;
+  }
+  row[MD] = lane < nh ? 1.0 : 0.0;
+  double diag = 0.0;
+#pragma unroll
+  for (int j = 0; j < MD; ++j) if (j == lane) diag = row[j];
+  double tr = 0.0;
+  for (int i = 0; i < nh; ++i) tr += __shfl_sync(0xffffffffu, diag, i);
+  const double lam = AND_LAMBDA * tr / nh;
+#pragma unroll
+  for (int j = 0; j < MD; ++j) if (j == lane && lane < nh) row[j] += lam;
+  bool ok = nh > 1 && tr > 0.0;
+#pragma unroll
+  for (int c = 0; c < MD; ++c) {
+    if (c < nh) {
+      // the first of the largest entries of the column at or below the diagonal
+      double best = lane >= c && lane < nh ? fabs(row[c]) : -1.0;
+      int piv = lane;
+#pragma unroll
+      for (int o = 1; o < MD; o *= 2) {
+        const double x = __shfl_xor_sync(0xffffffffu, best, o);
+        const int y = __shfl_xor_sync(0xffffffffu, piv, o);
+        if (x > best || (x == best && y < piv)) { best = x; piv = y; }
+      }
+      best = __shfl_sync(0xffffffffu, best, 0);
+      piv = __shfl_sync(0xffffffffu, piv, 0);
+      if (!(best > 0.0)) { ok = false; piv = c; }
+      const int from = lane == c ? piv : lane == piv ? c : lane;
+      double top[MD + 1];
+#pragma unroll
+      for (int j = 0; j <= MD; ++j) {
+        if (j >= c) {
+          row[j] = __shfl_sync(0xffffffffu, row[j], from);
+          top[j] = __shfl_sync(0xffffffffu, row[j], c);
+        }
+      }
+      if (lane != c && lane < nh && ok) {
+        const double f = row[c] / top[c];
+#pragma unroll
+        for (int j = 0; j <= MD; ++j) if (j > c) row[j] -= f * top[j];
+      }
+    }
+  }
+  double x = 0.0;
+#pragma unroll
+  for (int j = 0; j < MD; ++j) if (j == lane && lane < nh) x = row[MD] / row[j];
+  double sw = 0.0, l1 = 0.0;
+#pragma unroll
+  for (int i = MD - 1; i >= 0; --i) sw += __shfl_sync(0xffffffffu, x, i);
+  w = x / sw;
+#pragma unroll
+  for (int i = 0; i < MD; ++i) l1 += fabs(__shfl_sync(0xffffffffu, w, i));
+  return ok && isfinite(l1) && l1 < AND_MAX_L1;
+}
+
 // One problem's step, called by every thread of the CTA.  vold: v_k, vnew:
 // F(v_k) on entry and the mixed v on return, both at column offset `co`
 // (m columns); F and R: D history slots of stride `stride` (slot-major);
@@ -45,7 +121,7 @@ __device__ void anderson_step(int D, int m, int64_t co, int64_t stride, const T*
     for (int q = 0; q < MD; ++q) {
       if (q < nh) {
         const T rq = q == s ? r : __ldcg(R + (int64_t)q * stride + co + j);
-        acc[q] += (double)r * (double)rq;
+        acc[q] += widen(r) * widen(rq);
       }
     }
   }
@@ -78,79 +154,11 @@ __device__ void anderson_step(int D, int m, int64_t co, int64_t stride, const T*
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    // (G + lambda I) w = 1 by Gaussian elimination with partial pivoting, a
-    // row per lane (rows beyond nh are those of the identity): one thread's
-    // elimination, with the separate block sums, took 60 us of the step
     const int lane = threadIdx.x;
-    double row[MD + 1];
-    double tr = 0.0;
-    if (lane < nh) {
-#pragma unroll
-      for (int j = 0; j < MD; ++j) row[j] = j < nh ? (lane == s ? s_dot[j] : j == s ? s_dot[lane] : G[lane * D + j]) : 0.0;
-      G[s * D + lane] = s_dot[lane];
-      G[lane * D + s] = s_dot[lane];
-    } else {
-#pragma unroll
-      for (int j = 0; j < MD; ++j) row[j] = j == lane ? 1.0 : 0.0;
-    }
-    row[MD] = lane < nh ? 1.0 : 0.0;
-    double diag = 0.0;
-#pragma unroll
-    for (int j = 0; j < MD; ++j) if (j == lane) diag = row[j];
-    for (int i = 0; i < nh; ++i) tr += __shfl_sync(0xffffffffu, diag, i);
-    const double lam = AND_LAMBDA * tr / nh;
-#pragma unroll
-    for (int j = 0; j < MD; ++j) if (j == lane && lane < nh) row[j] += lam;
-    bool ok = nh > 1 && tr > 0.0;
-#pragma unroll
-    for (int c = 0; c < MD; ++c) {
-      if (c < nh) {
-        // the first of the largest entries of the column at or below the diagonal
-        int piv = c;
-        double best = fabs(__shfl_sync(0xffffffffu, row[c], c));
-        for (int i = c + 1; i < nh; ++i) {
-          const double x = fabs(__shfl_sync(0xffffffffu, row[c], i));
-          if (x > best) { best = x; piv = i; }
-        }
-        if (!(best > 0.0)) ok = false;
-        const int from = lane == c ? piv : lane == piv ? c : lane;
-        double top[MD + 1];
-#pragma unroll
-        for (int j = 0; j <= MD; ++j) {
-          row[j] = __shfl_sync(0xffffffffu, row[j], from);
-          top[j] = __shfl_sync(0xffffffffu, row[j], c);
-        }
-        if (lane > c && lane < nh && ok) {
-          const double f = row[c] / top[c];
-#pragma unroll
-          for (int j = 0; j <= MD; ++j) if (j >= c) row[j] -= f * top[j];
-        }
-      }
-    }
-    double w[MD];
-    double sw = 0.0, l1 = 0.0;
-#pragma unroll
-    for (int i = MD - 1; i >= 0; --i) {
-      w[i] = 0.0;
-      if (i < nh) {
-        double t = row[MD];
-#pragma unroll
-        for (int j = 0; j < MD; ++j) if (j > i && j < nh) t -= row[j] * w[j];
-        double x = 0.0;
-#pragma unroll
-        for (int j = 0; j < MD; ++j) if (j == i) x = t / row[j];
-        w[i] = __shfl_sync(0xffffffffu, x, i);
-        sw += w[i];
-      }
-    }
-    if (ok) {
-#pragma unroll
-      for (int i = 0; i < MD; ++i) if (i < nh) { w[i] /= sw; l1 += fabs(w[i]); }
-      ok = isfinite(l1) && l1 < AND_MAX_L1;
-    }
+    double w;
+    const bool ok = anderson_solve(D, nh, s, lane < MD ? s_dot[lane] : 0.0, G, lane, w);
+    if (lane < MD) s_alpha[lane] = w;
     if (lane == 0) {
-#pragma unroll
-      for (int i = 0; i < MD; ++i) s_alpha[i] = ok && i < nh ? w[i] : (i == s ? 1.0 : 0.0);
       // a first iterate, or a failed solve: the plain step; after a failure
       // the history restarts with the next iterate
       s_keep = ok;
@@ -161,7 +169,7 @@ __device__ void anderson_step(int D, int m, int64_t co, int64_t stride, const T*
   if (s_keep) {
     for (int j = threadIdx.x; j < m; j += blockDim.x) {
       double vm = 0.0;
-      for (int q = 0; q < nh; ++q) vm += s_alpha[q] * (double)__ldcg(F + (int64_t)q * stride + co + j);
+      for (int q = 0; q < nh; ++q) vm += s_alpha[q] * widen(__ldcg(F + (int64_t)q * stride + co + j));
       vnew[co + j] = (T)vm;
     }
   }

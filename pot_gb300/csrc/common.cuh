@@ -65,6 +65,17 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   return r;
 }
 
+// float -> double by integer operations (exact; denormals, infinities and NaN
+// by the conversion): the conversion issues at half a lane per clock and SM
+// here, a quarter of the rate of FP64 arithmetic.
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = b & 0x7f800000u, s = b & 0x80000000u;
+  if ((b << 1) == 0u) return __hiloint2double((int)s, 0);
+  if (e == 0u || e == 0x7f800000u) return (double)x;
+  return __hiloint2double((int)(s | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
 template <typename T> struct Vec;
 template <> struct Vec<float> { using type = float4; static constexpr int N = 4; };
 template <> struct Vec<double> { using type = double2; static constexpr int N = 2; };

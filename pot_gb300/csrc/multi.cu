@@ -842,7 +842,8 @@ TailCfg tail_config() {
 // Device bytes of the Anderson history: F and residual slots, Gram matrices, counts.
 size_t anderson_ws_bytes(size_t es, int64_t nprob, int64_t cols, int depth) {
   auto r = [](size_t b) { return (b + 255) / 256 * 256; };
-  return 2 * r(es * (size_t)depth * (size_t)cols) + r(8 * (size_t)nprob * depth * depth) + r(4 * (size_t)nprob);
+  return 2 * r(es * (size_t)depth * (size_t)cols) + r(8 * (size_t)nprob * depth * depth) + r(4 * (size_t)nprob) +
+         r(8 * OTG_ANDERSON_MAX_DEPTH * ((size_t)cols / 32 + (size_t)nprob)) + r(8 * (OTG_ANDERSON_MAX_DEPTH + 2) * (size_t)nprob);
 }
 
 // The one-read kernel's plan on the current device.
@@ -933,6 +934,8 @@ int launch_multi(const OtgMultiProblem* q, cudaStream_t st) {
     A.and_R = reinterpret_cast<T*>(atake(sizeof(T) * (size_t)A.and_depth * (size_t)q->total_cols));
     A.and_G = reinterpret_cast<double*>(atake(sizeof(double) * (size_t)q->nprob * A.and_depth * A.and_depth));
     A.and_cnt = reinterpret_cast<int32_t*>(atake(sizeof(int32_t) * (size_t)q->nprob));
+    A.and_part = reinterpret_cast<double*>(atake(8 * OTG_ANDERSON_MAX_DEPTH * ((size_t)q->total_cols / 32 + (size_t)q->nprob)));
+    A.and_w = reinterpret_cast<double*>(atake(8 * (OTG_ANDERSON_MAX_DEPTH + 2) * (size_t)q->nprob));
   }
   if (cudaMemsetAsync(ctlp, 0, 64, st) != cudaSuccess) return OTG_ERR_CUDA;
   int dev = 0, sms = 0, per = 0;

@@ -73,6 +73,7 @@ struct MultiArgs {
   int fG, fNK, fNC, fmp, fmm;
   T* fpart; T* fpairs;
   int32_t* fbad;
+  double* and_part; double* and_w;  // dots of the blocks of 32 columns, weights of the problems (mf_anderson)
 };
 
 // Tail kernel limits: columns, rows per CTA

@@ -534,6 +534,156 @@ __device__ __forceinline__ void mf_merge(const MultiArgs<T>& A, const MfPlace& f
   }
 }
 
+// ---------------------------------------------------------------------------
+// Anderson mixing of the next v (anderson.cuh), in three steps between grid
+// barriers: dots of the new residual with the history by blocks of 32 columns
+// over all warps, the weights by one warp per problem, the mixing by blocks.
+// A CTA per problem did the same in 145 us for 256 problems of 2048 columns:
+// two problems in a row on most SMs, each a chain of loads and of FP64.  Now
+// 100 us: dots 28, weights 20, mixing 23, the barriers and waits the rest.
+// ---------------------------------------------------------------------------
+constexpr int MF_ANDW = OTG_ANDERSON_MAX_DEPTH + 2;  // weights, whether to mix, slots in use
+constexpr int MF_ANDB = 4;                           // blocks of a warp in flight
+template <typename T>
+__device__ __noinline__ void mf_and_dots(const MultiArgs<T>& A, int nact, const T* vcur, const T* vnxt) {
+  constexpr int MD = OTG_ANDERSON_MAX_DEPTH;
+  const int lane = threadIdx.x & 31, D = A.and_depth;
+  int64_t b0, b1;
+  mt_share(__ldcg(A.colpre + nact), (long)blockIdx.x * FU_WARPS + (threadIdx.x >> 5), (long)gridDim.x * FU_WARPS, b0, b1);
+  MtSlot sl;
+  int64_t co = 0;
+  int m = 0, s = 0, nh = 0;
+  for (int64_t blk = b0; blk < b1;) {
+    if (sl.seek(A.colpre, nact, blk)) {
+      const int p = __ldcg(A.active + sl.k), cnt = __ldcg(A.and_cnt + p);
+      m = A.cols[p]; co = A.c_off[p];
+      s = cnt % D; nh = min(cnt + 1, D);
+    }
+    const int nb = (int)min((int64_t)MF_ANDB, min(b1, sl.hi) - blk), j0 = (int)(blk - sl.lo) * 32 + lane;
+    T f[MF_ANDB], r[MF_ANDB], h[MF_ANDB][MD];
+#pragma unroll
+    for (int i = 0; i < MF_ANDB; ++i) {
+      const int j = j0 + 32 * i;
+      const bool on = i < nb && j < m;
+      f[i] = on ? __ldcg(vnxt + co + j) : T(0);
+      r[i] = on ? __ldcg(vcur + co + j) : T(0);
+#pragma unroll
+      for (int q = 0; q < MD; ++q) h[i][q] = on && q < nh && q != s ? __ldcg(A.and_R + q * A.total_cols + co + j) : T(0);
+    }
+    double acc[MD];
+#pragma unroll
+    for (int q = 0; q < MD; ++q) acc[q] = 0.0;
+#pragma unroll
+    for (int i = 0; i < MF_ANDB; ++i) {
+      const int j = j0 + 32 * i;
+      if (i < nb) {
+        r[i] = f[i] - r[i];
+        if (j < m) {
+          A.and_F[s * A.total_cols + co + j] = f[i];
+          A.and_R[s * A.total_cols + co + j] = r[i];
+        }
+        const double rd = widen(r[i]);
+#pragma unroll
+        for (int q = 0; q < MD; ++q)
+          if (q < nh) acc[q] += rd * (q == s ? rd : widen(h[i][q]));
+      }
+    }
+    int o = 16;
+#pragma unroll
+    for (int g = MD / 2; g >= 1; g /= 2) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int q = 0; q < g; ++q) {
+        const double keep = up ? acc[q + g] : acc[q], give = up ? acc[q] : acc[q + g];
+        acc[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+      o >>= 1;
+    }
+    double d = acc[0];
+#pragma unroll
+    for (int q = 16 / MD; q > 0; q >>= 1) d += __shfl_xor_sync(0xffffffffu, d, q);
+    if (lane % (32 / MD) == 0) {
+      const int q = lane / (32 / MD);
+      A.and_part[blk * MD + q] = d;
+      for (int i = 1; i < nb; ++i) A.and_part[(blk + i) * MD + q] = 0.0;
+    }
+    blk += nb;
+  }
+}
+
+template <typename T>
+__device__ __noinline__ void mf_and_solve(const MultiArgs<T>& A, int nact) {
+  constexpr int MD = OTG_ANDERSON_MAX_DEPTH;
+  const int lane = threadIdx.x & 31, D = A.and_depth;
+  for (int k = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; k < nact; k += gridDim.x * FU_WARPS) {
+    const int p = __ldcg(A.active + k), cnt = __ldcg(A.and_cnt + p);
+    const int s = cnt % D, nh = min(cnt + 1, D);
+    const int64_t lo = __ldcg(A.colpre + k), hi = __ldcg(A.colpre + k + 1);
+    double d = 0.0;
+    for (int64_t b = lo + lane / MD; b < hi; b += 8 * (32 / MD)) {
+      double x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = b + i * (32 / MD) < hi ? __ldcg(A.and_part + (b + i * (32 / MD)) * MD + lane % MD) : 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) d += x[i];
+    }
+#pragma unroll
+    for (int o = MD; o < 32; o *= 2) d += __shfl_xor_sync(0xffffffffu, d, o);
+    double w;
+    const bool ok = anderson_solve(D, nh, s, d, A.and_G + (int64_t)p * D * D, lane, w);
+    double* out = A.and_w + (int64_t)p * MF_ANDW;
+    if (lane < MD) out[lane] = w;
+    if (lane == 0) {
+      out[MD] = ok ? 1.0 : 0.0;
+      out[MD + 1] = (double)nh;
+      // after a failure the history restarts with the next iterate
+      A.and_cnt[p] = ok || nh == 1 ? cnt + 1 : 0;
+    }
+  }
+}
+
+template <typename T>
+__device__ __noinline__ void mf_and_mix(const MultiArgs<T>& A, int nact, T* vnxt) {
+  constexpr int MD = OTG_ANDERSON_MAX_DEPTH;
+  const int lane = threadIdx.x & 31;
+  int64_t b0, b1;
+  mt_share(__ldcg(A.colpre + nact), (long)blockIdx.x * FU_WARPS + (threadIdx.x >> 5), (long)gridDim.x * FU_WARPS, b0, b1);
+  MtSlot sl;
+  int64_t co = 0;
+  int m = 0, nh = 0;
+  double w[MD];
+  for (int64_t blk = b0; blk < b1;) {
+    if (sl.seek(A.colpre, nact, blk)) {
+      const int p = __ldcg(A.active + sl.k);
+      m = A.cols[p]; co = A.c_off[p];
+      const double* at = A.and_w + (int64_t)p * MF_ANDW;
+#pragma unroll
+      for (int q = 0; q < MD; ++q) w[q] = __ldcg(at + q);
+      nh = __ldcg(at + MD) != 0.0 ? (int)__ldcg(at + MD + 1) : 0;
+    }
+    const int nb = (int)min((int64_t)MF_ANDB, min(b1, sl.hi) - blk), j0 = (int)(blk - sl.lo) * 32 + lane;
+    if (nh > 0) {  // (a plain step keeps F(v))
+      T h[MF_ANDB][MD];
+#pragma unroll
+      for (int i = 0; i < MF_ANDB; ++i)
+#pragma unroll
+        for (int q = 0; q < MD; ++q)
+          h[i][q] = q < nh && i < nb && j0 + 32 * i < m ? __ldcg(A.and_F + q * A.total_cols + co + j0 + 32 * i) : T(0);
+#pragma unroll
+      for (int i = 0; i < MF_ANDB; ++i) {
+        if (i < nb && j0 + 32 * i < m) {
+          double v = 0.0;
+#pragma unroll
+          for (int q = 0; q < MD; ++q)
+            if (q < nh) v += w[q] * widen(h[i][q]);
+          vnxt[co + j0 + 32 * i] = (T)v;
+        }
+      }
+    }
+    blk += nb;
+  }
+}
+
 // Active list and its prefix sums (one CTA): weights of the rows, padded
 // columns, 32-column blocks; the number of workers.
 template <typename T>
@@ -810,7 +960,11 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
     }
     if constexpr (LOGF) {
       if (A.and_depth > 0) {
-        mt_anderson<T>(A, nact, vcur, vnxt);
+        mf_and_dots<T>(A, nact, vcur, vnxt);
+        if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
+        mf_and_solve<T>(A, nact);
+        if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
+        mf_and_mix<T>(A, nact, vnxt);
         if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
       }
     }
