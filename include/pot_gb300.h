@@ -602,6 +602,17 @@ typedef struct OtgSplitGemm {
   int64_t batch;
   int64_t o_bstride, rowv_bstride, colv_bstride, addend_bstride;
 } OtgSplitGemm;
+/* otg_gw_facts: of the n x n matrix C1 and the m x m matrix C2 (contiguous)
+ * and the weights p, q: alpha = C1^2 p (n), beta = C2^2 q (m), facts[6]
+ * (double) = max |C1|, max |C2|, max p, max q, C1 symmetric, C2 symmetric (1
+ * or 0; check_symmetric == 0: both 1).  Symmetric: every |C_ij - C_ji| <=
+ * atol + rtol |C_ji| (the test of ot/gromov/_bregman.py:160-163).
+ * otg_gw_sums: out[0..2] = sum P, sum G o P, sum F o P (F null: 0) over
+ * `count` elements; out: 3 + 3 * 304 doubles, the rest scratch. */
+int otg_gw_facts(int dtype, const void* C1, int64_t n, const void* C2, int64_t m, const void* p, const void* q,
+                 int32_t check_symmetric, double rtol, double atol, double* facts, void* alpha, void* beta,
+                 cudaStream_t stream);
+int otg_gw_sums(int dtype, const void* P, const void* G, const void* F, int64_t count, double* out, cudaStream_t stream);
 int otg_split_half(const float* X, int64_t rows, int64_t cols, int64_t ldx, float scale, int transpose, void* hi,
                    void* lo, int64_t ld_out, cudaStream_t stream);
 int otg_gemm_split3(const OtgSplitGemm* g, cudaStream_t stream);

@@ -155,6 +155,9 @@ SIGNATURES = {
                                         c_i64, c_i64, c_vp, c_i64, c_i64, c_dbl, c_vp, c_i64, c_i64, c_i64, c_vp]),
     "otg_split_half": (ctypes.c_int, [c_vp, c_i64, c_i64, c_i64, ctypes.c_float, ctypes.c_int, c_vp, c_vp, c_i64,
                                       c_vp]),
+    "otg_gw_facts": (ctypes.c_int, [ctypes.c_int, c_vp, c_i64, c_vp, c_i64, c_vp, c_vp, c_i32, c_dbl, c_dbl, c_vp, c_vp,
+                                    c_vp, c_vp]),
+    "otg_gw_sums": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_vp, c_i64, c_vp, c_vp]),
     "otg_gemm_split3": (ctypes.c_int, [ctypes.POINTER(OtgSplitGemm), c_vp]),
     "otg_split_half_batched": (ctypes.c_int, [c_vp, c_i64, c_i64, c_i64, c_i64, ctypes.c_float, ctypes.c_int, c_vp,
                                               c_vp, c_i64, c_i64, c_i64, c_vp]),

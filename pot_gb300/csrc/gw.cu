@@ -264,6 +264,143 @@ __global__ void __launch_bounds__(256) split_half_kernel(const float* __restrict
   }
 }
 
+// ---------------------------------------------------------------------------
+// What the outer loop wants to know of the structure matrices before it
+// starts: alpha = C1^2 p, beta = C2^2 q, max |C1|, max |C2|, max p, max q and
+// whether the matrices are symmetric.  Bound by two reads of each matrix from
+// L2 and by latency; as some 35 elementwise and reduction launches it was
+// 0.35 ms of a 2048 x 2048 call, 20 us now.
+// ---------------------------------------------------------------------------
+template <typename T> __device__ __forceinline__ unsigned long long bits_of_abs(T x) {
+  return (unsigned long long)__double_as_longlong(fabs(widen(x)));  // orders like |x|, NaN last
+}
+
+// A warp per row: sum_j C_ij^2 w_j and max |C_ij|.  The last block: max w of
+// both sides (NaN if there is one), and the symmetry flags' start.
+template <typename T>
+__global__ void __launch_bounds__(256) gw_rows_kernel(const T* C1, int64_t n, const T* C2, int64_t m, const T* p, const T* q,
+                                                      double* facts, T* alpha, T* beta) {
+  __shared__ T s_mx[2][8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (blockIdx.x == gridDim.x - 1) {
+    for (int side = 0; side < 2; ++side) {
+      const T* w = side ? q : p;
+      const int64_t len = side ? m : n;
+      T mx = -INFINITY;
+      for (int64_t i = threadIdx.x; i < len; i += 256) mx = w[i] > mx || isnan(w[i]) ? w[i] : mx;
+      for (int o = 16; o > 0; o >>= 1) {
+        const T x = __shfl_xor_sync(0xffffffffu, mx, o);
+        mx = isnan(mx) ? mx : x > mx || isnan(x) ? x : mx;
+      }
+      if (lane == 0) s_mx[side][warp] = mx;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      T mx = s_mx[threadIdx.x][0];
+      for (int k = 1; k < 8; ++k) {
+        const T x = s_mx[threadIdx.x][k];
+        mx = isnan(mx) ? mx : x > mx || isnan(x) ? x : mx;
+      }
+      facts[2 + threadIdx.x] = (double)mx;
+      facts[4 + threadIdx.x] = 1.0;
+    }
+    return;
+  }
+  const int64_t b1 = (n + 7) / 8;
+  const bool second = blockIdx.x >= b1;
+  const T* C = second ? C2 : C1;
+  const T* w = second ? q : p;
+  const int64_t len = second ? m : n, row = (blockIdx.x - (second ? b1 : 0)) * 8 + warp;
+  if (row >= len) return;
+  const T* c = C + row * len;
+  // eight loads in flight, eight sums of their own
+  T s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, mx = 0;
+  bool bad = false;
+  for (int64_t j = lane; j < len; j += 256) {
+    T x[8], y[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const bool on = j + 32 * k < len;
+      x[k] = on ? __ldg(c + j + 32 * k) : T(0);
+      y[k] = on ? __ldg(w + j + 32 * k) : T(0);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      s[k] = fma(x[k] * x[k], y[k], s[k]);
+      mx = fmax(mx, fabs(x[k]));
+      bad |= isnan(x[k]);
+    }
+  }
+  const T t = warp_sum(((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+  mx = warp_max(mx);
+  if (__any_sync(0xffffffffu, bad)) mx = T(NAN);
+  if (lane == 0) {
+    (second ? beta : alpha)[row] = t;
+    atomicMax(reinterpret_cast<unsigned long long*>(facts) + (second ? 1 : 0), bits_of_abs(mx));
+  }
+}
+
+// Pairs of 32 x 32 tiles across the diagonal: clears the flag of a matrix
+// with an entry that is not close to its transpose (|a - b| <= atol +
+// rtol |b| both ways, or equal).
+template <typename T>
+__global__ void __launch_bounds__(256) gw_symmetric_kernel(const T* C1, int64_t n, const T* C2, int64_t m, T rtol, T atol,
+                                                           double* facts) {
+  __shared__ T tile[32][33];
+  const T* C = blockIdx.z ? C2 : C1;
+  const int64_t len = blockIdx.z ? m : n, r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
+  if (c0 < r0 || c0 >= len) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  T x[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t r = r0 + ty + 8 * k, c = c0 + tx;
+    x[k] = r < len && c < len ? C[r * len + c] : T(0);
+    const int64_t rt = c0 + ty + 8 * k, ct = r0 + tx;
+    tile[ty + 8 * k][tx] = rt < len && ct < len ? C[rt * len + ct] : T(0);
+  }
+  __syncthreads();
+  bool far = false;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const T a = x[k], b = tile[tx][ty + 8 * k], e = fabs(a - b);
+    far |= !(a == b || (isfinite(e) && e <= atol + fabs(rtol * a) && e <= atol + fabs(rtol * b)));
+  }
+  if (__any_sync(0xffffffffu, far) && tx == 0) facts[4 + blockIdx.z] = 0.0;
+}
+
+// sum T, sum G o T and (F given) sum F o T: float sums of up to eight terms,
+// fp64 beyond; blocks' sums in slots, added in order by a second launch.
+constexpr int GW_SUM_BLOCKS = 304;
+template <typename T>
+__global__ void __launch_bounds__(256) gw_sums_kernel(const T* P, const T* G, const T* F, int64_t count, double* part) {
+  double t[3] = {0.0, 0.0, 0.0};
+  for (int64_t i = (int64_t)blockIdx.x * 2048 + threadIdx.x; i < count; i += (int64_t)gridDim.x * 2048) {
+    T x[8], g[8], f[8], a[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const bool on = i + 256 * k < count;
+      x[k] = on ? __ldg(P + i + 256 * k) : T(0);
+      g[k] = on ? __ldg(G + i + 256 * k) : T(0);
+      f[k] = on && F ? __ldg(F + i + 256 * k) : T(0);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { a[0] += x[k]; a[1] = fma(g[k], x[k], a[1]); a[2] = fma(f[k], x[k], a[2]); }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] += widen(a[k]);
+  }
+  for (int k = 0; k < 3; ++k) {
+    const double s = block_sum_fixed(t[k]);
+    if (threadIdx.x == 0) part[k * GW_SUM_BLOCKS + blockIdx.x] = s;
+  }
+}
+__global__ void __launch_bounds__(256) gw_sums_final_kernel(const double* part, int blocks, double* out) {
+  for (int k = 0; k < 3; ++k) {
+    const double s = block_sum_slots(part + k * GW_SUM_BLOCKS, blocks);
+    if (threadIdx.x == 0) out[k] = s;
+  }
+}
+
 }  // namespace otg
 
 using namespace otg;
@@ -326,6 +463,41 @@ int otg_split_half_batched(const float* X, int64_t rows, int64_t cols, int64_t l
   if (grid.y > 65535 || batch > 65535) return OTG_ERR_UNSUPPORTED;
   split_half_kernel<<<grid, 256, 0, stream>>>(X, rows, cols, ldx, scale, transpose, static_cast<__half*>(hi),
                                               static_cast<__half*>(lo), ld_out, sx, so);
+  return cudaGetLastError() == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
+}
+
+int otg_gw_facts(int dtype, const void* C1, int64_t n, const void* C2, int64_t m, const void* p, const void* q,
+                 int32_t check_symmetric, double rtol, double atol, double* facts, void* alpha, void* beta,
+                 cudaStream_t stream) {
+  if (!C1 || !C2 || !p || !q || !facts || !alpha || !beta || n < 1 || m < 1) return OTG_ERR_ARG;
+  if (dtype != OTG_F32 && dtype != OTG_F64) return OTG_ERR_DTYPE;
+  const int64_t blocks = (n + 7) / 8 + (m + 7) / 8 + 1, tiles = (std::max(n, m) + 31) / 32;
+  if (blocks > INT32_MAX || tiles > 65535) return OTG_ERR_UNSUPPORTED;
+  if (cudaMemsetAsync(facts, 0, 6 * sizeof(double), stream) != cudaSuccess) return OTG_ERR_CUDA;
+  const dim3 grid((unsigned)tiles, (unsigned)tiles, 2);
+  auto run = [&](auto z) {
+    using T = decltype(z);
+    const T *c1 = static_cast<const T*>(C1), *c2 = static_cast<const T*>(C2);
+    gw_rows_kernel<T><<<(unsigned)blocks, 256, 0, stream>>>(c1, n, c2, m, static_cast<const T*>(p), static_cast<const T*>(q), facts,
+                                                            static_cast<T*>(alpha), static_cast<T*>(beta));
+    if (check_symmetric) gw_symmetric_kernel<T><<<grid, 256, 0, stream>>>(c1, n, c2, m, (T)rtol, (T)atol, facts);
+  };
+  if (dtype == OTG_F64) run(0.0); else run(0.f);
+  return cudaGetLastError() == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
+}
+
+int otg_gw_sums(int dtype, const void* P, const void* G, const void* F, int64_t count, double* out, cudaStream_t stream) {
+  if (!P || !G || !out || count < 1) return OTG_ERR_ARG;
+  if (dtype != OTG_F32 && dtype != OTG_F64) return OTG_ERR_DTYPE;
+  const int blocks = (int)std::min<int64_t>(GW_SUM_BLOCKS, (count + 2047) / 2048);
+  double* part = out + 3;
+  if (dtype == OTG_F64)
+    gw_sums_kernel<double><<<blocks, 256, 0, stream>>>(static_cast<const double*>(P), static_cast<const double*>(G),
+                                                       static_cast<const double*>(F), count, part);
+  else
+    gw_sums_kernel<float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(P), static_cast<const float*>(G),
+                                                      static_cast<const float*>(F), count, part);
+  gw_sums_final_kernel<<<1, 256, 0, stream>>>(part, blocks, out);
   return cudaGetLastError() == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
 }
 

@@ -44,8 +44,9 @@ class _Planes:
 
     def __init__(self, rows, cols, device):
         self.rows, self.cols = _pad(rows, 128), _pad(cols, 128)
-        self.hi = torch.zeros(self.rows, self.cols, dtype=torch.float16, device=device)
-        self.lo = torch.zeros_like(self.hi)
+        new = torch.empty if (self.rows, self.cols) == (rows, cols) else torch.zeros  # zeros beyond the data
+        self.hi = new(self.rows, self.cols, dtype=torch.float16, device=device)
+        self.lo = new(self.rows, self.cols, dtype=torch.float16, device=device)
 
     def fill(self, X, scale=1.0, transpose=False):
         lib = _lib.load()
@@ -56,9 +57,25 @@ class _Planes:
         return self
 
 
-def _bounds(C1, C2, p, q):
-    """[max |C1|, max |C2|, max p, max q] on the device."""
-    return torch.stack([C1.abs().max(), C2.abs().max(), p.max(), q.max()])
+def _facts(C1, C2, p, q, symmetric=False):
+    """([max |C1|, max |C2|, max p, max q, C1 symmetric, C2 symmetric] as
+    float64, C1^2 p, C2^2 q), all on the device; the symmetry (torch.allclose
+    of each matrix with its transpose) is tested on request."""
+    facts = torch.empty(6, dtype=torch.float64, device=C1.device)
+    alpha, beta = torch.empty_like(p), torch.empty_like(q)
+    _lib.check(_lib.load().otg_gw_facts(_lib.dtype_code(C1.dtype), _lib.ptr(C1), C1.shape[0], _lib.ptr(C2), C2.shape[0],
+                                        _lib.ptr(p), _lib.ptr(q), int(symmetric), 1e-5, 1e-10, _lib.ptr(facts),
+                                        _lib.ptr(alpha), _lib.ptr(beta), _lib.stream_handle(C1.device)), "otg_gw_facts")
+    return facts, alpha, beta
+
+
+def _sums(P, G, F=None):
+    """[sum P, sum G o P, sum F o P] as float64 on the device."""
+    out = torch.empty(3 + 3 * 304, dtype=torch.float64, device=P.device)
+    _lib.check(_lib.load().otg_gw_sums(_lib.dtype_code(P.dtype), _lib.ptr(P), _lib.ptr(G),
+                                       _lib.ptr(F) if F is not None else None, P.numel(), _lib.ptr(out),
+                                       _lib.stream_handle(P.device)), "otg_gw_sums")
+    return out[:3]
 
 
 class TensorProduct:
@@ -66,26 +83,29 @@ class TensorProduct:
     i.e. gwggrad (``ot/gromov/_utils.py:323``); float32 inputs on the
     tensor cores, float64 on the fp64 GEMM."""
 
-    def __init__(self, C1, C2, p, q, bounds=None):
+    def __init__(self, C1, C2, p, q, facts=None):
         self.dtype, self.device = C1.dtype, C1.device
         self.n, self.m = C1.shape[0], C2.shape[0]
         # constC_ij = alpha_i + beta_j, alpha = C1^2 p, beta = C2^2 q  (_utils.py:233-239)
-        self.alpha = ((C1 * C1) @ p).contiguous()
-        self.beta = ((C2 * C2) @ q).contiguous()
-        self.C1, self.hC2 = C1.contiguous(), (2.0 * C2).contiguous()
+        self.C1, C2 = C1.contiguous(), C2.contiguous()
+        if facts is None:
+            facts = _facts(self.C1, C2, p.contiguous(), q.contiguous())
+        bounds, self.alpha, self.beta = facts
         self.lib = _lib.load()
-        if self.dtype == torch.float32:
+        if self.dtype == torch.float64:
+            self.hC2 = 2.0 * C2
+        else:
             n, m = self.n, self.m
             # exact power-of-two prescales: C1, hC2 from their maxima, T from
             # T_ij <= min(max p, max q), the product C1 T from sum_l T_lk = q_k
-            c1max, c2max, pmax, qmax = (bounds if bounds is not None else _bounds(self.C1, C2, p, q).tolist())[:4]
+            c1max, c2max, pmax, qmax = (bounds if isinstance(bounds, list) else bounds.tolist())[:4]
             self.s1 = pow2_scale(c1max)
             self.s2 = pow2_scale(2.0 * c2max)
             tmax = min(pmax, qmax)
             self.sT = pow2_scale(tmax)
             self.e1 = pow2_scale(self.s1 * c1max * qmax * self.sT)
             self.A1 = _Planes(n, n, self.device).fill(self.C1, self.s1)
-            self.B2 = _Planes(m, m, self.device).fill(self.hC2, self.s2)
+            self.B2 = _Planes(m, m, self.device).fill(C2, 2.0 * self.s2)
             self.Tt = _Planes(m, n, self.device)
             self.P1 = _Planes(n, m, self.device)
             self.flag = torch.zeros(1, dtype=torch.int32, device=self.device)
@@ -210,24 +230,26 @@ def _entropic_gw(Mf, C1, C2, p, q, loss_fun, epsilon, symmetric, alpha, G0, max_
     kwargs = dict(kwargs)
     _check_gw_shapes(C1, C2, p, q, G0, Mf)
     bd = Boundary(C1, C2, p, q, G0, Mf)
-    C1d = bd.to_dev(C1)
-    C2d = bd.to_dev(C2, C1d.dtype)
+    C1d = bd.to_dev(C1).contiguous()
+    C2d = bd.to_dev(C2, C1d.dtype).contiguous()
     dt, dev = C1d.dtype, C1d.device
     n, m = C1d.shape[0], C2d.shape[0]
     Mfd = None if Mf is None else bd.to_dev(Mf, dt).contiguous()
     pd = torch.full((n,), 1.0 / n, dtype=dt, device=dev) if p is None else bd.to_dev(p, dt)
     qd = torch.full((m,), 1.0 / m, dtype=dt, device=dev) if q is None else bd.to_dev(q, dt)
     T = torch.outer(pd, qd) if G0 is None else bd.to_dev(G0, dt).contiguous()
-    # the operands' bounds and symmetry in one read (torch.allclose of each matrix with its transpose)
-    facts = _bounds(C1d, C2d, pd, qd)
-    if symmetric is None:
-        same = [torch.isclose(C, C.T, rtol=1e-5, atol=1e-10).all().to(dt)[None] for C in (C1d, C2d)]
-        facts = torch.cat([facts] + same)
+    # the operands' bounds and symmetry in one read
+    pc, qc = pd.contiguous(), qd.contiguous()
+    facts, c_row, c_col = _facts(C1d, C2d, pc, qc, symmetric is None)
     facts = facts.tolist()
     if symmetric is None:
         symmetric = facts[4] == 1.0 and facts[5] == 1.0
-    tp = TensorProduct(C1d, C2d, pd, qd, facts)
-    tpt = None if symmetric else TensorProduct(C1d.T.contiguous(), C2d.T.contiguous(), pd, qd, facts)
+    tp = TensorProduct(C1d, C2d, pd, qd, (facts, c_row, c_col))
+    if symmetric:
+        tpt = None
+    else:
+        C1t, C2t = C1d.T.contiguous(), C2d.T.contiguous()
+        tpt = TensorProduct(C1t, C2t, pd, qd, (facts,) + _facts(C1t, C2t, pc, qc)[1:])
     numItermax = kwargs.pop("numItermax", 1000)
     stopThr = kwargs.pop("stopThr", 1e-9)
     if warmstart:
@@ -264,7 +286,8 @@ def _entropic_gw(Mf, C1, C2, p, q, loss_fun, epsilon, symmetric, alpha, G0, max_
                 print("{:5d}|{:8e}|".format(cpt, err))
         cpt += 1
     # mass, losses and the GEMMs' abort flag in one read
-    last = torch.stack([T.sum(), (tp.grad(T) * T).sum(), (Mfd * T).sum() if Mfd is not None else T.new_zeros(())]).double()
+    T = T.contiguous()
+    last = _sums(T, tp.grad(T), Mfd)
     if dt == torch.float32:
         last = torch.cat([last, tp.flag.double()])
     last = last.tolist()
