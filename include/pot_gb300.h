@@ -156,6 +156,18 @@ int otg_gibbs_kernel(int dtype, const void* M, int64_t n, int64_t m, int64_t ldm
  * epsilon-scaling loop, ot/bregman/_sinkhorn.py:1534-1542. */
 int otg_dense_marginals(int dtype, const void* M, int64_t n, int64_t m, int64_t ldm, const void* u, const void* v,
                         double reg, double* rowsum, double* colsum, cudaStream_t stream);
+/* What sinkhorn_knopp_unbalanced returns beside the plan.  _vectors: ut = alw
+ * u, vt = bew v (null weights: copies), lu = log(u + 1e-300), lv.  _total:
+ * out[0] = vals[0] and out[1] = vals[0] + reg vals[1] + reg_m1 KL(P 1 | a) +
+ * reg_m2 KL(P^T 1 | b) in the working type (an infinite reg_m: no term), of
+ * the n x m plan P; KL(p | q) = sum p log(p / q + 1e-16).  scratch:
+ * otg_unbalanced_total_doubles() doubles. */
+int otg_unbalanced_vectors(int dtype, int64_t n, int64_t m, const void* u, const void* v, const void* alw, const void* bew,
+                           void* ut, void* vt, void* lu, void* lv, cudaStream_t stream);
+int64_t otg_unbalanced_total_doubles(int64_t n, int64_t m);
+int otg_unbalanced_total(int dtype, const void* P, int64_t n, int64_t m, int64_t ldp, const void* a, const void* b,
+                         const double* vals, double reg, double reg_m1, double reg_m2, double* scratch, void* out,
+                         cudaStream_t stream);
 
 /* Greenkhorn, the greedy coordinate Sinkhorn, on one dense problem.
  * Replaces ot/bregman/_sinkhorn.py:1034-1102 (greenkhorn, reached through

@@ -118,6 +118,11 @@ SIGNATURES = {
     "otg_sinkhorn_grad": (ctypes.c_int, [c_vp, c_i64, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_dbl, c_dbl, c_i32, c_vp,
                                          c_i64, c_vp, c_vp, c_vp, c_sz, c_vp, c_vp]),
     "otg_gibbs_kernel": (ctypes.c_int, [ctypes.c_int, c_vp, c_i64, c_i64, c_i64, c_dbl, c_vp, c_i64, c_vp]),
+    "otg_unbalanced_vectors": (ctypes.c_int, [ctypes.c_int, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp,
+                                              c_vp]),
+    "otg_unbalanced_total_doubles": (c_i64, [c_i64, c_i64]),
+    "otg_unbalanced_total": (ctypes.c_int, [ctypes.c_int, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_vp, c_dbl, c_dbl, c_dbl,
+                                            c_vp, c_vp, c_vp]),
     "otg_dense_marginals": (ctypes.c_int, [ctypes.c_int, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_dbl, c_vp, c_vp,
                                            c_vp]),
     "otg_greenkhorn_workspace_bytes": (c_sz, [ctypes.c_int, c_i64, c_i64]),

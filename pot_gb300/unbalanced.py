@@ -11,9 +11,8 @@ iteration, the previous pair kept on a zero ``K^T u`` or a non-finite
 scaling.  ``c = a b^T`` (``reg_type='kl'``) and ``c = 1``
 (``reg_type='entropy'``) are applied inside the passes; a user ``c`` is
 folded into the cost as ``M - reg log c``.  The plan and the costs of the
-log (``cost``, ``total_cost``) come from the plan and marginal kernels.
+log (``cost``, ``total_cost``) come from the plan kernel and ``csrc/unbalanced.cu``.
 """
-import ctypes
 import warnings
 
 import numpy as np
@@ -28,10 +27,6 @@ def _pair(reg_m):
     if isinstance(reg_m, (int, float)) or (hasattr(reg_m, "ndim") and np.ndim(reg_m) == 0):
         return float(reg_m), float(reg_m)
     return float(reg_m[0]), float(reg_m[1])
-
-
-def _kl_vec(p, q):
-    return torch.sum(p * torch.log(p / q + 1e-16))
 
 
 def sinkhorn_knopp_unbalanced(a, b, M, reg, reg_m, reg_type="kl", c=None, warmstart=None, numItermax=1000,
@@ -65,10 +60,13 @@ def sinkhorn_knopp_unbalanced(a, b, M, reg, reg_m, reg_type="kl", c=None, warmst
                 print("{:5s}|{:12s}".format("It.", "Err") + "\n" + "-" * 19)
             print("{:5d}|{:8e}|".format(i, e))
     u, v = r.u, r.v
-    al = torch.ones_like(u) if c_ones else ad
-    be = torch.ones_like(v) if c_ones else bv
-    ut, vt = (al * u).contiguous(), (be * v).contiguous()
     n, m = Md.shape
+    lib, st, code = _lib.load(), _lib.stream_handle(Md.device), _lib.dtype_code(Md.dtype)
+    ut, lu, vt, lv = torch.empty_like(u), torch.empty_like(u), torch.empty_like(v), torch.empty_like(v)
+    ac, bc = ad.contiguous(), bv.contiguous()
+    _lib.check(lib.otg_unbalanced_vectors(code, n, m, _lib.ptr(u), _lib.ptr(v), None if c_ones else _lib.ptr(ac),
+                                          None if c_ones else _lib.ptr(bc), _lib.ptr(ut), _lib.ptr(vt), _lib.ptr(lu),
+                                          _lib.ptr(lv), st), "otg_unbalanced_vectors")
     layout, Mp = pb._uniform_batch(Md[None])
     reg_t = torch.full((1,), reg, dtype=torch.float64, device=Md.device)
     P, vals = pb.batched_plan(layout, Mp, ut, vt, ad, bv, reg_t, _lib.OTG_METHOD_KNOPP, kl=not c_ones)
@@ -76,28 +74,15 @@ def sinkhorn_knopp_unbalanced(a, b, M, reg, reg_m, reg_type="kl", c=None, warmst
     if not log:
         return bd.out(P)
     Morig = bd.to_dev(M, Md.dtype) if cd is not None else Md
-    # the costs stay on the device, in double
-    cost = vals[0, 0] if cd is None else torch.sum(P * Morig).double()
+    # linear cost and sum P log(P / c + 1e-16); the latter comes with the plan for c = a b^T or c = 1
     if cd is not None:
-        reg_term = torch.sum(P * torch.log(P / cd + 1e-16)).double()
-    else:
-        reg_term = vals[0, 1]  # sum P log(P / c + 1e-16) for c = a b^T or c = 1
-    total = cost + reg * reg_term
-    if rm1 != float("inf") or rm2 != float("inf"):
-        lib = _lib.load()
-        rows = torch.empty(n, dtype=torch.float64, device=Md.device)
-        cols = torch.empty(m, dtype=torch.float64, device=Md.device)
-        lu, lv = torch.log(ut), torch.log(vt)
-        _lib.check(lib.otg_dense_marginals(_lib.dtype_code(Md.dtype), ctypes.c_void_p(Md.data_ptr()), n, m,
-                                           Md.stride(0), _lib.ptr(lu), _lib.ptr(lv), reg, _lib.ptr(rows),
-                                           _lib.ptr(cols), _lib.stream_handle(Md.device)), "otg_dense_marginals")
-        if rm1 != float("inf"):
-            total = total + rm1 * _kl_vec(rows, ad.double())
-        if rm2 != float("inf"):
-            total = total + rm2 * _kl_vec(cols, bv.double())
-    lg = {"err": _errs_as(bd, r.errs, Md, r), "logu": bd.out(torch.log(u + 1e-300)),
-          "logv": bd.out(torch.log(v + 1e-300)),
-          "cost": bd.scalar(cost.to(Md.dtype)), "total_cost": bd.scalar(total.to(Md.dtype))}
+        vals = torch.stack([torch.sum(P * Morig).double(), torch.sum(P * torch.log(P / cd + 1e-16)).double()])
+    scratch = torch.empty(lib.otg_unbalanced_total_doubles(n, m), dtype=torch.float64, device=Md.device)
+    costs = torch.empty(2, dtype=Md.dtype, device=Md.device)
+    _lib.check(lib.otg_unbalanced_total(code, _lib.ptr(P), n, m, m, _lib.ptr(ac), _lib.ptr(bc), _lib.ptr(vals), reg, rm1, rm2,
+                                        _lib.ptr(scratch), _lib.ptr(costs), st), "otg_unbalanced_total")
+    lg = {"err": _errs_as(bd, r.errs, Md, r), "logu": bd.out(lu), "logv": bd.out(lv),
+          "cost": bd.scalar(costs[0]), "total_cost": bd.scalar(costs[1])}
     return bd.out(P), lg
 
 
