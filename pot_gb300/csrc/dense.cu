@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(256) dense_rowsum_kernel(const T* __restrict__
   if (i >= n) return;
   const T ui = u[i] * L2E;
   double acc = 0.0;
-  for (int64_t j = lane; j < m; j += 32) acc += (double)ex2(fma(M[i * ldm + j], c, ui + v[j] * L2E));
+  for (int64_t j = lane; j < m; j += 32) acc += widen(ex2(fma(M[i * ldm + j], c, ui + v[j] * L2E)));
   acc = warp_sum(acc);
   if (lane == 0) rows[i] = acc;
 }
@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(256) dense_colsum_kernel(const T* __restrict__
   double acc = 0.0;
   if (j < m) {
     const T vj = v[j] * L2E;
-    for (int64_t i = warp; i < n; i += 8) acc += (double)ex2(fma(M[i * ldm + j], c, u[i] * L2E + vj));
+    for (int64_t i = warp; i < n; i += 8) acc += widen(ex2(fma(M[i * ldm + j], c, u[i] * L2E + vj)));
   }
   part[warp][lane] = acc;
   __syncthreads();

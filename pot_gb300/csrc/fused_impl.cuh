@@ -909,43 +909,51 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
       if (threadIdx.x < 6) {
         T t = s_mx[threadIdx.x][0];
         for (int w = 1; w < FU_WARPS; ++w) t = fmax(t, s_mx[threadIdx.x][w]);
-        Ll<double>::put(A.ell + 12 * (int64_t)blockIdx.x + 2 * threadIdx.x, (double)t, ep);
+        Ll<T>::put(A.ell + 12 * (int64_t)blockIdx.x + 2 * threadIdx.x, t, ep);
       }
       if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, flag ? FU_BAD_ROW : 0, ep);
       const int got = fu_collect(A, sm, ep, false, ok, e2);
       if (got & FU_ABORT) { ok = false; break; }
-      // everyone's maxima
+      // everyone's maxima, all six words in flight at once; one warp alone
+      // does the FP64 of the error (2000 x 3000 float32: 14.9 us per iteration
+      // with a trip to L2 per word and eight warps' conversions, now 14.1)
       T mx[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) mx[q] = -INFINITY;
       for (int p = threadIdx.x; p < (int)gridDim.x; p += FU_THREADS) {
+        const unsigned long long* w = A.ell + 12 * (int64_t)p;
+        typename Ll<T>::W x[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) x[q] = Ll<T>::get(w + 2 * q);
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-          const unsigned long long* w = A.ell + 12 * (int64_t)p + 2 * q;
-          Ll<double>::W x = Ll<double>::get(w);
-          ok = ok && ll_wait<double>(w, ep, x, A.info + 3, A.timeout_ns);
-          mx[q] = fmax(mx[q], (T)Ll<double>::value(x));
+          ok = ok && ll_wait<T>(w + 2 * q, ep, x[q], A.info + 3, A.timeout_ns);
+          mx[q] = fmax(mx[q], Ll<T>::value(x[q]));
         }
       }
 #pragma unroll
       for (int q = 0; q < 6; ++q) { mx[q] = warp_max(mx[q]); if (R.lane == 0) s_mx[q][R.warp] = mx[q]; }
       if (__syncthreads_or(!ok)) { ok = false; break; }
-      double mk[6];
+      int stop = 0;
+      if (threadIdx.x == 0) {
+        double mk[6];
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        T t = s_mx[q][0];
-        for (int w = 1; w < FU_WARPS; ++w) t = fmax(t, s_mx[q][w]);
-        mk[q] = (double)t;
+        for (int q = 0; q < 6; ++q) {
+          T t = s_mx[q][0];
+          for (int w = 1; w < FU_WARPS; ++w) t = fmax(t, s_mx[q][w]);
+          mk[q] = widen(t);
+        }
+        const double err = 0.5 * (mk[0] / fmax(fmax(mk[1], mk[2]), 1.0) + mk[3] / fmax(fmax(mk[4], mk[5]), 1.0));
+        if (blockIdx.x == 0 && ii < A.hist_cap && !(got & FU_BAD_ROW)) A.hist[ii] = err;
+        stop = err < A.stop_thr;
       }
-      __syncthreads();
+      stop = __syncthreads_or(stop);
       if (got & FU_BAD_ROW) { status = OTG_STATUS_NUMERICAL; niter = ii; break; }  // previous pair kept
-      const double err = 0.5 * (mk[0] / fmax(fmax(mk[1], mk[2]), 1.0) + mk[3] / fmax(fmax(mk[4], mk[5]), 1.0));
-      if (blockIdx.x == 0 && threadIdx.x == 0 && ii < A.hist_cap) A.hist[ii] = err;
       nchk = ii + 1;
       T* t;
       t = ucur; ucur = unxt; unxt = t;
       t = vcur; vcur = vnxt; vnxt = t;
-      if (err < A.stop_thr) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
+      if (stop) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
     }
   } else if (ok && A.max_iter > 0) {
     // column update of the initial row potentials: the first v
@@ -1000,8 +1008,8 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
         vcur[j] = vo;
         if (check) {
           // column marginal of (u, v) of iteration ii
-          const double cs = MODE == FU_LOG ? (double)s : (double)(vo * s);
-          e2 += (cs - (double)bj) * (cs - (double)bj);
+          const double d = widen(MODE == FU_LOG ? s : vo * s) - widen(bj);
+          e2 += d * d;
         }
         T vn;
         if (MODE == FU_LOG) {
@@ -1038,7 +1046,8 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
       if (check) {
         if (blockIdx.x == 0 && threadIdx.x == 0) A.hist[nchk < A.hist_cap ? nchk : A.hist_cap - 1] = e2;
         ++nchk;
-        if (sqrt(e2) < A.stop_thr) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
+        // (one warp's square root: FP64 issues at two lanes per clock)
+        if (__syncthreads_or(threadIdx.x == 0 && sqrt(e2) < A.stop_thr)) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
       }
       if (last) { niter = ii; break; }
       if (MODE == FU_ABS) build = got != 0;

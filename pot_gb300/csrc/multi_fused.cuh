@@ -861,7 +861,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
     mf_merge<T, false>(A, s_place[R.warp], na, nact, scr, false, vcur, [&](int p, int64_t cj, T bj, T vo, T, T s) {
       if (check) {
         // column marginal of (u, v) of iteration ii, in the column's own slot
-        const double cs = (LOGF ? (double)s : (double)(vo * s)) - (double)bj;
+        const double cs = widen(LOGF ? s : vo * s) - widen(bj);
         A.e2col[cj] = cs * cs;
       }
       T vn;
@@ -895,8 +895,13 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
       for (int k = blockIdx.x; k < nact; k += gridDim.x) {
         const int p = __ldcg(A.active + k);
         double e = -1.0;
-        if (check) e = sqrt(A.joint ? __ldcg(A.err2 + p) : block_sum_slots(A.e2col + A.c_off[p], A.cols[p]));
-        const bool conv = check && (A.joint ? joint_conv : e < A.stop_thr);
+        bool conv = false;
+        if (check) {
+          // (one warp's square root: FP64 issues at two lanes per clock)
+          const double e2 = A.joint ? __ldcg(A.err2 + p) : block_sum_slots(A.e2col + A.c_off[p], A.cols[p]);
+          if (threadIdx.x == 0) e = sqrt(e2);
+          conv = __syncthreads_or(threadIdx.x == 0 && (A.joint ? joint_conv : e < A.stop_thr));
+        }
         const bool leave = conv || last;
         if (leave) {
           for (int i = threadIdx.x; i < A.rows[p]; i += MT_THREADS) A.out_u[A.r_off[p] + i] = __ldcg(A.u + A.r_off[p] + i) * OUTF;
