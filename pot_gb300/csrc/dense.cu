@@ -630,9 +630,9 @@ __global__ void __launch_bounds__(256) dense_plan_kernel(const T* __restrict__ M
       if (LogDomain<METHOD>::value) p = ex2(fma(x, c, (ui + v[j]) * L2E));
       else p = ui * ex2(x * c) * v[j];
       if (P) P[i * ldp + j] = p;
-      racc = fma(x, p, racc);
+      if (loss) racc = fma(x, p, racc);
     }
-    if (loss) acc += (double)racc;
+    if (loss) acc += widen(racc);
   }
   if (loss) {
     acc = warp_sum(acc);
