@@ -67,16 +67,18 @@ __device__ __forceinline__ int mf_worker(int64_t total, int na, int64_t pos) {
   return w;
 }
 
-// Rows of slot k that start in [beg, end).
+// Rows of slot k in the share [beg, end): whole batches, those that start in
+// it (shares cut at any row had up to two partial batches more).
 template <typename T>
 __device__ __forceinline__ MfSpan mf_span(const MultiArgs<T>& A, int k, int64_t beg, int64_t end) {
   const int p = __ldcg(A.active + k);
   const int64_t base = __ldcg(A.urow_pre + k);
   const int wt = mf_weight(A, A.ldm[p]), n = A.rows[p];
+  const int64_t bw = (int64_t)wt * (16 / A.fNK);
   MfSpan s;
   s.k = k;
-  s.row = beg <= base ? 0 : (int)min((int64_t)n, (beg - base + wt - 1) / wt);
-  s.end = (int)max((int64_t)0, min((int64_t)n, (end - base + wt - 1) / wt));
+  s.row = beg <= base ? 0 : (int)min((int64_t)n, (beg - base + bw - 1) / bw * (16 / A.fNK));
+  s.end = end <= base ? 0 : (int)min((int64_t)n, (end - base + bw - 1) / bw * (16 / A.fNK));
   return s;
 }
 // First span of a share, and the one behind a span (k = nact: none).
@@ -472,7 +474,8 @@ __device__ __forceinline__ void mf_place(const MultiArgs<T>& A, MfPlace& P, int6
   P.co = A.c_off[P.p];
   const int64_t pos = __ldcg(A.urow_pre + P.k), total = __ldcg(A.urow_pre + nact);
   P.w0 = mf_worker(total, na, pos);
-  P.w1 = mf_worker(total, na, pos + (int64_t)(A.rows[P.p] - 1) * mf_weight(A, A.ldm[P.p]));
+  const int rb = 16 / A.fNK;  // the last batch's place
+  P.w1 = mf_worker(total, na, pos + (int64_t)((A.rows[P.p] - 1) / rb * rb) * mf_weight(A, A.ldm[P.p]));
   P.base = __ldcg(A.ucol_pre + P.k);
 }
 template <typename T>
@@ -757,10 +760,10 @@ __device__ __noinline__ void mf_rebuild(const MultiArgs<T>& A, int nact, const i
       // rows beyond the shared tile are streamed: up to twice the tile per CTA
       if (A.cols[p] > TL_MAXM || rcap > TL_MAXR || rcap * A.ldm[p] * (int64_t)sizeof(T) > 2 * A.tail_tile) tail = 0;
     }
-    // eight rows per worker at least, and a share never lighter than a row
-    // (each worker between a problem's first and last one then has a row of it)
+    // eight rows per worker at least, and a share never lighter than a batch
+    // (each worker between a problem's first and last one then has a batch of it)
     int64_t nw = s_run[3] / 8;
-    nw = min(nw, s_run[0] / mf_weight(A, A.fmm));
+    nw = min(nw, s_run[0] / ((int64_t)mf_weight(A, A.fmm) * (16 / A.fNK)));
     nw = max((int64_t)1, min(nw, (int64_t)nworkers));
     A.ctl[7] = (int)nw;
     A.ctl[2] = tail;
