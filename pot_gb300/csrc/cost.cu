@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
   const T* a = static_cast<const T*>(t.a) + t.r_off[p];
   const T* b = static_cast<const T*>(t.b) + t.c_off[p];
   T* P = t.P ? static_cast<T*>(t.P) + t.m_off[p] : nullptr;
+  const bool vec = ldm % W == 0 && ((uintptr_t)M | (uintptr_t)P) % 16 == 0;  // (the packed layout is)
   __shared__ T s_c;  // one warp's FP64 division
   if (threadIdx.x == 0) s_c = (T)(-OTG_LOG2E / t.reg[p]);
   __syncthreads();
@@ -311,7 +312,13 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
 #pragma unroll
       for (int q = 0; q < PL_ROWS; ++q) {
         const int i = min(ib + q * ry, i1 - 1);
-        unpack(ld_stream(reinterpret_cast<const V*>(M + (int64_t)i * ldm) + jv), x[q]);
+        const T* mp = M + (int64_t)i * ldm + j0;
+        if (vec) {
+          unpack(ld_stream(reinterpret_cast<const V*>(mp)), x[q]);
+        } else {
+#pragma unroll
+          for (int w = 0; w < W; ++w) x[q][w] = j0 + w < m ? __ldg(mp + w) : T(0);
+        }
         us[q] = u[i];
         as[q] = t.kl ? a[i] : T(1);
       }
@@ -347,7 +354,14 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
             T* op = reinterpret_cast<T*>(&o);
 #pragma unroll
             for (int w = 0; w < W; ++w) op[w] = pr[w];
-            reinterpret_cast<V*>(P + (int64_t)i * ldm)[jv] = o;
+            T* dst = P + (int64_t)i * ldm + j0;
+            if (vec) {
+              *reinterpret_cast<V*>(dst) = o;
+            } else {
+#pragma unroll
+              for (int w = 0; w < W; ++w)
+                if (j0 + w < m) dst[w] = pr[w];
+            }
           }
         }
       }
