@@ -28,9 +28,11 @@
 // already holds t_ij - s_i: the epilogue only exponentiates and sums (no
 // running max, no per-tile rescaling, no h slices in the stages).  A row
 // whose shifted sum leaves [2^-70, 2^100] writes nothing and its row block
-// is recomputed with the running max by the pass's fix-up launch (the first
-// pass of each side, which has no shift yet, and column-split passes keep
-// the running max throughout).
+// is recomputed with the running max by the pass's fix-up launch.  The first
+// pass of each side, which has no shift yet, keeps the running max
+// throughout.  The shifted-sum passes of one problem run in
+// online_stream_kernel (online_stream.cuh), those of pair batches in
+// online_batch_kernel; the pass kernel below runs the others.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <algorithm>
@@ -619,6 +621,8 @@ online_batch_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_consta
   constexpr bool FOLD = MODE == OL_FMAX || MODE == OL_FSUM;
   extern __shared__ unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_launch_next();
+  grid_wait_before();
   const int nunits = P.units_enc ? __ldcg(P.count) : __ldcg(P.count) * P.nrb;
   if ((int)blockIdx.x >= nunits) {  // the whole CTA, before any barrier or TMEM allocation
     if (P.fixup && threadIdx.x == 0) ol_fixup_done(P);
@@ -1146,6 +1150,25 @@ void ol_sum_window(float w, float& lo, float& hi) {
 size_t os_smem(bool narrow) { return (narrow ? OsGeo<true>::bytes : OsGeo<false>::bytes) + OS_SMEM_EXTRA; }
 static_assert(OsGeo<false>::bytes + OS_SMEM_EXTRA <= 232448, "shared memory of the shifted-sum pass");
 
+// A launch that may be set up while the kernel before it on the stream still
+// runs (the kernels wait for its end themselves, grid_wait_before): between a
+// pass and its fix-up, which is empty almost always, the set-up was most of
+// the fix-up's 3.6 us.
+template <typename... K, typename... A>
+void launch_next(void (*kernel)(K...), int ctas, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(OL_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);  // (errors: cudaGetLastError by the caller)
+}
+
 // Dynamic shared memory of every pass kernel instantiation (once).
 bool online_attr() {
   static std::once_flag once;
@@ -1285,15 +1308,13 @@ int otg_sinkhorn_online(const OtgOnlineProblem* p, cudaStream_t st) {
       // at least two tiles per range: a range that shares its rows pays about
       // 2 us for the slots, a tile takes 0.9 us
       W.clusters = (int)std::min<int64_t>((int64_t)W.row_pairs * std::max(1, W.tiles / 2), max_clusters);
-      if (P.narrow)
-        online_stream_kernel<true><<<2 * W.clusters, OL_THREADS, os_smem(true), st>>>(ah, al, bh, bl, rx, sx2, P, W);
-      else
-        online_stream_kernel<false><<<2 * W.clusters, OL_THREADS, os_smem(false), st>>>(ah, al, bh, bl, rx, sx2, P, W);
+      const int ctas = 2 * W.clusters;
+      if (P.narrow) launch_next(online_stream_kernel<true>, ctas, os_smem(true), st, ah, al, bh, bl, rx, sx2, P, W);
+      else launch_next(online_stream_kernel<false>, ctas, os_smem(false), st, ah, al, bh, bl, rx, sx2, P, W);
       OnlinePass Q = P;
       Q.fixup = 1; Q.units_enc = 1; Q.active = flist; Q.count = fcnt; Q.nrb = (int)(rows_pad / OL_M);
       Q.rows_per_pair = 0; Q.cols_per_pair = 0; Q.alpha_p = nullptr; Q.done_cnt = fdone;
-      online_batch_kernel<OL_FMAX><<<(unsigned)std::min<int64_t>(rows_pad / OL_M, sms), OL_THREADS, OL_SMEM, st>>>(
-          ah, al, bh, bl, rx, sx2, Q);
+      launch_next(online_batch_kernel<OL_FMAX>, (int)std::min<int64_t>(rows_pad / OL_M, sms), OL_SMEM, st, ah, al, bh, bl, rx, sx2, Q);
     }
     if (P.split > 1) online_finalize_kernel<<<(unsigned)((rows_pad + 255) / 256), 256, 0, st>>>(P);
     // the L1 error: the row slots summed in a fixed order (the same value in every run)
