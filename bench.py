@@ -77,10 +77,10 @@ sys.path.insert(0, HERE)
 
 METRIC = "Sinkhorn solves/s at marginal err 1e-6, warm vs plain, 1 GB300; % roofline"
 WS_N, WS_D, WS_REG, WS_TOL = 2048, 16, 0.02, 1e-6
-# DRAM traffic / algorithmic bytes of multi_sinkhorn_kernel, from one ncu capture of the
-# same workload on 128 pairs (profiles/multi_sinkhorn_warmstart_gmm2048.md); the launch's
-# traffic scales with the problem-iterations it processes
-MULTI_TRAFFIC_RATIO = 132.02 / 133.61  # ncu dram bytes / algorithmic bytes, one plain-arm launch on 128 pairs
+# DRAM traffic / algorithmic bytes of multi_fused_kernel, from one ncu capture on 64 blocks of
+# the same size (profiles/one_read_kernels.md); the launch's traffic scales with the
+# problem-iterations it processes
+MULTI_TRAFFIC_RATIO = 12.01 / 11.81
 EVAL_SEED = 10_000_000
 
 
@@ -215,7 +215,7 @@ def run_warmstart(args, pk):
             stt = out[2].cpu().numpy()
             err = out[4].cpu().numpy()
             L = ps.layout
-            passes = (nit + 2) + (nit + 1)  # column passes incl. the final check pass, row passes
+            passes = nit + 2  # the first column pass, one read per iteration
             alg = float((passes * L.rows_np * L.ldm_np * 4).sum())
             res[arm] = {"ms": ms, "kernel_ms": kms, "alg_bytes": alg, "niter_mean": float(nit.mean()),
                         "niter_max": int(nit.max()), "converged": int((stt == 0).sum()),
@@ -271,8 +271,8 @@ def run_warmstart(args, pk):
                    "held_out_seeds": [EVAL_SEED, EVAL_SEED + B - 1]},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / pk["hbm_gbs"], "traffic": p["alg_bytes"] * MULTI_TRAFFIC_RATIO,
-                     "traffic_src": "ncu capture on 128 pairs, scaled by problem-iterations",
-                     "kernel": "multi_sinkhorn_kernel (plain arm)",
+                     "traffic_src": "ncu capture on 64 blocks, scaled by problem-iterations",
+                     "kernel": "multi_fused_kernel (plain arm)",
                      "alg_bytes_per_launch": p["alg_bytes"], "launch_ms": p["kernel_ms"],
                      "peak_src": pk["src"] + " (of measured)" if pk["src"] == "measured" else pk["src"]},
         "e2e": {"value": W * B / e2e_s, "unit": "solves/s", "h2d_bytes_per_step": int(Xh.nbytes + Yh.nbytes),
@@ -345,7 +345,7 @@ def run_online(args, pk):
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                          "frac": achieved / pk["bf16_tflops"], "issued_multiplier": 3,
                          "issued_frac": 3 * achieved / pk["bf16_tflops"], "traffic": None,
-                         "kernel": "online_pass_kernel", "alg_flop_per_iteration": flop}}
+                         "kernel": "online_stream_kernel", "alg_flop_per_iteration": flop}}
 
 
 def aux_online(pk, n=65536, iters=20):
@@ -371,7 +371,7 @@ def aux_online(pk, n=65536, iters=20):
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                          "frac": achieved / pk["bf16_tflops"], "issued_multiplier": 3,
                          "issued_frac": 3 * achieved / pk["bf16_tflops"], "traffic": None,
-                         "kernel": "online_pass_kernel (+ online_finalize_kernel)",
+                         "kernel": "online_stream_kernel",
                          "alg_flop_per_iteration": flop}}
 
 
@@ -483,7 +483,7 @@ def run_ragged(args, pk):
     trials = next(iter(tune.tuner().trials.values()), [])
     nit = res.niter.cpu().numpy().astype(np.int64)
     L = res.layout
-    alg = float((((nit + 2) + (nit + 1)) * L.rows_np * L.ldm_np * 4).sum())
+    alg = float(((nit + 2) * L.rows_np * L.ldm_np * 4).sum())  # the first column pass, one read per iteration
     return {"metric": "batched Sinkhorn solves/s", "value": B / (ms * 1e-3), "unit": "solves/s", "ms_per_step": ms,
             "dtype": "f32", "config": {"workload": "%d uneven problems n,m~U[32,1024], d in {3,16}, reg=10^U[-3,-1] x "
                                                    "max cost, stopThr=1e-6" % B,
@@ -496,7 +496,7 @@ def run_ragged(args, pk):
                                                             for c, f, t in trials]},
             "roofline": {"bound": "hbm", "achieved": alg / (ms * 1e-3) / 1e9, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": alg / (ms * 1e-3) / 1e9 / pk["hbm_gbs"], "traffic": None,
-                         "kernel": "multi_sinkhorn_kernel (+ cost build)", "alg_bytes": alg}}
+                         "kernel": "multi_fused_kernel (+ cost build)", "alg_bytes": alg}}
 
 
 def run_dense(args, pk):
@@ -522,13 +522,16 @@ def run_dense(args, pk):
         kms.append(ms)
     bregman.read_result(r)
     ms = statistics.median(kms)
-    alg = ((r.niter + 2) + (r.niter + 1)) * n * n * 4.0
+    # the first column pass and one read per iteration; rows wider than 16384 floats: two passes per iteration
+    reads = r.niter + 2 if n <= 16384 else 2 * r.niter + 3
+    alg = reads * n * n * 4.0
     return {"metric": "dense Sinkhorn solves/s", "value": 1000.0 / ms, "unit": "solves/s", "ms_per_step": ms,
             "dtype": "f32", "config": {"workload": "dense log-Sinkhorn n=m=%d, reg=0.05, stopThr=1e-6" % n,
                                        "iterations": r.niter + 1, "l2": "M = %.2f GiB" % (n * n * 4 / 2**30)},
             "roofline": {"bound": "hbm", "achieved": alg / (ms * 1e-3) / 1e9, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": alg / (ms * 1e-3) / 1e9 / pk["hbm_gbs"], "traffic": None,
-                         "kernel": "dense_sinkhorn_kernel", "alg_bytes_per_launch": alg}}
+                         "kernel": "fused_sinkhorn_kernel" if n <= 16384 else "dense_sinkhorn_kernel",
+                         "alg_bytes_per_launch": alg}}
 
 
 def run_small(args, pk):
@@ -577,7 +580,7 @@ def run_small(args, pk):
     nit = np.array([i for i, _ in out["graph"]["niter"]])
     assert [i for i, _ in out["direct"]["niter"]] == list(nit)
     ms = out["graph"]["s"] * 1e3
-    alg = float(((nit + 1) * 2 * n * n * 8).mean())
+    alg = 2.0 * n * n * 8  # the cost in, the plan out; K stays in shared memory
     return {"metric": "dense Sinkhorn solves/s (n=m=1024, float64)", "value": 1.0 / out["graph"]["s"],
             "unit": "solves/s", "ms_per_step": ms, "dtype": "f64",
             "direct": {"value": 1.0 / out["direct"]["s"], "ms_per_solve": out["direct"]["s"] * 1e3},
@@ -587,7 +590,7 @@ def run_small(args, pk):
                        "niter_mean": float(nit.mean()), "l2": "cost 8 MiB, L2-resident (latency-bound)"},
             "roofline": {"bound": "hbm", "achieved": alg / (ms * 1e-3) / 1e9, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": alg / (ms * 1e-3) / 1e9 / pk["hbm_gbs"], "traffic": None,
-                         "kernel": "dense_sinkhorn_kernel (graph replay, host wall time)",
+                         "kernel": "fused_sinkhorn_kernel (graph replay, host wall time)",
                          "alg_bytes_per_launch": alg}}
 
 
@@ -812,17 +815,17 @@ def run_batch(args, pk):
         kms.append(ms)
     ms = statistics.median(kms)
     nit = res[4].cpu().numpy().astype(np.int64)
-    # algorithmic passes over each cost block: u and v per iteration plus the
-    # final check pass, and the plan (read the cost, write the plan); the
+    # algorithmic passes over each cost block: the first column pass, one read
+    # per iteration, and the plan (read the cost, write the plan); the
     # transpose the batch order costs here is not counted
-    alg = float((((2 * nit + 3) + 2) * n * n * 4.0).sum())
+    alg = float((((nit + 2) + 2) * n * n * 4.0).sum())
     return {"metric": "batched Sinkhorn solves/s (ot.batch.solve_batch)", "value": B / (ms * 1e-3),
             "unit": "solves/s", "ms_per_step": ms, "dtype": "f32",
             "config": {"workload": "%d problems %dx%d (GMM clouds d=16, cost / max), reg=0.05, tol=1e-6, "
                                    "log_sinkhorn" % (B, n, n), "niter_mean": float(nit.mean())},
             "roofline": {"bound": "hbm", "achieved": alg / (ms * 1e-3) / 1e9, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": alg / (ms * 1e-3) / 1e9 / pk["hbm_gbs"], "traffic": None,
-                         "kernel": "multi_sinkhorn_kernel on the transposed blocks (+ transpose, plan)",
+                         "kernel": "multi_fused_kernel on the transposed blocks (+ transpose, plan)",
                          "alg_bytes": alg}}
 
 

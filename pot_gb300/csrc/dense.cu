@@ -1,6 +1,12 @@
 // Dense-cost Sinkhorn (scaling and log-domain forms) as ONE persistent
 // cooperative kernel per solve, plus the plan / loss kernel.
 //
+// The entry points are here; most solves go on to the kernel that reads the
+// cost once per iteration (fused_impl.cuh).  The two-pass kernel below runs
+// the stabilised form, rows wider than 16384 floats or 8192 doubles,
+// whole-vector rows at odd addresses or strides, and calls whose scratch has
+// no room for the one-read kernel's words.
+//
 // Reference behaviour restated here: PythonOT/POT ot/bregman/_sinkhorn.py
 //   sinkhorn_knopp  :487-687  (v = b / K^T u ; u = 1 / (diag(1/a) K v), NaN/zero
 //                              revert :633-645, L2 column-marginal check every

@@ -2,6 +2,11 @@
 // problem in every half-step, so the time follows the batch's total work and
 // a slow problem is spread over the whole GPU instead of one CTA.
 //
+// Batches whose widest row the one-read kernel holds (multi_fused.cuh) go
+// there; the two-pass kernel below takes the others, and calls whose partials
+// have no room for that kernel's slots.  The tail kernel takes the last
+// problems of either.
+//
 // Reference behaviour (PythonOT/POT): per problem, the order and stopping test
 // of ot/bregman/_sinkhorn.py:880-899 (sinkhorn_log: v first, then u; L2
 // column-marginal error every 10th iteration); problems stop individually.

@@ -1,5 +1,7 @@
-"""Autotuner for the schedule of the work-balanced batch solver
-(``csrc/multi.cu``, ``otg_sinkhorn_multi``).
+"""Autotuner for the schedule of the work-balanced batch solver's two-pass
+kernel (``csrc/multi.cu``, ``otg_sinkhorn_multi``).  The one-read kernel, which
+takes most batches, cuts its own shares and uses only a grid smaller than one
+CTA per SM from it.
 
 The schedule divides the work of one launch and leaves each problem's
 iteration unchanged (results agree to rounding of the merge order):
