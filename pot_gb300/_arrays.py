@@ -16,6 +16,7 @@ def upload(device, arrays):
     for the stream each time: 30 of them were 2 ms of a 256-problem ragged
     call).  A capturing stream refuses it, as it does the pageable copy: a
     replay would read the host buffer after it went back to its pool."""
+    device = torch.device(device)
     if device.type != "cuda" or torch.cuda.is_current_stream_capturing():
         return [torch.from_numpy(np.ascontiguousarray(x)).to(device) for x in arrays]
     offs, total = [], 0
@@ -27,11 +28,10 @@ def upload(device, arrays):
     for x, o in zip(arrays, offs):
         view[o:o + x.nbytes] = np.ascontiguousarray(x).view(np.uint8).reshape(-1)
     dev = host.to(device, non_blocking=True)
-    return [dev[o:o + x.nbytes].view(_TORCH[x.dtype.char]) for x, o in zip(arrays, offs)]
+    return [dev[o:o + x.nbytes].view(_TORCH[x.dtype.kind, x.dtype.itemsize]) for x, o in zip(arrays, offs)]
 
 
-_TORCH = {np.dtype(k).char: v for k, v in (("int32", torch.int32), ("int64", torch.int64), ("float32", torch.float32),
-                                           ("float64", torch.float64))}
+_TORCH = {("i", 4): torch.int32, ("i", 8): torch.int64, ("f", 4): torch.float32, ("f", 8): torch.float64}
 
 
 class Boundary:

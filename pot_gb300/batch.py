@@ -482,7 +482,7 @@ def solve_sample_ragged(Xs, Ys, reg, as_=None, bs=None, reg_relative=False, max_
         return np.concatenate([np.asarray(x).reshape(-1) for x in arrays]).astype(ndt, copy=False)
 
     def weights(ws, sizes):
-        return packed(ws) if ws is not None else np.repeat((1.0 / np.asarray(sizes, dtype=np.float64)).astype(ndt), sizes)
+        return packed(ws) if ws is not None else np.repeat(np.array([1.0 / k for k in sizes]).astype(ndt), sizes)
 
     X, Y, ap, bp = upload(torch.device(device), [packed(Xs), packed(Ys), weights(as_, rows), weights(bs, cols)])
     x_off = np.concatenate([[0], np.cumsum([r * d for r, d in zip(rows, dims)])[:-1]])
