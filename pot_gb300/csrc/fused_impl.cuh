@@ -275,10 +275,10 @@ __device__ __forceinline__ void fu_rows(const FusedArgs<T>& A, const FuRow& R, T
       r = un = p1 == T(0) ? T(1) : p1 / t;
       if (myrow < nr && !fu_tame(un)) flag = FU_BAD_ROW;
     } else {
-      un = pow(p1 / (p2 * t), A.fi1);
+      un = pow_unit(p1 / (p2 * t), A.fi1);
       if (myrow < nr) {
         if (!isfinite(un)) flag = FU_BAD_ROW;
-        tr.d0 = fmax(tr.d0, fabs(un - p0)); tr.d1 = fmax(tr.d1, fabs(un)); tr.d2 = fmax(tr.d2, fabs(p0));
+        tr.d0 = pos_max(tr.d0, fabs(un - p0)); tr.d1 = pos_max(tr.d1, fabs(un)); tr.d2 = pos_max(tr.d2, fabs(p0));
       }
       r = p2 * un;
     }
@@ -891,24 +891,24 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
       int flag = fu_pass<T, MODE, NK, RES>(A, R, sm, red, rr, ring, ucur, unxt, H, held, ut, ep);
       ok = fu_merge<T, false>(A, R, s_s, s_m, ep, [&](int j, T, T s) {
         const T be = A.bew ? A.bew[j] : T(1);
-        const T vn = pow(A.b[j] / (be * s), A.fi2);
+        const T vn = pow_unit(A.b[j] / (be * s), A.fi2);
         if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
         const T vo = __ldcg(vcur + j);
         vnxt[j] = vn;
         Ll<T>::put(A.vll + j * Ll<T>::N, be * vn, ep);
-        vt.d0 = fmax(vt.d0, fabs(vn - vo));
-        vt.d1 = fmax(vt.d1, fabs(vn));
-        vt.d2 = fmax(vt.d2, fabs(vo));
+        vt.d0 = pos_max(vt.d0, fabs(vn - vo));
+        vt.d1 = pos_max(vt.d1, fabs(vn));
+        vt.d2 = pos_max(vt.d2, fabs(vo));
       });
       // this CTA's maxima and flags
       T mine[6] = {ut.d0, ut.d1, ut.d2, vt.d0, vt.d1, vt.d2};
 #pragma unroll
-      for (int q = 0; q < 6; ++q) { mine[q] = warp_max(mine[q]); if (R.lane == 0) s_mx[q][R.warp] = mine[q]; }
+      for (int q = 0; q < 6; ++q) { mine[q] = warp_pos_max(mine[q]); if (R.lane == 0) s_mx[q][R.warp] = mine[q]; }
       if (flag & FU_ABORT) ok = false;
       flag = __syncthreads_or(flag);  // either flag ends the solve with the previous pair
       if (threadIdx.x < 6) {
         T t = s_mx[threadIdx.x][0];
-        for (int w = 1; w < FU_WARPS; ++w) t = fmax(t, s_mx[threadIdx.x][w]);
+        for (int w = 1; w < FU_WARPS; ++w) t = pos_max(t, s_mx[threadIdx.x][w]);
         Ll<T>::put(A.ell + 12 * (int64_t)blockIdx.x + 2 * threadIdx.x, t, ep);
       }
       if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, flag ? FU_BAD_ROW : 0, ep);
@@ -928,11 +928,11 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
           ok = ok && ll_wait<T>(w + 2 * q, ep, x[q], A.info + 3, A.timeout_ns);
-          mx[q] = fmax(mx[q], Ll<T>::value(x[q]));
+          mx[q] = pos_max(mx[q], Ll<T>::value(x[q]));
         }
       }
 #pragma unroll
-      for (int q = 0; q < 6; ++q) { mx[q] = warp_max(mx[q]); if (R.lane == 0) s_mx[q][R.warp] = mx[q]; }
+      for (int q = 0; q < 6; ++q) { mx[q] = warp_pos_max(mx[q]); if (R.lane == 0) s_mx[q][R.warp] = mx[q]; }
       if (__syncthreads_or(!ok)) { ok = false; break; }
       int stop = 0;
       if (threadIdx.x == 0) {
@@ -940,7 +940,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
           T t = s_mx[q][0];
-          for (int w = 1; w < FU_WARPS; ++w) t = fmax(t, s_mx[q][w]);
+          for (int w = 1; w < FU_WARPS; ++w) t = pos_max(t, s_mx[q][w]);
           mk[q] = widen(t);
         }
         const double err = 0.5 * (mk[0] / fmax(fmax(mk[1], mk[2]), 1.0) + mk[3] / fmax(fmax(mk[4], mk[5]), 1.0));
