@@ -278,7 +278,12 @@ def _uniform_batch(M):
     if layout.ldm_np[0] == M.shape[2] and M.is_contiguous() and M.data_ptr() % 16 == 0:
         Mp = M.reshape(-1)
     else:
-        Mp = pack_dense(layout, M)
+        # every block at once: two launches (two per problem were 14 ms for 512 blocks of 37 x 63)
+        (B, n, m), ld = M.shape, int(layout.ldm_np[0])
+        buf = torch.empty(B, n, ld, dtype=M.dtype, device=M.device)
+        buf[:, :, :m].copy_(M)
+        buf[:, :, m:] = float("inf")
+        Mp = buf.view(-1)
     return layout, Mp
 
 
