@@ -50,11 +50,16 @@
 //
 // float64 log form, cost resident: this GPU issues FP64 at about two lanes
 // per clock and SM, and an exponential costs some twenty such operations.
-// The solver stores the plan of the current potentials,
-// K_ij = exp(x_ij + f_i + g_j) (row-normalised), and iterates scalings u, v
-// over it, f + log u and g + log v being the potentials: two FMAs per entry.
-// When a scaling leaves [2^-300, 2^300] the potentials absorb it and K is
-// rebuilt with running maxima.
+// The solver stores the plan of the current potentials with its rows
+// normalised to one, K_ij = exp(x_ij + f_i - log a_i + g_j), and iterates
+// scalings u, v over it, f + log u and g + log v being the potentials: two
+// FMAs per entry.  When a scaling leaves [2^-300, 2^300] the potentials absorb
+// it and K is rebuilt with running maxima.  A column of K may have underflowed
+// in part or altogether (g set by rows that are empty, or next to nothing in
+// b_j): an entry is off by at most 2^-1075, a column sum by 2^-1075 sum_i a_i
+// u_i.  A column sum that is not 2^53 times that is not used: the whole column
+// update is then taken with running maxima over the current row potentials,
+// and K is rebuilt from its result.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -67,8 +72,10 @@ namespace otg {
 
 constexpr int FU_RING = 9;  // most chunks in flight per group
 enum { FU_LOG = 0, FU_SCAL = 1, FU_UNB = 2, FU_ABS = 3 };
-// flags that a CTA publishes with its merge
-enum { FU_BAD_ROW = 1, FU_BAD_COL = 2, FU_ABORT = 4 };
+// Flags that a CTA publishes with its merge.  FU_ABS: FU_BAD_ROW a scaling to
+// absorb, FU_BAD_COL a column sum that cannot be used, FU_LOW_COL one that
+// cannot if there is a row scaling above 2^30 (FU_LOOSE).
+enum { FU_BAD_ROW = 1, FU_BAD_COL = 2, FU_ABORT = 4, FU_LOOSE = 8, FU_LOW_COL = 16 };
 
 template <typename T>
 struct FusedArgs {
@@ -80,6 +87,7 @@ struct FusedArgs {
   unsigned long long *part, *vll, *stll, *ell;   // published words, see Ll
   T* pairs;                  // [grid][m] (maximum, sum) pairs: first and fallback column pass
   T* vfix;                   // [m] v of the fallback column pass
+  double* mass;              // [grid] sum of a over the CTA's rows (FU_ABS)
   T *out_u, *out_v;
   double* hist; int hist_cap;
   int* info;                 // status, niter, nchecks, abort
@@ -174,8 +182,15 @@ __device__ __forceinline__ void fu_get_global(const FusedArgs<T>& A, int row, in
   }
 }
 
+// x >= lim > 0; false for a NaN.  (Doubles by integers: an FP64 comparison
+// issues at two lanes per clock.)
+__device__ __forceinline__ bool fu_at_least(float x, float lim) { return x >= lim; }
+__device__ __forceinline__ bool fu_at_least(double x, double lim) {
+  const long long b = __double_as_longlong(x);
+  return b >= __double_as_longlong(lim) && b <= 0x7ff0000000000000ll;
+}
 // A scaling of FU_ABS that needs no absorption: within [2^-300, 2^300].
-__device__ __forceinline__ bool fu_tame(double x) { return x > 4.9e-91 && x < 2.0e90; }
+__device__ __forceinline__ bool fu_tame(double x) { return fu_at_least(x, 0x1p-300) && !fu_at_least(x, 0x1p300); }
 
 // ---------------------------------------------------------------------------
 // Ring of the streamed form.  Chunk j of a group's pass is half (j & 1) of
@@ -272,8 +287,12 @@ __device__ __forceinline__ void fu_rows(const FusedArgs<T>& A, const FuRow& R, T
       r = un = T(1) / (p1 * t);
       if (myrow < nr && !isfinite(un)) flag = FU_BAD_ROW;
     } else if (MODE == FU_ABS) {
-      r = un = p1 == T(0) ? T(1) : p1 / t;
-      if (myrow < nr && !fu_tame(un)) flag = FU_BAD_ROW;
+      un = t;  // (the row's scaling is 1 / t)
+      r = p1 / t;
+      if (myrow < nr) {
+        if (!fu_tame(t)) flag |= FU_BAD_ROW;
+        else if (!fu_at_least(t, T(0x1p-30))) flag |= FU_LOOSE;
+      }
     } else {
       un = pow_unit(p1 / (p2 * t), A.fi1);
       if (myrow < nr) {
@@ -469,9 +488,8 @@ __device__ __forceinline__ int fu_pass(const FusedArgs<T>& A, const FuRow& R_, c
   return flag;
 }
 
-// Absorbing pass of FU_ABS: rows of K = exp(x + f + g) with f the exact row
-// update of g = sm.gs (running maximum), f into fref, scalings one; K into
-// the resident rows.
+// Absorbing pass of FU_ABS: rows of K with f the exact row update of g = sm.gs
+// (running maximum), f into fref, scalings one; K into the resident rows.
 template <typename T, int NK>
 __device__ __noinline__ void fu_build(const FusedArgs<T>& A, const FuRow& R, const FuSmem<T>& sm, T (*red)[FU_WARPS][fu_rb(NK)],
                                       T* unxt, unsigned ep) {
@@ -507,14 +525,15 @@ __device__ __noinline__ void fu_build(const FusedArgs<T>& A, const FuRow& R, con
       }
     }
     const T s = fu_group<T, 1, false>(one, R, A.G, red, par);
-    const T r = A.a[row] / s;
+    const T r = T(1) / s;
+    const typename FuV<T>::S ai = FuV<T>::all(A.a[row]);
     T* ks = sm.data + (row - R.r0) * A.mp;
 #pragma unroll
     for (int k = 0; k < NK; ++k) {
       if (k < A.kv) {
 #pragma unroll
         for (int w = 0; w < W; ++w) e[k][w] *= r;
-        acc[k].add_v(FuV<T>::of(e[k]));
+        acc[k].fma_s(FuV<T>::of(e[k]), ai);
         fu_put(ks + (k * R.gt + R.tg) * W, e[k]);
       }
     }
@@ -731,6 +750,15 @@ __device__ __forceinline__ bool fu_merge(const FusedArgs<T>& A, const FuRow& R, 
   return ok;
 }
 
+// The flags that any thread of the CTA has.
+__device__ __forceinline__ int fu_any(int bits) {
+  int all = 0;
+  if (__syncthreads_or(bits))
+    for (int f = 1; f <= FU_LOW_COL; f <<= 1)
+      if (__syncthreads_or(bits & f)) all |= f;
+  return all;
+}
+
 // The whole v of epoch `ep` into sm.vs (poll), the flags that the CTAs
 // published with it, and with `check` their error shares added in CTA order.
 // Every thread gets the same flags and error.
@@ -762,12 +790,7 @@ __device__ __forceinline__ int fu_collect(const FusedArgs<T>& A, const FuSmem<T>
       share += Ll<double>::value(w);
     }
   }
-  int all = 0;
-  if (__syncthreads_or(bits)) {
-    if (__syncthreads_or(bits & FU_BAD_ROW)) all |= FU_BAD_ROW;
-    if (__syncthreads_or(bits & FU_BAD_COL)) all |= FU_BAD_COL;
-    if (__syncthreads_or(bits & FU_ABORT)) all |= FU_ABORT;
-  }
+  const int all = fu_any(bits);
   if (check) e2 = block_sum_fixed(share);
   return all;
 }
@@ -827,6 +850,12 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
     for (int w = 0; w < Ll<T>::N; ++w) A.vll[j * Ll<T>::N + w] = 0ull;
   }
   for (int j = threadIdx.x; j < A.m * Ll<T>::N; j += FU_THREADS) A.part[(int64_t)blockIdx.x * A.m * Ll<T>::N + j] = 0ull;
+  if (MODE == FU_ABS) {
+    double w = 0.0;
+    for (int i = R.r0 + threadIdx.x; i < R.r1; i += FU_THREADS) w += widen(A.a[i]);
+    w = block_sum_fixed(w);
+    if (threadIdx.x == 0) A.mass[blockIdx.x] = w;
+  }
   if (threadIdx.x < 12) A.ell[(int64_t)12 * blockIdx.x + threadIdx.x] = 0ull;
   if (threadIdx.x == 0) A.stll[blockIdx.x] = 0ull;
   // beyond the row: v that adds nothing
@@ -956,28 +985,42 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
       if (stop) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
     }
   } else if (ok && A.max_iter > 0) {
-    // column update of the initial row potentials: the first v
-    int flag = 0;
-    if (LOGF) {
-      fu_collse<T, RES && MODE != FU_ABS>(A, R, sm, MODE == FU_ABS ? A.fref : ucur);
-      ok = fu_barrier(A.bar, gen, abort_flag, A.timeout_ns);
-      if (ok)
-        fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) {
-          Ll<T>::put(A.vll + j * Ll<T>::N, lg2(A.b[j]) - lse_value(mx, s), 1u);
+    // column update of the initial row potentials: the first v (FU_ABS takes
+    // it when it builds K)
+    int flag = 0, got = 0;
+    if (MODE != FU_ABS) {
+      if (LOGF) {
+        fu_collse<T, RES>(A, R, sm, ucur);
+        ok = fu_barrier(A.bar, gen, abort_flag, A.timeout_ns);
+        if (ok)
+          fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) {
+            Ll<T>::put(A.vll + j * Ll<T>::N, lg2(A.b[j]) - lse_value(mx, s), 1u);
+          });
+      } else {
+        fu_colsum<T, NK, RES>(A, R, sm, ucur, 1u);
+        ok = fu_merge<T, false>(A, R, s_s, s_m, 1u, [&](int j, T, T s) {
+          const T vn = A.b[j] / s;
+          if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
+          Ll<T>::put(A.vll + j * Ll<T>::N, vn, 1u);
         });
-    } else {
-      fu_colsum<T, NK, RES>(A, R, sm, ucur, 1u);
-      ok = fu_merge<T, false>(A, R, s_s, s_m, 1u, [&](int j, T, T s) {
-        const T vn = A.b[j] / s;
-        if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
-        Ll<T>::put(A.vll + j * Ll<T>::N, vn, 1u);
-      });
+      }
+      flag = __syncthreads_or(flag) ? FU_BAD_COL : 0;
+      if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, flag, 1u);
+      got = fu_collect(A, sm, 1u, false, ok, e2);
+      if (got & FU_ABORT) ok = false;
     }
-    flag = __syncthreads_or(flag) ? FU_BAD_COL : 0;
-    if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, flag, 1u);
-    int got = fu_collect(A, sm, 1u, false, ok, e2);
-    if (got & FU_ABORT) ok = false;
-    bool build = MODE == FU_ABS, again = false;
+    // FU_ABS: K is to be built, from a column update of its own (else the
+    // scalings are absorbed)
+    bool build = MODE == FU_ABS, absolute = true;
+    // Column sums below these may have lost bits to underflow (an entry's
+    // 2^-1075 with row scalings up to 2^30, 2^300; the sum's own roundings).
+    __shared__ T s_lim[2];  // (registers are what the passes have least of)
+    if (MODE == FU_ABS) {
+      double w = 0.0;
+      for (int p = threadIdx.x; p < (int)gridDim.x; p += FU_THREADS) w += __ldcg(A.mass + p);
+      w = block_sum_fixed(w);
+      if (threadIdx.x == 0) { s_lim[0] = (T)fmax(w * 0x1p-992, 0x1p-1000); s_lim[1] = (T)fmax(w * 0x1p-722, 0x1p-1000); }
+    }
     for (int ii = 0; ok; ++ii) {
       // sm.vs holds v of iteration ii, ucur u of iteration ii - 1
       if (MODE == FU_SCAL && (got & FU_BAD_COL)) {
@@ -988,11 +1031,21 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
       FuTrack<T> tr{T(0), T(0), T(0)};
       flag = 0;
       if (MODE == FU_ABS && build) {
-        for (int j = threadIdx.x; j < A.m; j += FU_THREADS) {
-          sm.gs[j] = ii == 0 ? sm.vs[j] : sm.gs[j] + lg2(sm.vs[j]);
-          sm.vs[j] = T(1);
+        if (absolute) {
+          // the first column update, or a column sum that cannot be used:
+          // the update of the current row potentials, with running maxima
+          for (int i = R.r0 + threadIdx.x; i < R.r1; i += FU_THREADS) A.fref[i] = __ldcg(A.fref + i) - lg2(__ldcg(ucur + i));
+          __syncthreads();
+          fu_collse<T, false>(A, R, sm, A.fref);
+          if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
+          fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) { A.vfix[j] = lg2(A.b[j]) - lse_value(mx, s); });
+          if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
         }
-        if (ii == 0) for (int j = A.m + threadIdx.x; j < A.mp; j += FU_THREADS) sm.vs[j] = T(0);
+        for (int j = threadIdx.x; j < A.mp; j += FU_THREADS) {
+          if (j < A.m) sm.gs[j] = absolute ? __ldcg(A.vfix + j) : sm.gs[j] + lg2(sm.vs[j]);
+          sm.vs[j] = j < A.m ? T(1) : T(0);
+        }
+        absolute = false;
         __syncthreads();
         fu_build<T, NK>(A, R, sm, red, unxt, ep);
       } else {
@@ -1017,7 +1070,10 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
           if (bj != T(0) && !(s >= T(8.470329472543003e-22))) flag |= FU_BAD_COL;  // 2^-70
         } else if (MODE == FU_ABS) {
           vn = bj == T(0) ? T(1) : bj / s;
-          if (!fu_tame(vn)) flag |= FU_BAD_COL;
+          if (bj != T(0)) {
+            if (!fu_at_least(s, s_lim[1])) flag |= fu_at_least(s, s_lim[0]) ? FU_LOW_COL : FU_BAD_COL;
+            if (!fu_tame(vn)) flag |= fu_at_least(vn, T(0x1p-900)) ? FU_BAD_ROW : FU_BAD_COL;  // (a denormal quotient)
+          }
         } else {
           vn = bj / s;
           if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
@@ -1029,11 +1085,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
         if (threadIdx.x == 0) Ll<double>::put(A.ell + 2 * blockIdx.x, e2, ep);
       }
       if (flag & FU_ABORT) ok = false;
-      int mine = 0;
-      if (__syncthreads_or(flag)) {
-        mine = __syncthreads_or(flag & FU_BAD_ROW) ? FU_BAD_ROW : 0;
-        if (__syncthreads_or(flag & FU_BAD_COL)) mine |= FU_BAD_COL;
-      }
+      const int mine = fu_any(flag & ~FU_ABORT);
       if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, mine, ep);
       got = fu_collect(A, sm, ep, check, ok, e2);
       if (got & FU_ABORT) { ok = false; break; }
@@ -1050,18 +1102,18 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
         if (__syncthreads_or(threadIdx.x == 0 && sqrt(e2) < A.stop_thr)) { status = OTG_STATUS_CONVERGED; niter = ii; break; }
       }
       if (last) { niter = ii; break; }
-      if (MODE == FU_ABS) build = got != 0;
-      if (MODE == FU_LOG) {
-        again = (got & FU_BAD_COL) != 0;
-        if (again) {
-          // a column sum too small to trust: the column update with running maxima
-          fu_collse<T, RES>(A, R, sm, ucur);
-          if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
-          fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) { A.vfix[j] = lg2(A.b[j]) - lse_value(mx, s); });
-          if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
-          for (int j = threadIdx.x; j < A.mp; j += FU_THREADS) sm.vs[j] = j < A.m ? __ldcg(A.vfix + j) : vpad;
-          __syncthreads();
-        }
+      if (MODE == FU_ABS) {
+        absolute = (got & FU_BAD_COL) || ((got & FU_LOW_COL) && (got & FU_LOOSE));
+        build = absolute || (got & FU_BAD_ROW);
+      }
+      if (MODE == FU_LOG && (got & FU_BAD_COL)) {
+        // a column sum too small to trust: the column update with running maxima
+        fu_collse<T, RES>(A, R, sm, ucur);
+        if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
+        fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) { A.vfix[j] = lg2(A.b[j]) - lse_value(mx, s); });
+        if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
+        for (int j = threadIdx.x; j < A.mp; j += FU_THREADS) sm.vs[j] = j < A.m ? __ldcg(A.vfix + j) : vpad;
+        __syncthreads();
       }
     }
   }
@@ -1080,7 +1132,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
   // Final state in natural units: this CTA's rows and its share of the columns.
   for (int i = R.r0 + threadIdx.x; i < R.r1; i += FU_THREADS) {
     const T u = __ldcg(ucur + i);
-    A.out_u[i] = MODE == FU_LOG ? u * LN2 : MODE == FU_ABS ? (__ldcg(A.fref + i) + lg2(u)) * LN2 : u;
+    A.out_u[i] = MODE == FU_LOG ? u * LN2 : MODE == FU_ABS ? (__ldcg(A.fref + i) - lg2(u)) * LN2 : u;
   }
   for (int j = cb + threadIdx.x; j < ce; j += FU_THREADS) {
     const T v = __ldcg(vcur + j);
@@ -1198,7 +1250,7 @@ bool fu_plan(int64_t n, int64_t m, bool abs, int grid, const FuDevice& d, FuPlan
 constexpr size_t FU_PACK_MAX = (size_t)16 << 30;
 
 // Workspace: published words, pairs, fallback v, padded rows.
-struct FuSpace { size_t part, vll, stll, ell, pairs, vfix, pack, total; };
+struct FuSpace { size_t part, vll, stll, ell, pairs, vfix, mass, pack, total; };
 template <typename T>
 FuSpace fu_space(int64_t n, int64_t m, int grid, const FuDevice& d) {
   FuSpace w{};
@@ -1212,6 +1264,7 @@ FuSpace fu_space(int64_t n, int64_t m, int grid, const FuDevice& d) {
   w.ell = take(96 * (size_t)grid);
   w.pairs = take(2 * sizeof(T) * (size_t)grid * m);
   w.vfix = take(sizeof(T) * (size_t)m);
+  w.mass = take(8 * (size_t)grid);
   w.pack = off;
   const bool streamed = !f.res || (sizeof(T) == 8 && !fu_plan<T>(n, m, true, grid, d, g));
   if (streamed && m % Vec<T>::N) {
@@ -1311,6 +1364,7 @@ int fused_run(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st) {
   A.part = (unsigned long long*)(base + w.part); A.vll = (unsigned long long*)(base + w.vll);
   A.stll = (unsigned long long*)(base + w.stll); A.ell = (unsigned long long*)(base + w.ell);
   A.pairs = (T*)(base + w.pairs); A.vfix = (T*)(base + w.vfix);
+  A.mass = (double*)(base + w.mass);
   A.out_u = (T*)p->out_u; A.out_v = (T*)p->out_v;
   A.hist = fs.hist; A.hist_cap = p->hist_cap; A.info = fs.info; A.bar = fs.bar;
   A.timeout_ns = fs.timeout_ns;
