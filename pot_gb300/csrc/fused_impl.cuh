@@ -19,10 +19,16 @@
 // three trips to L2) and the loads behind it one more trip, so the column
 // sums and the new v do not go through barriers: each value is stored in one
 // 64-bit word with the iteration number (a float64 in two such words) and the
-// reader polls the value itself.  A slot is rewritten only after its writer
-// has read all of the next v, which every reader of the slot has contributed
-// to, and v likewise, so single buffers are enough.  Per-iteration flags and
-// error shares travel the same way and every CTA takes the same decisions.
+// reader polls the value itself.  A slot of column sums is rewritten only
+// after its writer has read all of the next v and the flags, to which every
+// reader of the slot has contributed by then.  v, the per-iteration flags and
+// the error shares, which travel the same way so that every CTA takes the same
+// decisions, are rewritten only behind the merge, and nobody leaves the merge
+// before it has seen column sums of the iteration from every CTA, which a CTA
+// publishes when it is done with all three: single buffers are enough.  (With
+// more CTAs than columns some have no column to merge.  They wait for the
+// first column's sums like the CTA that owns it; without that nothing stood
+// between reading the flags of one iteration and writing those of the next.)
 //
 // Split.  A CTA of 8 warps (255 registers a thread: nothing may spill, as the
 // shared memory leaves an L1 of 28 KB and a spilled loop runs at L2 latency;
@@ -699,6 +705,15 @@ __device__ __forceinline__ bool fu_merge(const FusedArgs<T>& A, const FuRow& R, 
   const int sub = R.warp % per, mine = R.warp / per;
   const int step = per * SL;
   bool ok = true;
+  if (!PAIRS && mc == 0) {
+    // (a grid of more than m CTAs; a slot is not rewritten before this CTA's flags are out)
+    for (int p = threadIdx.x; p < np && ok; p += FU_THREADS) {
+      const unsigned long long* q = A.part + (int64_t)p * A.m * Ll<T>::N;
+      typename Ll<T>::W x = Ll<T>::get(q);
+      ok = ll_wait<T>(q, ep, x, A.info + 3, A.timeout_ns);
+    }
+    return __syncthreads_and(ok);
+  }
   for (int b0 = 0; b0 < ncb; b0 += at_once) {
     const int blk = b0 + mine;
     const int j = cb + blk * LC + R.lane % LC;

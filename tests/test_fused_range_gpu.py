@@ -84,3 +84,54 @@ def test_bins_of_every_magnitude(cuda, n, m, dtype, scale):
     assert float(a.min()) == 0.0 and 0.0 < float(a[a > 0].min()) < torch.finfo(dtype).tiny
     b *= float(a.double().sum() / b.double().sum())
     _check(_line(n, m, dtype, cuda), a, b, 0.01, 25)
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("n,m", [(16384, 32), (10000, 50), (2600, 96), (40000, 3), (6000, 1)])
+@pytest.mark.parametrize("method", ["log", "scaling", "unbalanced"])
+def test_more_ctas_than_columns(cuda, n, m, dtype, method):
+    """CTAs without a column of their own wait for nobody in the merge: many
+    iterations, every run the same bits and the right answer."""
+    g = torch.Generator(device=cuda)
+    g.manual_seed(n + m)
+    r = lambda *s: torch.rand(*s, generator=g, device=cuda, dtype=F64)  # noqa: E731
+    M = ((r(n, 1) - r(1, m)) ** 2).to(dtype)
+    a, b = r(n) + 0.2, r(m) + 0.2
+    a, b = (a / a.sum()).to(dtype), (b / b.sum()).to(dtype)
+    iters, kw, code = 3000, {}, {"log": LOG, "scaling": _lib.OTG_METHOD_KNOPP, "unbalanced": _lib.OTG_METHOD_UNB}[method]
+    if method == "unbalanced":
+        kw = {"unbalanced": (0.7, 0.7, 0), "check_period": 1}
+    runs = [bregman.solve_dense(M, a, b, 0.05, code, iters, 0.0, **kw) for _ in range(3)]
+    for s in runs:
+        assert s.status == _lib.STATUS_MAXITER
+        assert torch.equal(s.u, runs[0].u) and torch.equal(s.v, runs[0].v)
+    u, v = (runs[0].u.double(), runs[0].v.double())
+    # both marginals at the fixed point (unbalanced: u = (a / K v)^fi of the plan's own row sums)
+    if method == "unbalanced":
+        K = torch.exp(-M.double() / 0.05) * a.double()[:, None] * b.double()[None, :]
+        fi = 0.7 / 0.75
+        x, y = (a.double() / (K @ v)) ** fi, (b.double() / (K.T @ u)) ** fi
+    else:
+        if method == "scaling":
+            u, v = torch.log(u), torch.log(v)
+        P = torch.exp(u[:, None] + v[None, :] - M.double() / 0.05)
+        x, y, u, v = P.sum(1), P.sum(0), a.double(), b.double()
+    tol = 1e-8 if dtype == F64 else 2e-4
+    assert float(((x - u) / u).abs().max()) < tol and float(((y - v) / v).abs().max()) < tol
+
+
+def test_gradient_with_more_ctas_than_columns(cuda):
+    from pot_gb300._autograd import implicit_grads
+    n, m = 6000, 20
+    g = torch.Generator(device=cuda)
+    g.manual_seed(5)
+    r = lambda *s: torch.rand(*s, generator=g, device=cuda, dtype=F64)  # noqa: E731
+    M, a, b = r(n, m), r(n) + 0.3, r(m) + 0.3
+    a, b = a / a.sum(), b / b.sum()
+    s = bregman.solve_dense(M, a, b, 0.5, LOG, 2000, 1e-13)
+    P = torch.exp(s.u[:, None] + s.v[None, :] - M / 0.5)
+    ref = implicit_grads(P.cpu(), M.cpu(), a.cpu(), b.cpu(), 0.5)
+    for _ in range(200):
+        got = implicit_grads(P, M, a, b, 0.5)
+    for x, y in zip(got, ref):
+        assert float((x.cpu() - y).abs().max()) <= 1e-8 * max(1e-3, float(y.abs().max()))
