@@ -6,46 +6,55 @@
 // 128-point tiles every CTA read 36 KiB per tile from L2 at 22 B per
 // SM-cycle: 1660 cycles a tile, and n = 16384 left 24 of 152 SMs without a
 // row block.  Here
-//   - a cluster of two CTAs owns two row blocks; each CTA loads one half of a
-//     streamed tile and multicasts it to both (18 KiB per 128 points and SM);
-//   - a streamed tile is 256 points: one N = 256 MMA reads 12 KiB of shared
-//     memory in 128 cycles, where two N = 128 MMAs read 16 KiB, all that the
-//     shared memory delivers, with the arriving tiles still to be written;
+//   - a cluster of two CTAs owns two row blocks and takes them as one M = 256
+//     MMA (cta_group::2): each CTA holds its own row block and one half of
+//     the 256-point tile, both loaded for itself alone (18 KiB per 128 points
+//     and SM), the MMA reads the halves of both, and each CTA's TMEM gets its
+//     own 128 rows;
+//   - N = 256: per 128 cycles a CTA reads 8 KiB of shared memory, where two
+//     N = 128 MMAs of one CTA read 16 KiB, all that the shared memory
+//     delivers, with the arriving tiles still to be written;
 //   - the (row pair, tile) units are cut into one contiguous range per
 //     cluster; a row pair that several clusters share leaves its row sums in
 //     slots, and the last CTA to arrive adds the slots in order (the sums are
 //     all relative to the row's one shift) and finishes the rows.  No CTA
 //     waits for another cluster.
-// Measured, one pass: 16384 x 16384, d = 64: 106.6 -> 59.9 us (1.87 PFLOP/s
-// issued, the rate of the bf16 GEMM); 3000 x 3000, d = 40: 22.5 -> 9.2 us;
-// 500 x 500 (launch latency): 6.7 -> 6.8 us.  Programmatic launches of the
-// pass and of its fix-up: 30 iterations at 16384 x 16384 4.63 -> 4.40 ms, at
-// 500 x 500 1.05 -> 0.82 ms.
-// Stages hold one plane of a tile (hi, then lo with the extension columns) so
-// that a stage is free after 8 or 5 MMAs; two resident row tiles, two
-// 256-column accumulators.
+// Measured, a pass and its fix-up (time of 30 more iterations over 60): 16384
+// x 16384, d = 64: 62.3 us, 19456 x 19456: 79.8, 65536 x 65536: 936; with the
+// halves copied into both CTAs and an N = 256 MMA in each: 64.3, 84.2, 979.
+// (With a row block per CTA and 128-point tiles the pass alone took 106.6 at
+// 16384 x 16384.)  3000 x 3000, d = 40: 12.8; 500 x 500, d = 10 (launch
+// latency): 8.8.  Programmatic
+// launches of the pass and of its fix-up: 30 iterations at 16384 x 16384 4.63
+// -> 4.40 ms, at 500 x 500 1.05 -> 0.82 ms.
+// Stages hold one plane of a CTA's half tile (hi, then lo with the extension
+// columns) so that a stage is free after 8 or 5 MMAs; two resident row tiles,
+// two 256-column accumulators.
+//
+// Barriers of the pair.  The even CTA (the leader) issues the MMAs, so its
+// barriers count what both CTAs load (`full`, `res_full`: each CTA's copies
+// complete on the leader's barrier) and what both epilogues release (`acce`).
+// The MMAs' completion arrives in both (`empty`, `res_empty`, `accf`).
 #pragma once
 
 namespace otg {
 
 constexpr int OS_N = 256;              // streamed points per tile
 constexpr int OS_NBUF = 2;             // TMEM accumulators of 256 columns
-constexpr int OS_MAXST = 8;            // barrier slots (stages): 4 wide, 8 narrow
+constexpr int OS_MAXST = 16;           // barrier slots (stages): 8 wide, 16 narrow
 constexpr int OS_MAX_CLUSTERS = 128;   // ranges of a pass at most (room for their partial sums)
-constexpr uint32_t OS_EXT = OS_N * 32; // extension columns of a tile (8 KiB)
 
 // Shared-memory plan by plane width (64 or 16 halves).
 template <bool NARROW> struct OsGeo {
   static constexpr uint32_t row = NARROW ? 32 : 128;           // bytes of a plane row
-  static constexpr uint32_t plane = OS_N * row;                // a stage: one plane of a tile
-  static constexpr int ns = NARROW ? 8 : 4;                    // stages
-  static constexpr uint32_t res_plane = OL_M * row;
-  static constexpr uint32_t res = 2 * res_plane + OL_EXT;      // resident hi, lo, extension
-  static constexpr uint32_t ring = ns * plane, ext = ns / 2 * OS_EXT;
+  static constexpr uint32_t plane = OL_M * row;                // a stage: one plane of half a tile
+  static constexpr int ns = NARROW ? 16 : 8;                   // stages
+  static constexpr uint32_t res = 2 * plane + OL_EXT;          // resident hi, lo, extension
+  static constexpr uint32_t ring = ns * plane, ext = ns / 2 * OL_EXT;
   static constexpr uint32_t bytes = 2 * res + ring + ext;
 };
 static_assert(OsGeo<false>::res % 1024 == 0 && OsGeo<true>::res % 1024 == 0, "swizzle atoms stay aligned");
-constexpr size_t OS_SMEM_EXTRA = 1024 /*align*/ + 256 /*barriers, flags*/ + 3 * OL_M * 4 /*column groups' sums*/;
+constexpr size_t OS_SMEM_EXTRA = 1024 /*align*/ + 512 /*barriers, flags*/ + 3 * OL_M * 4 /*column groups' sums*/;
 
 struct OsWork {          // what a pass adds to OnlinePass
   int row_pairs, tiles;  // pairs of row blocks, 256-point tiles
@@ -62,22 +71,49 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Load a box into the same shared-memory offset of both CTAs of the pair;
-// each CTA's barrier at that offset gets the bytes.
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* tmap, int x, int y, uint64_t* bar) {
+// The shared::cluster address of an object of the leader at this CTA's offset.
+__device__ __forceinline__ uint32_t leader_addr(const void* p) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_addr(p)));
+  return r;
+}
+// TMA load into this CTA whose bytes complete on the leader's barrier.
+__device__ __forceinline__ void tma_load_2d_leader(void* dst, const CUtensorMap* tmap, int x, int y, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster "
-      "[%0], [%1, {%2, %3}], [%4], %5;"
-      :: "r"(smem_addr(dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(smem_addr(bar)),
-         "h"((unsigned short)3)
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      :: "r"(smem_addr(dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+// Arrive on the leader's barrier.  (Nothing in memory is handed over, only
+// TMEM columns, which the tcgen05 fences order: no cluster-scope release,
+// whose fence cost 0.27 us a tile: 16384 x 16384, d = 64, 77 us a pass.)
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory");
+}
+// D (+)= A B^T over the pair: rows of both CTAs' A tiles, points of both
+// halves of B (descriptors: the same offsets in either CTA).  Leader only.
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // Arrive on the barrier at this offset in both CTAs of the pair once every
 // MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
   asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
       :: "r"(smem_addr(bar)), "h"((unsigned short)3) : "memory");
+}
+// TMEM of the pair, by one full warp of each CTA.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(slot)), "r"(ncols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(taddr), "r"(ncols) : "memory");
 }
 
 // Programmatic launches (a no-op in ordinary ones): the next kernel may be
@@ -116,7 +152,7 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
   int* uflag = reinterpret_cast<int*>(tslot + 1);       // a row of the unit failed
   int* dead = uflag + 1;                                // an epilogue warp gave up
   int* last = uflag + 2;                                // this CTA finishes the row block
-  float* red = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(bars) + 256);
+  float* red = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(bars) + 512);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank(), cid = blockIdx.x >> 1;
   const int T = W.tiles;
@@ -124,14 +160,14 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
   const int64_t u0 = os_first(cid, units, W.clusters), u1 = os_first(cid + 1, units, W.clusters);
   if (threadIdx.x == 0) {
     for (int k = 0; k < 2; ++k) { mbar_init(res_full + k, 1); mbar_init(res_empty + k, 1); }
-    for (int k = 0; k < OS_NBUF; ++k) { mbar_init(accf + k, 1); mbar_init(acce + k, OL_EPI); }
-    for (int k = 0; k < OS_MAXST; ++k) { mbar_init(full + k, 1); mbar_init(empty + k, 2); }  // free in both CTAs
+    for (int k = 0; k < OS_NBUF; ++k) { mbar_init(accf + k, 1); mbar_init(acce + k, 2 * OL_EPI); }
+    for (int k = 0; k < OS_MAXST; ++k) { mbar_init(full + k, 1); mbar_init(empty + k, 1); }
     *uflag = 0;
     *dead = 0;
     fence_mbar_init();
     prefetch_tmap(&tAh); prefetch_tmap(&tAl); prefetch_tmap(&tBh); prefetch_tmap(&tBl); prefetch_tmap(&tR); prefetch_tmap(&tS);
   }
-  if (warp == OL_EPI + 1) tmem_alloc(tslot, OS_NBUF * OS_N);
+  if (warp == OL_EPI + 1) tmem_alloc_pair(tslot, OS_NBUF * OS_N);
   tc_fence_before();
   cluster_sync_all();  // the peer's barriers are set before anything arrives on them
   tc_fence_after();
@@ -141,8 +177,10 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
 
   if (warp == OL_EPI) {
     // producer: per segment (row pair, tiles of the range) the CTA's own
-    // resident rows, then its half of every stage, for both CTAs
+    // resident rows, then its half of every tile; the leader's barriers
+    // expect both CTAs' bytes
     if (lane == 0) {
+      const bool leader = rank == 0;
       int q = 0, seg = 0;
       bool ok = true;
       for (int64_t u = u0; u < u1 && ok; ++seg) {
@@ -150,39 +188,40 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
         const int r0 = (2 * rp + rank) * OL_M, rs = seg & 1;
         if (seg > 1 && !mbar_wait(res_empty + rs, ((seg >> 1) - 1) & 1, P.abort_flag, P.timeout_ns)) { ok = false; break; }
         unsigned char* res = resident + rs * G::res;
-        mbar_arrive_expect_tx(res_full + rs, G::res);
-        tma_load_2d(res, &tAh, 0, r0, res_full + rs);
-        tma_load_2d(res + G::res_plane, &tAl, 0, r0, res_full + rs);
-        tma_load_2d(res + 2 * G::res_plane, &tR, 0, r0, res_full + rs);
+        const uint32_t rbar = leader_addr(res_full + rs);
+        if (leader) mbar_arrive_expect_tx(res_full + rs, 2 * G::res);
+        tma_load_2d_leader(res, &tAh, 0, r0, rbar);
+        tma_load_2d_leader(res + G::plane, &tAl, 0, r0, rbar);
+        tma_load_2d_leader(res + 2 * G::plane, &tR, 0, r0, rbar);
         for (int k = 0; k < 2 * (t1 - t0); ++k, ++q) {
           const int s = q % G::ns, y = (t0 + (k >> 1)) * OS_N + rank * OL_M;
           if (!mbar_wait(empty + s, ((q / G::ns) & 1) ^ 1, P.abort_flag, P.timeout_ns)) { ok = false; break; }
-          unsigned char* st = ring + s * G::plane + rank * G::res_plane;
-          if (k & 1) {
-            mbar_arrive_expect_tx(full + s, G::plane + OS_EXT);
-            tma_load_2d_pair(st, &tBl, 0, y, full + s);
-            tma_load_2d_pair(exts + (s >> 1) * OS_EXT + rank * OL_EXT, &tS, 0, y, full + s);
-          } else {
-            mbar_arrive_expect_tx(full + s, G::plane);
-            tma_load_2d_pair(st, &tBh, 0, y, full + s);
-          }
+          const uint32_t bar = leader_addr(full + s);
+          if (leader) mbar_arrive_expect_tx(full + s, 2 * (G::plane + ((k & 1) ? OL_EXT : 0u)));
+          tma_load_2d_leader(ring + s * G::plane, (k & 1) ? &tBl : &tBh, 0, y, bar);
+          if (k & 1) tma_load_2d_leader(exts + (s >> 1) * OL_EXT, &tS, 0, y, bar);
         }
         u += t1 - t0;
       }
-      // copies in flight land, and both CTAs' releases of the last stages
-      // arrive, before the CTA leaves
+      // Copies in flight land and the MMAs' arrivals are in before the CTA
+      // leaves (the leader's waits cover the copies of both; the pair leaves
+      // together).
       const uint64_t w0 = globaltimer();
       for (int k = q > G::ns ? q - G::ns : 0; k < q; ++k) {
-        while (!mbar_try_wait(full + k % G::ns, (k / G::ns) & 1)) if (globaltimer() - w0 > P.timeout_ns) break;
+        if (leader)
+          while (!mbar_try_wait(full + k % G::ns, (k / G::ns) & 1)) if (globaltimer() - w0 > P.timeout_ns) break;
         while (!mbar_try_wait(empty + k % G::ns, (k / G::ns) & 1)) if (globaltimer() - w0 > P.timeout_ns) break;
       }
-      for (int k = seg > 2 ? seg - 2 : 0; k < seg; ++k)
-        while (!mbar_try_wait(res_full + (k & 1), (k >> 1) & 1)) if (globaltimer() - w0 > P.timeout_ns) break;
+      for (int k = seg > 2 ? seg - 2 : 0; k < seg; ++k) {
+        if (leader)
+          while (!mbar_try_wait(res_full + (k & 1), (k >> 1) & 1)) if (globaltimer() - w0 > P.timeout_ns) break;
+        while (!mbar_try_wait(res_empty + (k & 1), (k >> 1) & 1)) if (globaltimer() - w0 > P.timeout_ns) break;
+      }
     }
   } else if (warp == OL_EPI + 1) {
     // MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_f16(OL_M, OS_N, false);
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc = umma_idesc_f16(2 * OL_M, OS_N, false);
       int q = 0, n = 0, seg = 0;
       bool ok = true;
       for (int64_t u = u0; u < u1 && ok; ++seg) {
@@ -194,7 +233,7 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
           if (!mbar_wait(acce + b, ((n / OS_NBUF) & 1) ^ 1, P.abort_flag, P.timeout_ns)) { ok = false; break; }
           const uint32_t dst = tmem + (uint32_t)(b * OS_N);
           const uint64_t ah = NARROW ? umma_desc_k32(res) : umma_desc_k128(res);
-          const uint64_t al = NARROW ? umma_desc_k32(res + G::res_plane) : umma_desc_k128(res + G::res_plane);
+          const uint64_t al = NARROW ? umma_desc_k32(res + G::plane) : umma_desc_k128(res + G::plane);
           int s = q % G::ns;
           if (!mbar_wait(full + s, (q / G::ns) & 1, P.abort_flag, P.timeout_ns)) { ok = false; break; }
           tc_fence_after();
@@ -202,8 +241,8 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < (NARROW ? 1 : OL_K / 16); ++kk) {
             const uint64_t o = (uint64_t)(kk * 32) >> 4;
-            umma_f16(dst, ah + o, bh + o, idesc, kk ? 1u : 0u);
-            umma_f16(dst, al + o, bh + o, idesc, 1);
+            umma_f16_pair(dst, ah + o, bh + o, idesc, kk ? 1u : 0u);
+            umma_f16_pair(dst, al + o, bh + o, idesc, 1);
           }
           umma_commit_pair(empty + s);
           ++q;
@@ -214,14 +253,14 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < (NARROW ? 1 : OL_K / 16); ++kk) {
             const uint64_t o = (uint64_t)(kk * 32) >> 4;
-            umma_f16(dst, ah + o, bl + o, idesc, 1);
+            umma_f16_pair(dst, ah + o, bl + o, idesc, 1);
           }
-          umma_f16(dst, umma_desc_k32(res + 2 * G::res_plane), umma_desc_k32(exts + (s >> 1) * OS_EXT), idesc, 1);
+          umma_f16_pair(dst, umma_desc_k32(res + 2 * G::plane), umma_desc_k32(exts + (s >> 1) * OL_EXT), idesc, 1);
           umma_commit_pair(empty + s);
           ++q;
-          umma_commit(accf + b);
+          umma_commit_pair(accf + b);
         }
-        if (ok) umma_commit(res_empty + rs);
+        if (ok) umma_commit_pair(res_empty + rs);
         u += t1 - t0;
       }
       // every MMA has completed before the accumulators go
@@ -255,7 +294,7 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
         tmem_ld32u(addr + 32, v);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(acce + b);
+        if (lane == 0) mbar_arrive_leader(leader_addr(acce + b));
         ol_fsum_acc(v, sm, sc);
       }
       if (!ok) *dead = 1;
@@ -308,7 +347,7 @@ online_stream_kernel(const __grid_constant__ CUtensorMap tAh, const __grid_const
   cluster_sync_all();  // nothing of the pair's is in flight towards either CTA
   if (warp == OL_EPI + 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, OS_NBUF * OS_N);
+    tmem_dealloc_pair(tmem, OS_NBUF * OS_N);
   }
 }
 
