@@ -9,6 +9,7 @@
 // value = value_linear + reg * sum T log(T + 1e-16) or the KL form).
 #include <algorithm>
 #include "common.cuh"
+#include "launch.cuh"
 #include "../../include/pot_gb300.h"
 
 namespace otg {
@@ -800,15 +801,11 @@ int otg_lazy_loss(int dtype, const void* X, const void* Y, int64_t n, int64_t m,
   const unsigned blocks = (unsigned)((n + LL_ROWS - 1) / LL_ROWS);
   const double c = -OTG_LOG2E / reg;
   if (dtype == OTG_F64) {
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(lazy_loss_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return OTG_ERR_CUDA;
+    if (!allow_smem((const void*)lazy_loss_kernel<double>, smem)) return OTG_ERR_CUDA;
     lazy_loss_kernel<double><<<blocks, 256, smem, stream>>>((const double*)X, (const double*)Y, n, m, d,
                                                             (const double*)f, (const double*)g, c, out);
   } else if (dtype == OTG_F32) {
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(lazy_loss_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return OTG_ERR_CUDA;
+    if (!allow_smem((const void*)lazy_loss_kernel<float>, smem)) return OTG_ERR_CUDA;
     lazy_loss_kernel<float><<<blocks, 256, smem, stream>>>((const float*)X, (const float*)Y, n, m, d,
                                                            (const float*)f, (const float*)g, (float)c, out);
   } else {

@@ -73,6 +73,7 @@
 #include "dense_common.cuh"
 #include "fused.cuh"
 #include "fused_ops.cuh"
+#include "launch.cuh"
 
 namespace otg {
 
@@ -1294,10 +1295,7 @@ FuSpace fu_space(int64_t n, int64_t m, int grid, const FuDevice& d) {
 template <typename T, int MODE, int NK, bool RES>
 int fu_start(FusedArgs<T>& A, const FuPlan& f, cudaStream_t st) {
   const void* k = (const void*)fused_sinkhorn_kernel<T, MODE, NK, RES>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) != cudaSuccess) {
-    cudaGetLastError();
-    return OTG_ERR_UNSUPPORTED;
-  }
+  if (!allow_smem(k, f.smem)) return OTG_ERR_UNSUPPORTED;
   void* args[] = {&A};
   return cudaLaunchCooperativeKernel(k, dim3(f.grid), dim3(FU_THREADS), args, f.smem, st) == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
 }

@@ -265,7 +265,7 @@ bool grad_plan(int64_t n, int64_t m, GradPlan& f) {
 template <int NK>
 int grad_start(GradArgs& G, const GradPlan& f, cudaStream_t st) {
   const void* k = (const void*)sinkhorn_grad_kernel<NK>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) != cudaSuccess) return OTG_ERR_CUDA;
+  if (!allow_smem(k, f.smem)) return OTG_ERR_CUDA;
   void* args[] = {&G};
   return cudaLaunchCooperativeKernel(k, dim3(f.grid), dim3(FU_THREADS), args, f.smem, st) == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
 }

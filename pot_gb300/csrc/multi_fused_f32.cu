@@ -2,6 +2,7 @@
 #include <cmath>
 #include "multi_common.cuh"
 #include "multi_fused.cuh"
+#include "launch.cuh"
 
 namespace otg {
 
@@ -26,7 +27,7 @@ namespace {
 template <bool LOGF, int NK>
 int start(const MultiArgs<float>& A, int grid, size_t smem, int32_t* leaving, cudaStream_t st) {
   const void* k = (const void*)multi_fused_kernel<float, LOGF, NK>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return OTG_ERR_CUDA;
+  if (!allow_smem(k, smem)) return OTG_ERR_CUDA;
   MultiArgs<float> a = A;
   void* args[] = {&a, &leaving};
   return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(MT_THREADS), args, smem, st) == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
