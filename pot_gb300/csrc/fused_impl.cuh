@@ -50,9 +50,14 @@
 // potential less log a_i, so e_ij is the row's previous plan entry over a_i
 // and s_i is near one; rows whose s_i leaves [2^-30, 2^30] (first iterations
 // from a far start, zero weights, non-finite input) take the running-maximum
-// form on the same entries.  A column whose sum is below 2^-70 may have lost
-// terms to underflow: then the whole grid recomputes the column update with
-// running maxima (one extra pass) in that iteration.
+// form on the same entries.  What can be lost in a column sum are entries
+// below 2^-126 (2^-1074 in float64) times the row factors a_i / s_i, together
+// 2^-96 (2^-1044) of the mass.  A column sum that is not 2^26 (2^59) times
+// that is recomputed in that iteration with running maxima: one more pass over
+// such columns and two grid barriers.  (Bounds that know neither the type nor
+// the mass, and a pass over all columns, made Gaussian histograms, whose tails
+// meet them in every iteration, slower than two passes: 8192^2 float32 278 us
+// per iteration, two passes 95; 3000 x 1100 float64 439, two passes 845.)
 //
 // float64 log form, cost resident: this GPU issues FP64 at about two lanes
 // per clock and SM, and an exponential costs some twenty such operations.
@@ -94,7 +99,7 @@ struct FusedArgs {
   unsigned long long *part, *vll, *stll, *ell;   // published words, see Ll
   T* pairs;                  // [grid][m] (maximum, sum) pairs: first and fallback column pass
   T* vfix;                   // [m] v of the fallback column pass
-  double* mass;              // [grid] sum of a over the CTA's rows (FU_ABS)
+  double* mass;              // [grid] sum of a over the CTA's rows (log forms)
   T *out_u, *out_v;
   double* hist; int hist_cap;
   int* info;                 // status, niter, nchecks, abort
@@ -189,13 +194,6 @@ __device__ __forceinline__ void fu_get_global(const FusedArgs<T>& A, int row, in
   }
 }
 
-// x >= lim > 0; false for a NaN.  (Doubles by integers: an FP64 comparison
-// issues at two lanes per clock.)
-__device__ __forceinline__ bool fu_at_least(float x, float lim) { return x >= lim; }
-__device__ __forceinline__ bool fu_at_least(double x, double lim) {
-  const long long b = __double_as_longlong(x);
-  return b >= __double_as_longlong(lim) && b <= 0x7ff0000000000000ll;
-}
 // A scaling of FU_ABS that needs no absorption: within [2^-300, 2^300].
 __device__ __forceinline__ bool fu_tame(double x) { return fu_at_least(x, 0x1p-300) && !fu_at_least(x, 0x1p300); }
 
@@ -587,11 +585,13 @@ __device__ __noinline__ void fu_colsum(const FusedArgs<T>& A, const FuRow& R, co
 }
 
 // Column log-sum-exps alone (log forms: first iteration and the fallback):
-// (maximum, sum) pairs of x_ij + u_i over the CTA's rows, four vectors of a
-// thread at a time.
-template <typename T, bool TILE>
+// (maximum, sum) pairs of x_ij + u_i over the CTA's rows, sixteen loads of a
+// thread in flight: four rows of four vectors.  MARKED: only vectors with a
+// column whose sm.vs is NaN, sixteen rows of one, as few threads have several
+// (8192^2 float32, an eighth of the columns marked: four by four 67 us).
+template <typename T, bool TILE, bool MARKED>
 __device__ __noinline__ void fu_collse(const FusedArgs<T>& A_, const FuRow& R_, const FuSmem<T>& sm_, const T* u) {
-  constexpr int W = Vec<T>::N, KB = 4;
+  constexpr int W = Vec<T>::N, KB = MARKED ? 1 : 4, RW = 16 / KB;
   const FusedArgs<T> A = A_;
   const FuRow R = R_;
   const FuSmem<T> sm = sm_;
@@ -602,21 +602,31 @@ __device__ __noinline__ void fu_collse(const FusedArgs<T>& A_, const FuRow& R_, 
     for (int k = 0; k < KB; ++k)
 #pragma unroll
       for (int w = 0; w < W; ++w) { mx[k][w] = -INFINITY; s[k][w] = 0; }
-    // four rows per update: one rescaling exponential for them
-    for (int row = R.ga; row < R.gb; row += 4) {
-      T ui[4];
+    bool on = true;
+    if (MARKED) {
+      const int at = (k0 * R.gt + R.tg) * W;
+      T v[W];
+      fu_get(sm.vs + at, v);
+      on = false;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) ui[q] = row + q < R.gb ? __ldcg(u + row + q) : T(-INFINITY);
-      // the block's sixteen loads in flight at once (vectors beyond the row
-      // read its first one and are not stored)
-      T x[KB][4][W];
+      for (int w = 0; w < W; ++w) on |= at + w < A.m && isnan(v[w]);
+      if (!__syncthreads_or(on)) continue;
+    }
+    // one rescaling exponential per column for the rows of an update
+    for (int row = on ? R.ga : R.gb; row < R.gb; row += RW) {
+      T ui[RW];
+#pragma unroll
+      for (int q = 0; q < RW; ++q) ui[q] = row + q < R.gb ? __ldcg(u + row + q) : T(-INFINITY);
+      // (vectors beyond the row read its first one and are not stored)
+      T x[KB][RW][W];
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
         const int at = ((k0 + k) * R.gt + R.tg) * W, col = at < A.mv ? at : 0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < RW; ++q) {
           const int r = min(row + q, R.gb - 1);
           if (TILE) fu_get(sm.data + (r - R.r0) * A.mp + col, x[k][q]);
+          else if (MARKED) unpack(ld_stream(reinterpret_cast<const typename Vec<T>::type*>(A.M + (int64_t)r * A.ldm + col)), x[k][q]);
           else fu_get_global(A, r, col, pad, x[k][q]);
         }
       }
@@ -624,14 +634,14 @@ __device__ __noinline__ void fu_collse(const FusedArgs<T>& A_, const FuRow& R_, 
       for (int k = 0; k < KB; ++k) {
 #pragma unroll
         for (int w = 0; w < W; ++w) {
-          T t[4], top = mx[k][w];
+          T t[RW], top = mx[k][w];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) { t[q] = row + q < R.gb ? fma(x[k][q][w], A.c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
+          for (int q = 0; q < RW; ++q) { t[q] = row + q < R.gb ? fma(x[k][q][w], A.c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
           // (an empty column so far: the sums stay zero)
           const T ref = top == -INFINITY ? T(0) : top;
           T sum = s[k][w] * ex2(mx[k][w] - ref);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) sum += ex2(t[q] - ref);
+          for (int q = 0; q < RW; ++q) sum += ex2(t[q] - ref);
           s[k][w] = sum;
           mx[k][w] = top;
         }
@@ -691,22 +701,22 @@ __device__ __noinline__ void fu_collse(const FusedArgs<T>& A_, const FuRow& R_, 
 // Merge: this CTA's share of the columns over the grid's slots.  LC lanes
 // take adjacent columns and 32 / LC lanes share a column's slots, as do `per`
 // warps; partial sums are added in lane and warp order, so the sum of a
-// column is the same in every run.  fin(j, mx, s) finishes column j.
+// column is the same in every run.  fin(j, s) finishes column j.
 // ---------------------------------------------------------------------------
-template <typename T, bool PAIRS, typename Fin>
-__device__ __forceinline__ bool fu_merge(const FusedArgs<T>& A, const FuRow& R, T* s_s, T* s_m, unsigned ep, Fin&& fin) {
+template <typename T, typename Fin>
+__device__ __forceinline__ bool fu_merge(const FusedArgs<T>& A, const FuRow& R, T* s_s, unsigned ep, Fin&& fin) {
   const int np = gridDim.x;
   const int cb = (int)((int64_t)A.m * blockIdx.x / gridDim.x), ce = (int)((int64_t)A.m * (blockIdx.x + 1) / gridDim.x);
   const int mc = ce - cb;
   int LC = 32;
-  if (!PAIRS) while (LC > 4 && LC / 2 >= mc) LC /= 2;
+  while (LC > 4 && LC / 2 >= mc) LC /= 2;
   const int SL = 32 / LC, ncb = (mc + LC - 1) / LC;
   const int per = ncb >= FU_WARPS ? 1 : (ncb ? FU_WARPS / ncb : 1);
   const int at_once = FU_WARPS / per;
   const int sub = R.warp % per, mine = R.warp / per;
   const int step = per * SL;
   bool ok = true;
-  if (!PAIRS && mc == 0) {
+  if (mc == 0) {
     // (a grid of more than m CTAs; a slot is not rewritten before this CTA's flags are out)
     for (int p = threadIdx.x; p < np && ok; p += FU_THREADS) {
       const unsigned long long* q = A.part + (int64_t)p * A.m * Ll<T>::N;
@@ -719,51 +729,81 @@ __device__ __forceinline__ bool fu_merge(const FusedArgs<T>& A, const FuRow& R, 
     const int blk = b0 + mine;
     const int j = cb + blk * LC + R.lane % LC;
     const bool live = mine < at_once && blk < ncb && j < ce;
-    T mx = -INFINITY, s = 0;
+    T s = 0;
     if (live) {
-      if (PAIRS) {
-        for (int p = sub; p < np; p += per) {
-          const T* q = A.pairs + 2 * ((int64_t)p * A.m + j);
-          lse_merge(mx, s, __ldcg(q), __ldcg(q + 1));
-        }
-      } else {
-        constexpr int U = sizeof(T) == 8 ? 4 : 8;
-        const int64_t stride = (int64_t)step * A.m * Ll<T>::N;
-        int p = sub * SL + R.lane / LC;
-        const unsigned long long* q = A.part + ((int64_t)p * A.m + j) * Ll<T>::N;
-        for (; p < np; p += U * step, q += U * stride) {
-          typename Ll<T>::W x[U];
+      constexpr int U = sizeof(T) == 8 ? 4 : 8;
+      const int64_t stride = (int64_t)step * A.m * Ll<T>::N;
+      int p = sub * SL + R.lane / LC;
+      const unsigned long long* q = A.part + ((int64_t)p * A.m + j) * Ll<T>::N;
+      for (; p < np; p += U * step, q += U * stride) {
+        typename Ll<T>::W x[U];
 #pragma unroll
-          for (int k = 0; k < U; ++k)
-            if (p + k * step < np) x[k] = Ll<T>::get(q + k * stride);
+        for (int k = 0; k < U; ++k)
+          if (p + k * step < np) x[k] = Ll<T>::get(q + k * stride);
 #pragma unroll
-          for (int k = 0; k < U; ++k)
-            if (p + k * step < np) {
-              ok = ok && ll_wait<T>(q + k * stride, ep, x[k], A.info + 3, A.timeout_ns);
-              s += Ll<T>::value(x[k]);
-            }
-        }
+        for (int k = 0; k < U; ++k)
+          if (p + k * step < np) {
+            ok = ok && ll_wait<T>(q + k * stride, ep, x[k], A.info + 3, A.timeout_ns);
+            s += Ll<T>::value(x[k]);
+          }
       }
     }
-    if (!PAIRS) {
-      __syncwarp();
-      for (int o = LC; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    }
+    __syncwarp();
+    for (int o = LC; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (per > 1) {
       s_s[R.warp * 32 + R.lane] = s;
-      if (PAIRS) s_m[R.warp * 32 + R.lane] = mx;
       __syncthreads();
-      if (live && sub == 0 && R.lane < LC) {
-        for (int q = 1; q < per; ++q) {
-          if (PAIRS) lse_merge(mx, s, s_m[(R.warp + q) * 32 + R.lane], s_s[(R.warp + q) * 32 + R.lane]);
-          else s += s_s[(R.warp + q) * 32 + R.lane];
-        }
-      }
+      if (live && sub == 0 && R.lane < LC)
+        for (int q = 1; q < per; ++q) s += s_s[(R.warp + q) * 32 + R.lane];
       __syncthreads();
     }
-    if (live && sub == 0 && R.lane < LC) fin(j, mx, s);
+    if (live && sub == 0 && R.lane < LC) fin(j, s);
   }
   return ok;
+}
+
+// The same of (maximum, sum) pairs, behind a grid barrier: the column update
+// log2 b - log2 sum exp into vfix and, as epoch `pub`, the published v.  `ep`:
+// only columns whose v of that epoch is NaN.  Blocks of 32 columns go around
+// the CTAs (the marked ones are neighbours), a block's slots around the warps.
+// Out of line: it runs once or for columns that underflowed, and its registers
+// must not weigh on the passes.
+template <typename T>
+__device__ __noinline__ void fu_merge_pairs(const FusedArgs<T>& A, T* s_s, T* s_m, unsigned ep, unsigned pub) {
+  constexpr int U = 10;  // slots of a warp in flight (19 of 152)
+  const int warp = threadIdx.x >> 5, np = gridDim.x;
+  for (int j0 = 32 * blockIdx.x; j0 < A.m; j0 += 32 * gridDim.x) {
+    const int j = j0 + (threadIdx.x & 31);
+    bool live = j < A.m;
+    if (ep) {
+      if (live) live = isnan(Ll<T>::value(Ll<T>::get(A.vll + j * Ll<T>::N)));
+      if (!__any_sync(0xffffffffu, live)) continue;  // (the same in every warp)
+    }
+    T mx = -INFINITY, s = 0;
+    if (live)
+      for (int p = warp; p < np; p += U * FU_WARPS) {
+        T m2[U], s2[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+          const bool in = p + k * FU_WARPS < np;
+          const T* q = A.pairs + 2 * ((int64_t)(in ? p + k * FU_WARPS : p) * A.m + j);
+          m2[k] = in ? __ldcg(q) : T(-INFINITY);
+          s2[k] = in ? __ldcg(q + 1) : T(0);
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) lse_merge(mx, s, m2[k], s2[k]);
+      }
+    s_s[threadIdx.x] = s;
+    s_m[threadIdx.x] = mx;
+    __syncthreads();
+    if (live && warp == 0) {
+      for (int q = 1; q < FU_WARPS; ++q) lse_merge(mx, s, s_m[q * 32 + threadIdx.x], s_s[q * 32 + threadIdx.x]);
+      const T vn = lg2(A.b[j]) - lse_value(mx, s);
+      A.vfix[j] = vn;
+      if (pub) Ll<T>::put(A.vll + j * Ll<T>::N, vn, pub);
+    }
+    __syncthreads();
+  }
 }
 
 // The flags that any thread of the CTA has.
@@ -866,7 +906,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
     for (int w = 0; w < Ll<T>::N; ++w) A.vll[j * Ll<T>::N + w] = 0ull;
   }
   for (int j = threadIdx.x; j < A.m * Ll<T>::N; j += FU_THREADS) A.part[(int64_t)blockIdx.x * A.m * Ll<T>::N + j] = 0ull;
-  if (MODE == FU_ABS) {
+  if (LOGF) {
     double w = 0.0;
     for (int i = R.r0 + threadIdx.x; i < R.r1; i += FU_THREADS) w += widen(A.a[i]);
     w = block_sum_fixed(w);
@@ -934,7 +974,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
       const unsigned ep = (unsigned)ii + 2u;
       FuTrack<T> ut{T(-INFINITY), T(-INFINITY), T(-INFINITY)}, vt = ut;
       int flag = fu_pass<T, MODE, NK, RES>(A, R, sm, red, rr, ring, ucur, unxt, H, held, ut, ep);
-      ok = fu_merge<T, false>(A, R, s_s, s_m, ep, [&](int j, T, T s) {
+      ok = fu_merge<T>(A, R, s_s, ep, [&](int j, T s) {
         const T be = A.bew ? A.bew[j] : T(1);
         const T vn = pow_unit(A.b[j] / (be * s), A.fi2);
         if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
@@ -1006,15 +1046,12 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
     int flag = 0, got = 0;
     if (MODE != FU_ABS) {
       if (LOGF) {
-        fu_collse<T, RES>(A, R, sm, ucur);
+        fu_collse<T, RES, false>(A, R, sm, ucur);
         ok = fu_barrier(A.bar, gen, abort_flag, A.timeout_ns);
-        if (ok)
-          fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) {
-            Ll<T>::put(A.vll + j * Ll<T>::N, lg2(A.b[j]) - lse_value(mx, s), 1u);
-          });
+        if (ok) fu_merge_pairs(A, s_s, s_m, 0u, 1u);
       } else {
         fu_colsum<T, NK, RES>(A, R, sm, ucur, 1u);
-        ok = fu_merge<T, false>(A, R, s_s, s_m, 1u, [&](int j, T, T s) {
+        ok = fu_merge<T>(A, R, s_s, 1u, [&](int j, T s) {
           const T vn = A.b[j] / s;
           if (s == T(0) || !isfinite(vn)) flag |= FU_BAD_COL;
           Ll<T>::put(A.vll + j * Ll<T>::N, vn, 1u);
@@ -1028,14 +1065,19 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
     // FU_ABS: K is to be built, from a column update of its own (else the
     // scalings are absorbed)
     bool build = MODE == FU_ABS, absolute = true;
-    // Column sums below these may have lost bits to underflow (an entry's
-    // 2^-1075 with row scalings up to 2^30, 2^300; the sum's own roundings).
+    // Column sums below s_lim[1] may have lost bits to underflow (FU_ABS: with
+    // row scalings up to 2^300, s_lim[0] up to 2^30): a part of the mass, and
+    // no less than the roundings of denormals.
     __shared__ T s_lim[2];  // (registers are what the passes have least of)
-    if (MODE == FU_ABS) {
+    if (LOGF) {
       double w = 0.0;
       for (int p = threadIdx.x; p < (int)gridDim.x; p += FU_THREADS) w += __ldcg(A.mass + p);
       w = block_sum_fixed(w);
-      if (threadIdx.x == 0) { s_lim[0] = (T)fmax(w * 0x1p-992, 0x1p-1000); s_lim[1] = (T)fmax(w * 0x1p-722, 0x1p-1000); }
+      if (threadIdx.x == 0) {
+        s_lim[0] = (T)fmax(w * 0x1p-992, 0x1p-1000);
+        s_lim[1] = (T)(MODE == FU_ABS ? fmax(w * 0x1p-722, 0x1p-1000) : sizeof(T) == 8 ? fmax(w * 0x1p-985, 0x1p-1000)
+                                                                                       : fmax(w * 0x1p-70, 0x1p-100));
+      }
     }
     for (int ii = 0; ok; ++ii) {
       // sm.vs holds v of iteration ii, ucur u of iteration ii - 1
@@ -1052,9 +1094,9 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
           // the update of the current row potentials, with running maxima
           for (int i = R.r0 + threadIdx.x; i < R.r1; i += FU_THREADS) A.fref[i] = __ldcg(A.fref + i) - lg2(__ldcg(ucur + i));
           __syncthreads();
-          fu_collse<T, false>(A, R, sm, A.fref);
+          fu_collse<T, false, false>(A, R, sm, A.fref);
           if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
-          fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) { A.vfix[j] = lg2(A.b[j]) - lse_value(mx, s); });
+          fu_merge_pairs(A, s_s, s_m, 0u, 0u);
           if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
         }
         for (int j = threadIdx.x; j < A.mp; j += FU_THREADS) {
@@ -1072,7 +1114,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
       t = vcur; vcur = vnxt; vnxt = t;
       const bool check = ii % A.period == 0, last = ii + 1 == A.max_iter;
       e2 = 0.0;
-      ok = fu_merge<T, false>(A, R, s_s, s_m, ep, [&](int j, T, T s) {
+      ok = fu_merge<T>(A, R, s_s, ep, [&](int j, T s) {
         const T bj = A.b[j], vo = sm.vs[j];
         vcur[j] = vo;
         if (check) {
@@ -1083,7 +1125,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
         T vn;
         if (MODE == FU_LOG) {
           vn = bj == T(0) ? T(-INFINITY) : vo + lg2(bj / s);
-          if (bj != T(0) && !(s >= T(8.470329472543003e-22))) flag |= FU_BAD_COL;  // 2^-70
+          if (bj != T(0) && !fu_at_least(s, s_lim[1])) { flag |= FU_BAD_COL; vn = T(NAN); }
         } else if (MODE == FU_ABS) {
           vn = bj == T(0) ? T(1) : bj / s;
           if (bj != T(0)) {
@@ -1123,12 +1165,15 @@ __global__ void __launch_bounds__(FU_THREADS, 1) fused_sinkhorn_kernel(const __g
         build = absolute || (got & FU_BAD_ROW);
       }
       if (MODE == FU_LOG && (got & FU_BAD_COL)) {
-        // a column sum too small to trust: the column update with running maxima
-        fu_collse<T, RES>(A, R, sm, ucur);
+        // column sums too small to trust (NaN in v): their update with running maxima
+        fu_collse<T, RES, true>(A, R, sm, ucur);
         if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
-        fu_merge<T, true>(A, R, s_s, s_m, 0, [&](int j, T mx, T s) { A.vfix[j] = lg2(A.b[j]) - lse_value(mx, s); });
+        fu_merge_pairs(A, s_s, s_m, ep, 0u);
         if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
-        for (int j = threadIdx.x; j < A.mp; j += FU_THREADS) sm.vs[j] = j < A.m ? __ldcg(A.vfix + j) : vpad;
+        for (int j = threadIdx.x; j < A.m; j += FU_THREADS) {  // (sm.vs was the merge's scratch)
+          const T v = Ll<T>::value(Ll<T>::get(A.vll + j * Ll<T>::N));
+          sm.vs[j] = isnan(v) ? __ldcg(A.vfix + j) : v;
+        }
         __syncthreads();
       }
     }

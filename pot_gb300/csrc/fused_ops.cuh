@@ -175,6 +175,18 @@ __device__ __forceinline__ T fu_group(T (&s)[RB], const FuRow& R, int G, T (*red
   return t;
 }
 
+// x >= lim > 0; false for a NaN.  (Doubles by integers: an FP64 comparison
+// issues at two lanes per clock.)
+__device__ __forceinline__ bool fu_at_least(float x, float lim) { return x >= lim; }
+__device__ __forceinline__ bool fu_at_least(double x, double lim) {
+  const long long b = __double_as_longlong(x);
+  return b >= __double_as_longlong(lim) && b <= 0x7ff0000000000000ll;
+}
+// 2^k, a normal number.
+template <typename T> __device__ __forceinline__ T exp2_of(int k);
+template <> __device__ __forceinline__ float exp2_of<float>(int k) { return __int_as_float((127 + k) << 23); }
+template <> __device__ __forceinline__ double exp2_of<double>(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+
 template <typename T>
 __device__ __forceinline__ bool fu_near_one(T t) { return t >= T(9.313225746154785e-10) && t <= T(1073741824.0); }  // 2^-30, 2^30
 

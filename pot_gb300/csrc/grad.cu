@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) sinkhorn_grad_kernel(const __gr
   unsigned ep = 1;
   double e2 = 0.0;
   gr_pass<NK, 0>(G, R, sm, red, 0.0, ep);
-  bool ok = fu_merge<double, false>(A, R, s_s, s_s, ep, [&](int j, double, double s) { Ll<double>::put(A.vll + 2 * j, s, ep); });
+  bool ok = fu_merge<double>(A, R, s_s, ep, [&](int j, double s) { Ll<double>::put(A.vll + 2 * j, s, ep); });
   if (__syncthreads_or(!ok)) ok = false;
   if (threadIdx.x == 0) ll_st(A.stll + blockIdx.x, 0, ep);
   if (fu_collect(A, sp, ep, false, ok, e2) & FU_ABORT) return;  // sp: the right-hand side
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) sinkhorn_grad_kernel(const __gr
     ++ep;
     __syncthreads();  // p is whole
     gr_pass<NK, 1>(G, R, sm, red, 0.0, ep);
-    ok = fu_merge<double, false>(A, R, s_s, s_s, ep, [&](int j, double, double s) {
+    ok = fu_merge<double>(A, R, s_s, ep, [&](int j, double s) {
       const double bj = A.b[j];
       Ll<double>::put(A.vll + 2 * j, bj * sm.vs[j] - s + (beta * bp) * bj, ep);
     });

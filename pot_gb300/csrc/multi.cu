@@ -956,6 +956,7 @@ int launch_multi(const OtgMultiProblem* q, cudaStream_t st) {
     A.fpart = reinterpret_cast<T*>(A.pcol);
     A.fpairs = A.fpart + span;
     A.fbad = A.nsr;
+    A.flim = A.rchunk;
     int grid = sms;
     if (q->grid > 0 && q->grid < grid) grid = q->grid;
     const int rc = multi_fused_launch(A, LOGF, f.NK, grid, f.smem, leaving, st);

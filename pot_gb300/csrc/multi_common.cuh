@@ -73,6 +73,7 @@ struct MultiArgs {
   int fG, fNK, fNC, fmp, fmm;
   T* fpart; T* fpairs;
   int32_t* fbad;
+  int32_t* flim;            // per problem: exponent below which a column sum cannot be trusted
   double* and_part; double* and_w;  // dots of the blocks of 32 columns, weights of the problems (mf_anderson)
 };
 

@@ -369,10 +369,11 @@ __device__ __forceinline__ bool mf_pass(const MultiArgs<T>& A, const FuRow& R, c
 }
 
 // Column log-sum-exp pairs (LOGF) or column sums of u alone over a worker's
-// share: the first v, and the fallback of problems flagged in A.fbad.
-template <typename T, bool LOGF>
-__device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_, int w, int na, int nact, bool flagged) {
-  constexpr int W = Vec<T>::N, KB = 4;
+// share: the first v, and (MARKED) the columns whose `marks` is NaN of problems
+// flagged in A.fbad.
+template <typename T, bool LOGF, bool MARKED>
+__device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_, int w, int na, int nact, const T* marks) {
+  constexpr int W = Vec<T>::N, KB = MARKED ? 1 : 4, RW = 16 / KB;
   const MultiArgs<T> A = A_;
   const FuRow R = R_;
   const int64_t total = __ldcg(A.urow_pre + nact);
@@ -380,8 +381,9 @@ __device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_,
   mf_range(total, w, na, beg, end);
   for (MfSpan sp = mf_next(A, mt_find(A.urow_pre, nact, beg), nact, beg, end); sp.k < nact; sp = mf_next(A, sp.k + 1, nact, beg, end)) {
     const int p = __ldcg(A.active + sp.k);
-    if (flagged && __ldcg(A.fbad + p) == 0) continue;
-    const int ldm = A.ldm[p], nv = ldm / W;
+    if (MARKED && __ldcg(A.fbad + p) == 0) continue;
+    const int ldm = A.ldm[p], nv = ldm / W, m = A.cols[p];
+    const int64_t co = A.c_off[p];
     const T c = (T)(-OTG_LOG2E / A.reg[p]);
     const T* Mp = A.M + A.m_off[p];
     const T* up = A.u + A.r_off[p];
@@ -392,18 +394,25 @@ __device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_,
       for (int k = 0; k < KB; ++k)
 #pragma unroll
         for (int x = 0; x < W; ++x) { mx[k][x] = -INFINITY; s[k][x] = 0; }
-      for (int row = sp.row; row < sp.end; row += 4) {
-        T ui[4];
+      bool on = true;
+      if (MARKED) {
+        const int j = k0 * R.gt + R.tg;
+        on = false;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) ui[q] = row + q < sp.end ? __ldcg(up + row + q) : (LOGF ? T(-INFINITY) : T(0));
-        // the block's sixteen loads in flight at once (vectors beyond the row
-        // read its first one and are not stored)
-        T x[KB][4][W];
+        for (int x = 0; x < W; ++x) on |= j * W + x < m && isnan(__ldcg(marks + co + j * W + x));
+      }
+      for (int row = on ? sp.row : sp.end; row < sp.end; row += RW) {
+        T ui[RW];
+#pragma unroll
+        for (int q = 0; q < RW; ++q) ui[q] = row + q < sp.end ? __ldcg(up + row + q) : (LOGF ? T(-INFINITY) : T(0));
+        // sixteen loads in flight at once (vectors beyond the row read its
+        // first one and are not stored)
+        T x[KB][RW][W];
 #pragma unroll
         for (int k = 0; k < KB; ++k) {
           const int j = (k0 + k) * R.gt + R.tg < nv ? (k0 + k) * R.gt + R.tg : 0;
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
+          for (int q = 0; q < RW; ++q)
             unpack(ld_stream(reinterpret_cast<const typename Vec<T>::type*>(Mp + (int64_t)min(row + q, sp.end - 1) * ldm) + j), x[k][q]);
         }
 #pragma unroll
@@ -412,19 +421,19 @@ __device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_,
           for (int y = 0; y < W; ++y) {
             if (LOGF) {
               // rows beyond the share have u = -inf
-              T t[4], top = mx[k][y];
+              T t[RW], top = mx[k][y];
 #pragma unroll
-              for (int q = 0; q < 4; ++q) { t[q] = row + q < sp.end ? fma(x[k][q][y], c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
+              for (int q = 0; q < RW; ++q) { t[q] = row + q < sp.end ? fma(x[k][q][y], c, ui[q]) : T(-INFINITY); top = fmax(top, t[q]); }
               // (an empty column so far: the sums stay zero)
               const T ref = top == -INFINITY ? T(0) : top;
               T sum = s[k][y] * ex2(mx[k][y] - ref);
 #pragma unroll
-              for (int q = 0; q < 4; ++q) sum += ex2(t[q] - ref);
+              for (int q = 0; q < RW; ++q) sum += ex2(t[q] - ref);
               s[k][y] = sum;
               mx[k][y] = top;
             } else {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) s[k][y] = fma(ex2(x[k][q][y] * c), ui[q], s[k][y]);
+              for (int q = 0; q < RW; ++q) s[k][y] = fma(ex2(x[k][q][y] * c), ui[q], s[k][y]);
             }
           }
         }
@@ -432,7 +441,7 @@ __device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_,
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
         const int j = (k0 + k) * R.gt + R.tg;
-        if (j < nv) {
+        if (j < nv && on) {
 #pragma unroll
           for (int y = 0; y < W; ++y) {
             if (LOGF) {
@@ -452,8 +461,11 @@ __device__ __noinline__ void mf_colpass(const MultiArgs<T>& A_, const FuRow& R_,
 // are added in worker order, a block per warp, or (`split`) the 8 warps of a
 // CTA share a block's slots (their sums in warp order).  The place of the
 // first block (looked up once until the shares change) is in `P`.
-// fin(p, cj, b, v, mx, s) finishes column cj (packed like b) of problem p.
-struct MfPlace { int64_t lo, hi, base, co, b0, b1; int k, p, m, w0, w1, split; };
+// fin(p, cj, b, v, mx, s, lim) finishes column cj (packed like b) of problem
+// p.  `marks`: only the columns whose mark is NaN, of problems in A.fbad.
+// Column sums below 2^lim may have lost bits to underflow (as in fused_impl.cuh,
+// a part of the problem's mass).
+struct MfPlace { int64_t lo, hi, base, co, b0, b1; int k, p, m, w0, w1, split, lim; };
 
 // A block costs a warp about 1.0 us for its place, v and b and 0.6 us per eight
 // slots, all of it latency; split, the CTA 1.3 us and an eighth of the slots.
@@ -472,6 +484,7 @@ __device__ __forceinline__ void mf_place(const MultiArgs<T>& A, MfPlace& P, int6
   P.p = __ldcg(A.active + P.k);
   P.m = A.cols[P.p];
   P.co = A.c_off[P.p];
+  P.lim = __ldcg(A.flim + P.p);
   const int64_t pos = __ldcg(A.urow_pre + P.k), total = __ldcg(A.urow_pre + nact);
   P.w0 = mf_worker(total, na, pos);
   const int rb = 16 / A.fNK;  // the last batch's place
@@ -490,26 +503,26 @@ __device__ __noinline__ MfPlace mf_first_place(const MultiArgs<T>& A, int na, in
   return P;
 }
 template <typename T, bool PAIRS, typename Fin>
-__device__ __forceinline__ void mf_merge(const MultiArgs<T>& A, const MfPlace& first, int na, int nact, T (*scr)[2][32], bool flagged,
+__device__ __forceinline__ void mf_merge(const MultiArgs<T>& A, const MfPlace& first, int na, int nact, T (*scr)[2][32], const T* marks,
                                          const T* vcur, Fin&& fin) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   MfPlace P = first;
   const bool split = P.split;
   for (int64_t blk = P.b0; blk < P.b1; ++blk) {
     mf_place(A, P, blk, na, nact);
-    if (flagged && __ldcg(A.fbad + P.p) == 0) continue;
+    if (marks && __ldcg(A.fbad + P.p) == 0) continue;
     const int j = (int)(blk - P.lo) * 32 + lane;
     T mx = -INFINITY, s = 0, bj = 0, vo = 0;
     const int step = split ? FU_WARPS : 1;
-    if (j < P.m) {
+    bool on = j < P.m;
+    if (marks && on) on = isnan(__ldcg(marks + P.co + j));
+    if (on) {
       bj = A.b[P.co + j];
       vo = __ldcg(vcur + P.co + j);
       int w = P.w0 + (split ? warp : 0);
       if (PAIRS) {
-        for (; w <= P.w1; w += step) {
-          const T* q = A.fpairs + 2 * (P.base + (int64_t)w * A.fmm + j);
-          lse_merge(mx, s, __ldcg(q), __ldcg(q + 1));
-        }
+        if (w <= P.w1)
+          lse_merge_strided(mx, s, A.fpairs + 2 * (P.base + (int64_t)w * A.fmm + j), 2 * (int64_t)step * A.fmm, (P.w1 - w) / step + 1);
       } else {
         const T* q = A.fpart + P.base + j;
         for (; w <= P.w1; w += 8 * step) {
@@ -533,7 +546,7 @@ __device__ __forceinline__ void mf_merge(const MultiArgs<T>& A, const MfPlace& f
       }
       __syncthreads();
     }
-    if (j < P.m && (!split || warp == 0)) fin(P.p, P.co + j, bj, vo, mx, s);
+    if (on && (!split || warp == 0)) fin(P.p, P.co + j, bj, vo, mx, s, P.lim);
   }
 }
 
@@ -816,7 +829,14 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
       if (LOGF) A.u[ri] = A.warm_u ? A.warm_u[ri] * L2E : T(0);
       else A.u[ri] = A.warm_u ? exp(A.warm_u[ri]) : T(1);
     }
+    double mass = 0.0;
+    if (LOGF) {
+      for (int i = threadIdx.x; i < A.rows[p]; i += MT_THREADS) mass += widen(A.a[A.r_off[p] + i]);
+      mass = block_sum_fixed(mass);
+    }
     if (threadIdx.x == 0) {
+      const int e = mass > 0.0 && isfinite(mass) ? ilogb(mass) + 1 : 0;
+      A.flim[p] = sizeof(T) == 8 ? max(e - 985, -1000) : max(e - 70, -100);
       leaving[p] = 0;
       A.fbad[p] = 0;
       A.err2[p] = 0.0;
@@ -847,9 +867,9 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
   look_up();
 
   // the column update of the initial u: the first v
-  if (wid < na) mf_colpass<T, LOGF>(A, R, wid, na, nact, false);
+  if (wid < na) mf_colpass<T, LOGF, false>(A, R, wid, na, nact, (const T*)nullptr);
   if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) return;
-  mf_merge<T, LOGF>(A, s_place[R.warp], na, nact, scr, false, vcur, [&](int, int64_t cj, T bj, T, T mx, T s) {
+  mf_merge<T, LOGF>(A, s_place[R.warp], na, nact, scr, (const T*)nullptr, vcur, [&](int, int64_t cj, T bj, T, T mx, T s, int) {
     vcur[cj] = LOGF ? lg2(bj) - lse_value(mx, s) : bj / s;
   });
   if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) return;
@@ -861,7 +881,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
     const bool check = ii % A.period == 0, last = ii + 1 == A.max_iter;
     int32_t* any_bad = A.leave_cnt + 2;
     if (blockIdx.x == 0 && threadIdx.x == 0) any_bad[(ii + 1) & 1] = 0;  // last read an iteration ago
-    mf_merge<T, false>(A, s_place[R.warp], na, nact, scr, false, vcur, [&](int p, int64_t cj, T bj, T vo, T, T s) {
+    mf_merge<T, false>(A, s_place[R.warp], na, nact, scr, (const T*)nullptr, vcur, [&](int p, int64_t cj, T bj, T vo, T, T s, int lim) {
       if (check) {
         // column marginal of (u, v) of iteration ii, in the column's own slot
         const double cs = widen(LOGF ? s : vo * s) - widen(bj);
@@ -871,7 +891,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
       if (LOGF) {
         vn = bj == T(0) ? T(-INFINITY) : vo + lg2(bj / s);
         if (A.relax) vn = fma(A.omega, vn - vo, vo);
-        if (bj != T(0) && !(s >= T(8.470329472543003e-22))) {  // 2^-70: terms may have underflowed
+        if (bj != T(0) && !fu_at_least(s, exp2_of<T>(lim))) {  // terms may have underflowed
+          vn = T(NAN);
           A.fbad[p] = 1;
           any_bad[ii & 1] = 1;
         }
@@ -946,10 +967,10 @@ __global__ void __launch_bounds__(MT_THREADS, 1) multi_fused_kernel(const __grid
       }
     }
     if (bad) {
-      // column sums too small to trust: those problems' column update with running maxima
-      if (wid < na) mf_colpass<T, LOGF>(A, R, wid, na, nact, true);
+      // column sums too small to trust (NaN in v): their update with running maxima
+      if (wid < na) mf_colpass<T, LOGF, true>(A, R, wid, na, nact, vnxt);
       if (!fu_barrier(A.bar, gen, abort_flag, A.timeout_ns)) { ok = false; break; }
-      mf_merge<T, true>(A, s_place[R.warp], na, nact, scr, true, vcur, [&](int, int64_t cj, T bj, T vo, T mx, T s) {
+      mf_merge<T, true>(A, s_place[R.warp], na, nact, scr, vnxt, vcur, [&](int, int64_t cj, T bj, T vo, T mx, T s, int) {
         const T vn = lg2(bj) - lse_value(mx, s);
         vnxt[cj] = A.relax ? fma(A.omega, vn - vo, vo) : vn;
       });
