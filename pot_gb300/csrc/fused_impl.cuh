@@ -49,8 +49,11 @@
 // Range of the shortcut.  Log form: the shift of row i is its previous
 // potential less log a_i, so e_ij is the row's previous plan entry over a_i
 // and s_i is near one; rows whose s_i leaves [2^-30, 2^30] (first iterations
-// from a far start, zero weights, non-finite input) take the running-maximum
-// form on the same entries.  What can be lost in a column sum are entries
+// from a far start, non-finite input) take the running-maximum form on the
+// same entries.  Rows of no weight have a shift of -inf: their entries are
+// zeros, their potential -inf.  (With a shift of u - log a they were not
+// numbers and went through the running maxima with the rows of their batch:
+// half of the rows empty, 8192^2 float32 98 us per iteration, now 59.)  What can be lost in a column sum are entries
 // below 2^-126 (2^-1074 in float64) times the row factors a_i / s_i, together
 // 2^-96 (2^-1044) of the mass.  A column sum that is not 2^26 (2^59) times
 // that is recomputed in that iteration with running maxima: one more pass over
@@ -244,7 +247,11 @@ __device__ __forceinline__ void fu_publish_cols(const FusedArgs<T>& A, const FuR
 // the CTA's column sums.  q0, q1, q2: scalars of the group's rows, lane l of
 // a warp holding row 32 k + l (reloaded every 32 rows unless `held`).
 // ---------------------------------------------------------------------------
-template <typename T> struct FuHeld { T q0, q1, q2; };
+template <typename T> struct FuHeld {
+  T q0, q1, q2;
+  // log form (u, log2 a, a): a row of no weight adds nothing to any column
+  __device__ __forceinline__ T shift() const { return q2 == T(0) ? T(-INFINITY) : q0 - q1; }
+};
 
 template <typename T, int MODE>
 __device__ __forceinline__ void fu_fetch(const FusedArgs<T>& A, int row, int end, const T* ucur, FuHeld<T>& H) {
@@ -286,7 +293,9 @@ __device__ __forceinline__ void fu_rows(const FusedArgs<T>& A, const FuRow& R, T
       for (int q = LPR / 2; q > 0; q >>= 1) t += __shfl_xor_sync(0xffffffffu, t, q);
     }
     if (MODE == FU_LOG) {
-      un = p0 - lg2(t);
+      // (a row of no weight: its entries are zeros, its sum is not looked at)
+      if (p2 == T(0)) t = T(1);
+      un = p2 == T(0) ? T(-INFINITY) : p0 - lg2(t);
       r = p2 / t;
     } else if (MODE == FU_SCAL) {
       r = un = T(1) / (p1 * t);
@@ -405,7 +414,7 @@ __device__ __forceinline__ int fu_pass(const FusedArgs<T>& A, const FuRow& R_, c
 #pragma unroll
       for (int q = 0; q < decltype(nq)::value; ++q) {
         const uint32_t xq = xa + min(q, nr - 1) * pitch;
-        const typename V::S h = V::all(MODE == FU_LOG ? __shfl_sync(0xffffffffu, H.q0 - H.q1, at + q) : T(0));
+        const typename V::S h = V::all(MODE == FU_LOG ? __shfl_sync(0xffffffffu, H.shift(), at + q) : T(0));
         V t = V::zero();
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
@@ -418,7 +427,7 @@ __device__ __forceinline__ int fu_pass(const FusedArgs<T>& A, const FuRow& R_, c
     };
     if (!RES) {
       // the two halves of the row, each as it lands
-      const typename V::S h = V::all(MODE == FU_LOG ? __shfl_sync(0xffffffffu, H.q0 - H.q1, at) : T(0));
+      const typename V::S h = V::all(MODE == FU_LOG ? __shfl_sync(0xffffffffu, H.shift(), at) : T(0));
       V t = V::zero();
 #pragma unroll
       for (int half = 0; half < 2; ++half) {

@@ -273,7 +273,7 @@ __device__ __forceinline__ bool mf_pass(const MultiArgs<T>& A, const FuRow& R, c
 #pragma unroll
         for (int q = 0; q < RB; ++q) {
           const uint32_t xq = xb + (uint32_t)min(q, nr - 1) * pitch;
-          const typename V::S h = V::all(LOGF ? __shfl_sync(0xffffffffu, q0 - q1, at + q) : T(0));
+          const typename V::S h = V::all(LOGF ? __shfl_sync(0xffffffffu, q2 == T(0) ? T(-INFINITY) : q0 - q1, at + q) : T(0));
           V t4 = V::zero();
 #pragma unroll
           for (int k = 0; k < KV; ++k) {
@@ -298,9 +298,13 @@ __device__ __forceinline__ bool mf_pass(const MultiArgs<T>& A, const FuRow& R, c
       const T uo = __shfl_sync(0xffffffffu, q0, at + myrow), ai = __shfl_sync(0xffffffffu, q2, at + myrow);
       T un, r;
       if constexpr (LOGF) {
+        // a row of no weight adds nothing to any column
+        const bool none = ai == T(0);
+        if (none) t = T(1);
         un = uo - lg2(t);
         r = ai / t;
         if (A.relax) { un = fma(A.omega, un - uo, uo); r = ai * ex2(un - uo); }
+        if (none) { un = T(-INFINITY); r = T(0); }
         if (!__all_sync(0xffffffffu, myrow >= nr || fu_near_one(t))) {
           // running maxima, on the same entries (the slot is not refilled yet)
           T mx[RB];
@@ -330,6 +334,7 @@ __device__ __forceinline__ bool mf_pass(const MultiArgs<T>& A, const FuRow& R, c
           un = la - lse_value(mg, t);
           r = ai / t;
           if (A.relax) { un = fma(A.omega, un - uo, uo); r = ex2(un + mg); }
+          if (none) { un = T(-INFINITY); r = T(0); }
         }
       } else {
         un = ai / t;

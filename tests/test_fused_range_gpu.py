@@ -135,3 +135,19 @@ def test_gradient_with_more_ctas_than_columns(cuda):
         got = implicit_grads(P, M, a, b, 0.5)
     for x, y in zip(got, ref):
         assert float((x.cpu() - y).abs().max()) <= 1e-8 * max(1e-3, float(y.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("n,m", [(1024, 1024), (3000, 4100), (2300, 2500)])
+def test_half_of_the_bins_empty(cuda, n, m, dtype):
+    """Empty rows beside full ones in every batch of rows; a forbidden entry
+    in an empty row and a row forbidden but for one entry."""
+    a, b = torch.ones(n, dtype=F64, device=cuda), torch.ones(m, dtype=F64, device=cuda)
+    a[::2], b[1::3] = 0.0, 0.0
+    a[17:40] = 0.0
+    a, b = (a / a.sum()).to(dtype), (b / b.sum()).to(dtype)
+    M = _line(n, m, dtype, cuda)
+    M[4, :100] = math.inf
+    M[5, :] = math.inf
+    M[5, 9] = 0.5
+    _check(M, a, b, 0.02, 20)
