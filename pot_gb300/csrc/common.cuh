@@ -137,6 +137,42 @@ __device__ __forceinline__ double widen(float x) {
 }
 __device__ __forceinline__ double widen(double x) { return x; }
 
+// Running sums that lose nothing next to float64 ones.  float: two lanes of
+// packed fp32 operations (even and odd terms), each with the rounding errors of
+// its additions in a second float (D. E. Knuth, TAOCP 2, 4.2.2): seven packed
+// operations for two terms, where widening and an FP64 addition issue at two
+// lanes per clock and SM; double: a plain sum.
+template <typename T> struct Sum2;
+template <> struct Sum2<float> {
+  uint64_t hi = 0ull, lo = 0ull;
+  __device__ __forceinline__ void add_(uint64_t x) {
+    const uint64_t m1 = pack2(-1.f, -1.f), s = add2(hi, x), b = fma2(hi, m1, s);
+    lo = add2(lo, add2(fma2(fma2(b, m1, s), m1, hi), fma2(b, m1, x)));
+    hi = s;
+  }
+  __device__ __forceinline__ void add(float x, float y) { add_(pack2(x, y)); }
+  // + x0 y0, x1 y1, the products' roundings kept too
+  __device__ __forceinline__ void fma_(float x0, float y0, float x1, float y1) {
+    const uint64_t x = pack2(x0, x1), y = pack2(y0, y1), p = mul2(x, y);
+    lo = add2(lo, fma2(x, y, fma2(p, pack2(-1.f, -1.f), 0ull)));
+    add_(p);
+  }
+  // (an infinite sum has no error term)
+  __device__ __forceinline__ double value() const {
+    float h0, h1, l0, l1;
+    unpack2(hi, h0, h1);
+    unpack2(lo, l0, l1);
+    const double h = widen(h0) + widen(h1);
+    return isfinite(h0) && isfinite(h1) ? h + widen(l0 + l1) : h;
+  }
+};
+template <> struct Sum2<double> {
+  double hi = 0.0;
+  __device__ __forceinline__ void add(double x, double y) { hi += x; hi += y; }
+  __device__ __forceinline__ void fma_(double x0, double y0, double x1, double y1) { hi = fma(x1, y1, fma(x0, y0, hi)); }
+  __device__ __forceinline__ double value() const { return hi; }
+};
+
 template <typename T> struct Vec;
 template <> struct Vec<float> { using type = float4; static constexpr int N = 4; };
 template <> struct Vec<double> { using type = double2; static constexpr int N = 2; };
