@@ -258,15 +258,19 @@ __global__ void __launch_bounds__(256) transpose_batched_kernel(const T* __restr
 // Bound by the read of M and the write of T.  A CTA takes 1024 columns (fewer
 // for narrow problems, with more rows side by side) of a range of rows; a
 // thread keeps what belongs to its 16-byte vector of columns in registers and
-// streams rows.  float: the logarithm of an entry is the exponent that the
-// entry is computed from, clamped at log 1e-16 (off by at most 0.7e-16 per
-// entry of the sum where T is that small), so there is no logarithm per entry;
-// the sums run in float over up to eight rows of a vector (32 entries) and in
-// fp64 beyond, as an fp64 addition issues at two lanes per clock.  double:
-// fp64 throughout.  128 problems of 512 x 512 float: 290 us with a row per
-// CTA, scalar loads, a logarithm and three fp64 additions per pair of entries;
-// 68 us with hardware conversions to fp64 and a division per warp, now 59.
+// streams rows.  The sums keep their rounding errors (Sum2) over up to eight
+// rows of a vector and run in fp64 beyond, as an fp64 addition issues at two
+// lanes per clock.  float, log form: the logarithm of an entry above 2e-9 is the
+// exponent that the entry is computed from (there log(p + 1e-16) is log p in
+// float32, and the exponent has its one rounding), that of a smaller one the
+// hardware's.  128 problems of 512 x 512 float, a
+// call: 293 us with a row per CTA, scalar loads, a logarithm and three fp64
+// additions per pair of entries, 108 now.  (76 with plain float sums of 32
+// entries, which drop what is 2^-24 of their largest.)
 constexpr int PL_ROWS = 8;   // rows in flight, and between fp64 additions
+// log2 in the hardware's approximation (relative error 2^-22 below 1/2)
+__device__ __forceinline__ float fast_lg2(float x) { return __log2f(x); }
+__device__ __forceinline__ double fast_lg2(double x) { return lg2(x); }
 template <typename T, int METHOD>
 __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int row_tiles) {
   using V = typename Vec<T>::type;
@@ -290,22 +294,20 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
   if (threadIdx.x == 0) s_c = (T)(-OTG_LOG2E / t.reg[p]);
   __syncthreads();
   const T c = s_c;
-  const T L2E = T(OTG_LOG2E), LN2 = T(OTG_LN2), L16 = T(-36.841361487904734);  // log 1e-16
-  constexpr bool FAST = sizeof(T) == 4;
+  const T L2E = T(OTG_LOG2E), LN2 = T(OTG_LN2);
+  const bool fast = sizeof(T) == 4 && METHOD == OTG_METHOD_LOG && !t.kl;
   double lin = 0, reg_term = 0, mass = 0;
   for (int unit = blockIdx.x; unit < row_tiles * chunks; unit += gridDim.x) {
     const int jv = (unit % chunks) * cx + tx, tile = unit / chunks;
     const int i0 = (int)((int64_t)n * tile / row_tiles), i1 = (int)((int64_t)n * (tile + 1) / row_tiles);
     if (jv >= nv) continue;
     const int j0 = jv * W;
-    T vj[W], lv[W], bj[W];
+    T vj[W], bj[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       const bool in = j0 + w < m;
       vj[w] = in ? v[j0 + w] : T(0);
       bj[w] = in ? b[j0 + w] : T(1);
-      // float: log2 of what the column brings to the entry, less log2 b (KL form)
-      if (FAST) lv[w] = (METHOD == OTG_METHOD_LOG ? T(0) : lg2(vj[w])) - (t.kl ? lg2(bj[w]) : T(0));
     }
     for (int ib = i0 + ty; ib < i1; ib += PL_ROWS * ry) {
       // the loads of eight rows in flight
@@ -323,32 +325,27 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
         us[q] = u[i];
         as[q] = t.kl ? a[i] : T(1);
       }
-      T lr = 0, rr = 0, mr = 0;
+      Sum2<T> lr, rr, mr;
 #pragma unroll
       for (int q = 0; q < PL_ROWS; ++q) {
         const int i = ib + q * ry;
         if (i < i1) {
           const T ui = us[q], ai = as[q];
-          T lu = 0;
-          if (FAST) lu = (METHOD == OTG_METHOD_LOG ? T(0) : lg2(ui)) - (t.kl ? lg2(ai) : T(0));
-          T pr[W];
+          T pr[W], lg[W];
 #pragma unroll
           for (int w = 0; w < W; ++w) {
-            T e;  // log2 of the entry without the scalings (scaling form), with the potentials (log form)
+            T e = 0;
             if (METHOD == OTG_METHOD_LOG) { e = fma(x[q][w], c, (ui + vj[w]) * L2E); pr[w] = ex2(e); }
-            else { e = x[q][w] * c; pr[w] = ui * ex2(e) * vj[w]; }
-            if (j0 + w < m) {
-              lr = fma(x[q][w], pr[w], lr);
-              mr += pr[w];
-              if (FAST) {
-                const T lg = (e + lu + lv[w]) * LN2;
-                rr = fma(pr[w], lg < L16 ? L16 : lg, rr);  // (a NaN stays one)
-              } else if (t.kl) {
-                rr = fma(pr[w], log(pr[w] / (ai * bj[w]) + T(1e-16)), rr);
-              } else {
-                rr = fma(pr[w], log(pr[w] + T(1e-16)), rr);
-              }
-            }
+            else pr[w] = ui * ex2(x[q][w] * c) * vj[w];
+            if (fast) lg[w] = (pr[w] > T(2e-9) ? e : fast_lg2(pr[w] + T(1e-16))) * LN2;
+            else lg[w] = log((t.kl ? pr[w] / (ai * bj[w]) : pr[w]) + T(1e-16));
+            if (j0 + w >= m) x[q][w] = pr[w] = lg[w] = T(0);
+          }
+#pragma unroll
+          for (int w = 0; w < W; w += 2) {
+            lr.fma_(x[q][w], pr[w], x[q][w + 1], pr[w + 1]);
+            mr.add(pr[w], pr[w + 1]);
+            rr.fma_(pr[w], lg[w], pr[w + 1], lg[w + 1]);
           }
           if (P) {
             V o;
@@ -366,7 +363,7 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
           }
         }
       }
-      lin += widen(lr); mass += widen(mr); reg_term += widen(rr);
+      lin += lr.value(); mass += mr.value(); reg_term += rr.value();
     }
   }
   __shared__ double red[3][8];
