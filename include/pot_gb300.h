@@ -496,7 +496,7 @@ int otg_batched_sqdist(const OtgCostTable* t, int32_t max_rows, cudaStream_t str
  * potentials; knopp: scalings).  out_vals[3p] = sum M*T, out_vals[3p+1] =
  * sum T log(T + 1e-16) (kl = 0) or sum T log(T/(a b^T) + 1e-16) (kl = 1),
  * out_vals[3p+2] = sum T, all fp64.  P may be NULL (values only); it uses
- * M's layout.  Replaces ot/batch/_linear.py:326-345 and _utils.py:4-21. */
+ * M's layout (columns cols[p] .. ldm[p] - 1 are neither read nor written).  Replaces ot/batch/_linear.py:326-345 and _utils.py:4-21. */
 typedef struct OtgPlanTable {
   int32_t dtype, method, nprob, kl;
   const void* M;

@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
     const int i0 = (int)((int64_t)n * tile / row_tiles), i1 = (int)((int64_t)n * (tile + 1) / row_tiles);
     if (jv >= nv) continue;
     const int j0 = jv * W;
+    const bool whole = vec && j0 + W <= m;  // what lies behind column m is the caller's
     T vj[W], bj[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) {
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
       for (int q = 0; q < PL_ROWS; ++q) {
         const int i = min(ib + q * ry, i1 - 1);
         const T* mp = M + (int64_t)i * ldm + j0;
-        if (vec) {
+        if (whole) {
           unpack(ld_stream(reinterpret_cast<const V*>(mp)), x[q]);
         } else {
 #pragma unroll
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(256) batched_plan_kernel(OtgPlanTable t, int r
 #pragma unroll
             for (int w = 0; w < W; ++w) op[w] = pr[w];
             T* dst = P + (int64_t)i * ldm + j0;
-            if (vec) {
+            if (whole) {
               *reinterpret_cast<V*>(dst) = o;
             } else {
 #pragma unroll
