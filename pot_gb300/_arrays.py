@@ -17,8 +17,9 @@ def upload(device, arrays):
     call).  A capturing stream refuses it, as it does the pageable copy: a
     replay would read the host buffer after it went back to its pool."""
     device = torch.device(device)
+    arrays = [np.asarray(x) for x in arrays]
     if device.type != "cuda" or torch.cuda.is_current_stream_capturing():
-        return [torch.from_numpy(np.ascontiguousarray(x)).to(device) for x in arrays]
+        return [torch.from_numpy(np.ascontiguousarray(x)).view(x.shape).to(device) for x in arrays]
     offs, total = [], 0
     for x in arrays:
         offs.append(total)
@@ -28,10 +29,8 @@ def upload(device, arrays):
     for x, o in zip(arrays, offs):
         view[o:o + x.nbytes] = np.ascontiguousarray(x).view(np.uint8).reshape(-1)
     dev = host.to(device, non_blocking=True)
-    return [dev[o:o + x.nbytes].view(_TORCH[x.dtype.kind, x.dtype.itemsize]) for x, o in zip(arrays, offs)]
-
-
-_TORCH = {("i", 4): torch.int32, ("i", 8): torch.int64, ("f", 4): torch.float32, ("f", 8): torch.float64}
+    return [dev[o:o + x.nbytes].view(torch.from_numpy(np.empty(0, x.dtype)).dtype).view(x.shape)
+            for x, o in zip(arrays, offs)]
 
 
 class Boundary:
