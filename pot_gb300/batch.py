@@ -59,7 +59,11 @@ class RaggedLayout:
         nsr_max = np.maximum(1, np.minimum(64, (rows + 15) // 16)).astype(np.int32)
         partials = nsr_max.astype(np.int64) * cols
         pc_off = np.concatenate([[0], np.cumsum(partials)[:-1]]).astype(np.int64)
-        self.max_ldm, self.chunk_partials = int(ldm.max()), int(partials.sum())
+        # (the one-read kernel wants a row and a column of every problem)
+        self.max_ldm = int(ldm.max()) if self.B and self.total_m else 0
+        if self.B and min(rows.min(), cols.min()) == 0:
+            self.max_ldm = 0
+        self.chunk_partials = int(partials.sum())
         self.nsr_max_np = nsr_max
         i32 = np.int32
         (self.m_off, self.r_off, self.c_off, self.pc_off, self.rows, self.cols, self.ldm, self.order, self.nsr_max) = upload(
