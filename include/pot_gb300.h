@@ -108,8 +108,14 @@ typedef struct OtgDenseProblem {
   int64_t ldk;
 } OtgDenseProblem;
 
-/* Workspace size for otg_sinkhorn_dense (device bytes, 256-byte aligned). */
+/* Workspace size for otg_sinkhorn_dense (device bytes, 256-byte aligned).
+ * _least: what it runs with at all (and all that the stabilised form uses);
+ * between the two sizes the solver takes two passes over the cost per
+ * iteration instead of one.  The difference can be as large as the cost: costs
+ * that do not stay on chip and whose rows are not whole 16-byte vectors are
+ * copied into padded rows. */
 size_t otg_dense_workspace_bytes(int dtype, int64_t n, int64_t m, int hist_cap, int grid);
+size_t otg_dense_workspace_least(int dtype, int64_t n, int64_t m, int hist_cap, int grid);
 /* Byte offset inside the workspace of the result block:
  *   double err_hist[hist_cap]; then int32 info[8] 256-byte aligned after it
  *   (info[0] status, info[1] niter = last loop index, info[2] number of
@@ -120,8 +126,9 @@ int otg_sinkhorn_dense(const OtgDenseProblem* p, void* workspace, cudaStream_t s
 
 /* Whether a stored Gibbs kernel (OtgDenseProblem::K, otg_gibbs_kernel) would
  * save work in this solve: 1 for a float64 scaling form whose passes read the
- * cost from memory, 0 when the solver keeps the problem on chip (it then
- * exponentiates every entry once by itself) and for every other form. */
+ * cost from memory, 0 when the solver exponentiates every entry once by itself
+ * (the problem stays on chip, or is copied into padded rows) and for every
+ * other form.  workspace_bytes: what the solve will be given (0: enough). */
 int otg_dense_wants_gibbs(const OtgDenseProblem* p);
 
 /* Plan and/or loss from potentials: P = exp(-M/reg + u + v) (log form) or

@@ -102,6 +102,7 @@ class OtgOnlineProblem(ctypes.Structure):
 SIGNATURES = {
     "otg_abi_layout": (ctypes.c_int, [ctypes.c_char_p, ctypes.POINTER(c_i64), c_i32]),
     "otg_dense_workspace_bytes": (c_sz, [ctypes.c_int, c_i64, c_i64, ctypes.c_int, ctypes.c_int]),
+    "otg_dense_workspace_least": (c_sz, [ctypes.c_int, c_i64, c_i64, ctypes.c_int, ctypes.c_int]),
     "otg_dense_info_offset": (c_sz, [ctypes.c_int, c_i64, c_i64, ctypes.c_int, ctypes.c_int]),
     "otg_sinkhorn_dense": (ctypes.c_int, [ctypes.POINTER(OtgDenseProblem), c_vp, c_vp]),
     "otg_dense_wants_gibbs": (ctypes.c_int, [ctypes.POINTER(OtgDenseProblem)]),

@@ -80,8 +80,17 @@ def solve_dense(M, a, b, reg, method, max_iter, stop_thr, warm_u=None, warm_v=No
         grid = default_grid(n, m, M.dtype) if method == _lib.OTG_METHOD_STAB else 0
     dt = _lib.dtype_code(M.dtype)
     cap = max(2, max_iter // check_period + 2)
-    wsb = lib.otg_dense_workspace_bytes(dt, n, m, cap, grid)
-    ws = torch.empty(wsb, dtype=torch.uint8, device=M.device)
+    # the stabilised form runs the two-pass kernel, and so does a solve without
+    # room for what the one-read kernel wants (up to a padded copy of the cost)
+    least = lib.otg_dense_workspace_least(dt, n, m, cap, grid)
+    wsb = least if method == _lib.OTG_METHOD_STAB else lib.otg_dense_workspace_bytes(dt, n, m, cap, grid)
+    try:
+        ws = torch.empty(wsb, dtype=torch.uint8, device=M.device)
+    except torch.cuda.OutOfMemoryError:
+        if wsb == least:
+            raise
+        wsb = least
+        ws = torch.empty(wsb, dtype=torch.uint8, device=M.device)
     out_u = torch.empty(n, dtype=M.dtype, device=M.device)
     out_v = torch.empty(m, dtype=M.dtype, device=M.device)
     p = _lib.OtgDenseProblem(
@@ -113,6 +122,7 @@ def solve_dense(M, a, b, reg, method, max_iter, stop_thr, warm_u=None, warm_v=No
     r.hist = None
     if read_back:
         read_result(r)
+        _release(r)
     return r
 
 
@@ -135,6 +145,17 @@ def read_result(r):
     if r.status == _lib.STATUS_ABORTED:
         raise RuntimeError("pot_gb300: a device-side wait timed out; the solve was abandoned")
     return r
+
+
+# a workspace with a copy of the cost is not kept for the error history in it
+_KEEP_BYTES = 64 << 20
+
+
+def _release(r):
+    """Gives a large workspace back once its results are read."""
+    if r.workspace.numel() >= _KEEP_BYTES:
+        r.hist = r.hist.clone()
+        r.workspace = None
 
 
 def _errs_as(bd, errs, like, r=None):
@@ -205,17 +226,18 @@ def _warm(bd, warmstart, dtype, n=None, m=None):
 
 def _run_single(bd, a, b, M, reg, method, numItermax, stopThr, verbose, warn, warmstart, want_plan):
     wu, wv = _warm(bd, warmstart, M.dtype, M.shape[0], M.shape[1])
+    # (the plan first: the workspace can do with less memory, the plan cannot)
+    P = torch.empty_like(M) if want_plan else None
     r = solve_dense(M, a, b, reg, method, numItermax, stopThr, wu, wv, read_back=False)
-    P = None
     lib = _lib.load()
     if want_plan:
         # launched behind the solve, before the host waits for its result
-        P = torch.empty_like(M)
         _lib.check(lib.otg_dense_plan(_lib.dtype_code(M.dtype), method, ctypes.c_void_p(M.data_ptr()),
                                       M.shape[0], M.shape[1], M.stride(0), _lib.ptr(r.u), _lib.ptr(r.v),
                                       float(reg), _lib.ptr(P), P.stride(0), None,
                                       _lib.stream_handle(M.device)), "otg_dense_plan")
     read_result(r)
+    _release(r)
     if r.status == _lib.STATUS_NUMERICAL:
         warnings.warn("Warning: numerical errors at iteration %d" % r.niter)
     if verbose:

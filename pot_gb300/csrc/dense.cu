@@ -897,6 +897,11 @@ size_t otg_dense_workspace_bytes(int dtype, int64_t n, int64_t m, int hist_cap, 
   return make_layout<float>(n, m, hist_cap, grid).total_fused;
 }
 
+size_t otg_dense_workspace_least(int dtype, int64_t n, int64_t m, int hist_cap, int grid) {
+  if (dtype == OTG_F64) return make_layout<double>(n, m, hist_cap, grid).total;
+  return make_layout<float>(n, m, hist_cap, grid).total;
+}
+
 size_t otg_dense_info_offset(int dtype, int64_t n, int64_t m, int hist_cap, int grid) {
   if (dtype == OTG_F64) return make_layout<double>(n, m, hist_cap, grid).off_hist;
   return make_layout<float>(n, m, hist_cap, grid).off_hist;
@@ -912,7 +917,9 @@ int otg_sinkhorn_dense(const OtgDenseProblem* p, void* workspace, cudaStream_t s
 
 int otg_dense_wants_gibbs(const OtgDenseProblem* p) {
   if (!p || p->method != OTG_METHOD_KNOPP || p->dtype != OTG_F64) return 0;
-  return fused_resident(p) ? 0 : 1;
+  const Layout L = make_layout<double>(p->n, p->m, p->hist_cap, p->grid);
+  if (L.total_fused == L.total || (p->workspace_bytes > 0 && p->workspace_bytes < L.total_fused)) return 1;
+  return fused_holds_gibbs(p) ? 0 : 1;
 }
 
 int otg_dense_plan(int dtype, int method, const void* M, int64_t n, int64_t m, int64_t ldm,

@@ -26,16 +26,17 @@ size_t fused_bytes(int dtype, int64_t n, int64_t m, int requested_grid);
 // alignment); returns OTG_ERR_UNSUPPORTED when it does not.
 int fused_launch(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st);
 
-// Whether that launch would keep the cost in shared memory for the whole solve.
-bool fused_resident(const OtgDenseProblem* p);
+// Whether that launch (scaling form) makes K = exp(-M/reg) by itself once: in
+// shared memory, or with the copy into whole-vector rows.
+bool fused_holds_gibbs(const OtgDenseProblem* p);
 
 // Per-type parts (fused_f32.cu, fused_f64.cu).
 int fused_launch_f32(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st);
 int fused_launch_f64(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st);
 size_t fused_bytes_f32(int64_t n, int64_t m, int requested_grid);
 size_t fused_bytes_f64(int64_t n, int64_t m, int requested_grid);
-bool fused_resident_f32(const OtgDenseProblem* p);
-bool fused_resident_f64(const OtgDenseProblem* p);
+bool fused_holds_gibbs_f32(const OtgDenseProblem* p);
+bool fused_holds_gibbs_f64(const OtgDenseProblem* p);
 
 inline size_t fused_bytes(int dtype, int64_t n, int64_t m, int requested_grid) {
   return dtype == OTG_F64 ? fused_bytes_f64(n, m, requested_grid) : fused_bytes_f32(n, m, requested_grid);
@@ -43,8 +44,8 @@ inline size_t fused_bytes(int dtype, int64_t n, int64_t m, int requested_grid) {
 inline int fused_launch(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st) {
   return p->dtype == OTG_F64 ? fused_launch_f64(p, fs, st) : fused_launch_f32(p, fs, st);
 }
-inline bool fused_resident(const OtgDenseProblem* p) {
-  return p->dtype == OTG_F64 ? fused_resident_f64(p) : fused_resident_f32(p);
+inline bool fused_holds_gibbs(const OtgDenseProblem* p) {
+  return p->dtype == OTG_F64 ? fused_holds_gibbs_f64(p) : fused_holds_gibbs_f32(p);
 }
 
 }  // namespace otg

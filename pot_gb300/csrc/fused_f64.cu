@@ -8,5 +8,5 @@ template <> int fu_launch_log<double>(FusedArgs<double>& A, const FuPlan& f, boo
 
 int fused_launch_f64(const OtgDenseProblem* p, const FusedState& fs, cudaStream_t st) { return fused_run<double>(p, fs, st); }
 size_t fused_bytes_f64(int64_t n, int64_t m, int requested_grid) { return fused_run_bytes<double>(n, m, requested_grid); }
-bool fused_resident_f64(const OtgDenseProblem* p) { return fused_run_resident<double>(p); }
+bool fused_holds_gibbs_f64(const OtgDenseProblem* p) { return fused_run_holds_gibbs<double>(p); }
 }  // namespace otg

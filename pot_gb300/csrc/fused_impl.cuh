@@ -1454,10 +1454,10 @@ size_t fused_run_bytes(int64_t n, int64_t m, int requested_grid) {
 }
 
 template <typename T>
-bool fused_run_resident(const OtgDenseProblem* p) {
+bool fused_run_holds_gibbs(const OtgDenseProblem* p) {
   FuPlan f;
   int mode;
-  return fu_choose<T>(p, mode, fu_device(), f) && f.res;
+  return fu_choose<T>(p, mode, fu_device(), f) && (f.res || p->m % Vec<T>::N != 0);
 }
 
 }  // namespace otg
