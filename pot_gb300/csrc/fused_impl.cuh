@@ -63,7 +63,7 @@
 // per iteration, two passes 95; 3000 x 1100 float64 439, two passes 845.)
 //
 // float64 log form, cost resident: this GPU issues FP64 at about two lanes
-// per clock and SM, and an exponential costs some twenty such operations.
+// per clock and SM, and an exponential costs some ten such operations.
 // The solver stores the plan of the current potentials with its rows
 // normalised to one, K_ij = exp(x_ij + f_i - log a_i + g_j), and iterates
 // scalings u, v over it, f + log u and g + log v being the potentials: two
@@ -200,12 +200,6 @@ __device__ __forceinline__ void fu_get_global(const FusedArgs<T>& A, int row, in
 // A scaling of FU_ABS that needs no absorption: within [2^-300, 2^300].
 __device__ __forceinline__ bool fu_tame(double x) { return fu_at_least(x, 0x1p-300) && !fu_at_least(x, 0x1p300); }
 
-// ---------------------------------------------------------------------------
-// Ring of the streamed form.  Chunk j of a group's pass is half (j & 1) of
-// row ga + j / 2, mp / 2 elements per slot.  The chunks of the next pass
-// follow those of this one (the cost does not change), so the ring never runs
-// dry over the hand-over.
-// ---------------------------------------------------------------------------
 // Column sums of the CTA, over the row groups in group order, to its slot.
 template <typename T, int NK>
 __device__ __forceinline__ void fu_publish_cols(const FusedArgs<T>& A, const FuRow& R, const FuSmem<T>& sm,
@@ -432,7 +426,7 @@ __device__ __forceinline__ int fu_pass(const FusedArgs<T>& A, const FuRow& R_, c
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const uint32_t xc = xa + (uint32_t)ring.slot * chunk, vc = va + half * (NK / 2) * hop;
-        if (!fu_landed(full + ring.slot, ring.phase, A.info + 3, A.timeout_ns)) flag |= FU_ABORT;
+        if (!mbar_wait(full + ring.slot, ring.phase, A.info + 3, A.timeout_ns)) flag |= FU_ABORT;
         if (half == 0 || kv > NK / 2) {
 #pragma unroll
           for (int kk = 0; kk < NK / 2; ++kk) {

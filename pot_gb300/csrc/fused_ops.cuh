@@ -111,7 +111,11 @@ template <> struct FuV<double> {
   __device__ __forceinline__ double max_with(double m) const { return fmax(m, fmax(a, b)); }
 };
 
-// Chunk j into `slot`; `rows`: rows of the group, M0: its first one.
+// Ring of the streamed form.  Chunk j of a group's pass is half (j & 1) of its
+// row j / 2, `half` elements per slot.  The chunks of the next pass follow
+// those of this one (the cost does not change), so the ring never runs dry
+// over the hand-over.  Chunk j into `slot`; `rows`: rows of the group, M0: its
+// first one.
 template <typename T>
 __device__ __forceinline__ void fu_issue(const T* M0, int64_t ldm, int mv, int half, int rows, T* slots, uint64_t* full, int j,
                                          int slot) {
@@ -124,11 +128,6 @@ __device__ __forceinline__ void fu_issue(const T* M0, int64_t ldm, int mv, int h
   } else {
     mbar_arrive(full + slot);
   }
-}
-
-// Wait for a chunk (bounded: false after timeout_ns or an abort elsewhere).
-__device__ __forceinline__ bool fu_landed(uint64_t* bar, uint32_t parity, int* abort_flag, uint64_t timeout_ns) {
-  return mbar_wait(bar, parity, abort_flag, timeout_ns);
 }
 
 // ---------------------------------------------------------------------------

@@ -2,10 +2,10 @@
 // problem in every half-step, so the time follows the batch's total work and
 // a slow problem is spread over the whole GPU instead of one CTA.
 //
-// Batches whose widest row the one-read kernel holds (multi_fused.cuh) go
-// there; the two-pass kernel below takes the others, and calls whose partials
-// have no room for that kernel's slots.  The tail kernel takes the last
-// problems of either.
+// Batches whose widest block the one-read kernel takes (multi_fused.cuh: up to
+// 16384 float32 or 8192 float64 columns) run there; the two-pass kernel below
+// takes wider ones, and calls whose partials have no room for that kernel's
+// slots.  The tail kernel takes the last problems of either.
 //
 // Reference behaviour (PythonOT/POT): per problem, the order and stopping test
 // of ot/bregman/_sinkhorn.py:880-899 (sinkhorn_log: v first, then u; L2
@@ -30,10 +30,6 @@
 // the history with the plain step).  u is always the exact row update of the
 // v in use, so the stop test measures exactly what it measures for plain
 // sinkhorn_log: the column marginal of (u, v) with u = rowT(v).
-//
-// Batches whose widest block the one-read kernel takes (multi_fused.cuh: up to
-// 16384 float32 or 8192 float64 columns) run there; the kernel of this file
-// is for wider ones and for callers whose workspace has no room for it.
 //
 // One persistent cooperative launch.  Each iteration:
 //   column pass : units (problem, row chunk, slab of 32*VW columns) over all
@@ -962,14 +958,14 @@ int launch_multi(const OtgMultiProblem* q, cudaStream_t st) {
     const int rc = multi_fused_launch(A, LOGF, f.NK, grid, f.smem, leaving, st);
     if (rc != OTG_OK) return rc;
   } else {
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, multi_sinkhorn_kernel<T, LOGF>, MT_THREADS, 0);
-  int grid = sms * std::min(per, MtBlocks<T>::value);
-  if (q->grid > 0 && q->grid < grid) grid = q->grid;
-  if (grid < 1) return OTG_ERR_UNSUPPORTED;
-  void* args[] = {&A, &leaving};
-  e = cudaLaunchCooperativeKernel((const void*)multi_sinkhorn_kernel<T, LOGF>, dim3(grid), dim3(MT_THREADS),
-                                  args, 0, st);
-  if (e != cudaSuccess) return OTG_ERR_CUDA;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, multi_sinkhorn_kernel<T, LOGF>, MT_THREADS, 0);
+    int grid = sms * std::min(per, MtBlocks<T>::value);
+    if (q->grid > 0 && q->grid < grid) grid = q->grid;
+    if (grid < 1) return OTG_ERR_UNSUPPORTED;
+    void* args[] = {&A, &leaving};
+    e = cudaLaunchCooperativeKernel((const void*)multi_sinkhorn_kernel<T, LOGF>, dim3(grid), dim3(MT_THREADS),
+                                    args, 0, st);
+    if (e != cudaSuccess) return OTG_ERR_CUDA;
   }
   if (A.tail_max > 0) {
     // behind the batch kernel on the stream; returns at once unless it was handed problems
