@@ -29,8 +29,20 @@ def upload(device, arrays):
     for x, o in zip(arrays, offs):
         view[o:o + x.nbytes] = np.ascontiguousarray(x).view(np.uint8).reshape(-1)
     dev = host.to(device, non_blocking=True)
-    return [dev[o:o + x.nbytes].view(torch.from_numpy(np.empty(0, x.dtype)).dtype).view(x.shape)
-            for x, o in zip(arrays, offs)]
+    out = [dev[o:o + x.nbytes].view(_torch_dtype(x.dtype)) for x, o in zip(arrays, offs)]
+    return [t if x.ndim == 1 else t.view(x.shape) for t, x in zip(out, arrays)]
+
+
+_TORCH = {}
+
+
+def _torch_dtype(dtype):
+    """The torch type of a numpy type, asked for once each (4 us, nine times
+    per batch layout)."""
+    t = _TORCH.get(dtype)
+    if t is None:
+        t = _TORCH[dtype] = torch.from_numpy(np.empty(0, dtype)).dtype
+    return t
 
 
 class Boundary:

@@ -82,11 +82,12 @@ def solve_dense(M, a, b, reg, method, max_iter, stop_thr, warm_u=None, warm_v=No
     cap = max(2, max_iter // check_period + 2)
     # the stabilised form runs the two-pass kernel, and so does a solve without
     # room for what the one-read kernel wants (up to a padded copy of the cost)
-    least = lib.otg_dense_workspace_least(dt, n, m, cap, grid)
-    wsb = least if method == _lib.OTG_METHOD_STAB else lib.otg_dense_workspace_bytes(dt, n, m, cap, grid)
+    size = lib.otg_dense_workspace_least if method == _lib.OTG_METHOD_STAB else lib.otg_dense_workspace_bytes
+    wsb = size(dt, n, m, cap, grid)
     try:
         ws = torch.empty(wsb, dtype=torch.uint8, device=M.device)
     except torch.cuda.OutOfMemoryError:
+        least = lib.otg_dense_workspace_least(dt, n, m, cap, grid)
         if wsb == least:
             raise
         wsb = least
